@@ -70,4 +70,97 @@ constexpr int T_O = 256;
 
 __device__ __forceinline__ float max3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
 
+// ------------------------------------------------------------------------------------------------
+// Softmax of one 64-column sub-tile of one branch.  Thread = query row.
+//
+// Two warpgroups per branch take alternate sub-tiles (score buffer u = sub-tile & 1 belongs to warpgroup u), so that
+// one of them works on its exponentials while the other waits for scores, loads them or stores its probabilities.
+// Both accumulate into the same O_b and must use one reference maximum: sub-tile t first finds its own row maximum,
+// then takes over the running one that sub-tile t-1 published (`m_row` in shared memory),
+// keeps it unless the tile exceeds it by more than 2^8 (always at t = 0, otherwise rare), publishes the result and only
+// then starts its exponentials: the serial part between two sub-tiles is the short maximum pass.  Raising the
+// maximum rescales O_b once P_b V of sub-tile t-1 has completed, so P never leaves fp16 range and the final division by
+// l is exact.  Each warpgroup keeps its own share of the row sum l, relative to the maximum it last saw.
+// ------------------------------------------------------------------------------------------------
+struct SoftmaxState {
+  float m = -INFINITY, l = 0.f;
+};
+struct DropRow {                 // dropout of one query row: this row's half of every 2 x 2 block hash (see sm100.cuh)
+  uint32_t key, row2, thresh;
+  int row_odd;
+};
+
+// t_s: this thread's lane and the sub-tile's score columns in TMEM; t_o, O_COLS: the branch's accumulator; nv: visible columns of
+// this row (the rest get -inf, probability 0); wait_m / publish_m: hand-over of the running maximum; wait_pv: P_b V of
+// sub-tile t-1 has completed (false: a bounded wait gave up).
+template <bool BF, bool DROP, int O_COLS, class WaitM, class PublishM, class WaitPv>
+__device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, uint32_t t_o, int t, int nv, float sl2, volatile float* m_row,
+                                                const DropRow& dr, WaitM wait_m, PublishM publish_m, WaitPv wait_pv) {
+  uint32_t sr[64];
+  tmem_ld32(t_s, sr);
+  tmem_ld32(t_s + 32, sr + 32);
+  tc_wait_ld();
+  if (nv < 64) {
+#pragma unroll
+    for (int i = 0; i < 64; ++i)
+      if (i >= nv) sr[i] = 0xff800000u;
+  }
+  float mx[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) mx[c] = __uint_as_float(sr[c]);
+#pragma unroll
+  for (int i = 2; i < 32; ++i) mx[i & 3] = max3(mx[i & 3], __uint_as_float(sr[2 * i]), __uint_as_float(sr[2 * i + 1]));
+  const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+  float m_prev = -INFINITY;
+  if (t > 0) {
+    wait_m();
+    m_prev = *m_row;
+  }
+  const bool need = (m_tile - m_prev) * sl2 > 8.f;       // t = 0: infinity
+  const float m = need ? m_tile : m_prev;
+  if (need) *m_row = m;
+  publish_m();
+  if (__any_sync(0xffffffffu, need) && t > 0) {
+    if (!wait_pv()) return false;
+    tc_fence_after();
+    const float scale = need ? ex2((m_prev - m) * sl2) : 1.f;
+#pragma unroll 1
+    for (int c = 0; c < O_COLS / 16; ++c) {
+      uint32_t o[16];
+      tmem_ld16(t_o + c * 16, o);
+      tc_wait_ld();
+#pragma unroll
+      for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * scale);
+      tmem_st16(t_o + c * 16, o);
+    }
+  }
+  if (m != st.m) {
+    st.l *= ex2((st.m - m) * sl2);
+    st.m = m;
+  }
+  const f32x2 sl2_2 = pk2(sl2, sl2), neg_2 = pk2(-m * sl2, -m * sl2);
+  f32x2 sum2[2] = {pk2(0.f, 0.f), pk2(0.f, 0.f)};
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    const f32x2 x = fma2(pk2u(sr[2 * i], sr[2 * i + 1]), sl2_2, neg_2);
+    float x0, x1;
+    up2(x, x0, x1);
+    const float p0 = ex2(x0), p1 = ex2(x1);
+    sum2[i & 1] = add2(sum2[i & 1], pk2(p0, p1));          // the softmax denominator is taken before dropout
+    sr[i] = pack2<BF>(p0, p1);
+  }
+  float sa, sb;
+  up2(add2(sum2[0], sum2[1]), sa, sb);
+  st.l += sa + sb;
+  if constexpr (DROP) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      sr[i] &= drop_pair_mask(drop_hash(dr.key, dr.row2, uint32_t(t * 32 + i)), dr.row_odd, dr.thresh);
+  }
+  tmem_st32(t_s, sr);
+  tc_wait_st();
+  tc_fence_before();
+  return true;
+}
+
 }  // namespace da

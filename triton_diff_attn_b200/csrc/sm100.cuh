@@ -388,12 +388,6 @@ __device__ __forceinline__ float ex2(float x) {
 // kernels are bound by instruction issue around the exp unit, not by the unit's rate.  With the packed f32x2
 // instructions the routine costs 10 instructions per pair; every 3rd, 4th, 6th pair of the forward then measured
 // 0.825, 0.821, 0.804 ms against 0.804 ms without it.  The routine is not kept.)
-// the same, pinned in program order relative to other volatile statements (barrier arrivals between two groups of them)
-__device__ __forceinline__ float ex2v(float x) {
-  float y;
-  asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
   __half2 h = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&h);
