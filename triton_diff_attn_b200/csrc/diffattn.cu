@@ -307,6 +307,11 @@ int fwd_impl(const DiffAttnParams* p) {
   a.drop_thresh = p->dropout_threshold; a.seed_lo = uint32_t(p->dropout_seed); a.seed_hi = uint32_t(p->dropout_seed >> 32);
   a.drop_scale = 256.f / float(256u - p->dropout_threshold);
   a.gain = p->gain; a.yg = static_cast<__half*>(p->y_gained);
+  // outputs leave through TMA stores: dense [B*H, N, 2D] maps with 128-row boxes
+  CUtensorMap my, ma2;
+  const long long bh = (long long)p->B * p->H;
+  if ((rc = make_map<BF>(&my, p->y, DV, p->N, (int)bh, 1, DV, (int64_t)p->N * DV, (int64_t)p->N * DV * bh, 128, "y"))) return rc;
+  if ((rc = make_map<BF>(&ma2, p->a2, DV, p->N, (int)bh, 1, DV, (int64_t)p->N * DV, (int64_t)p->N * DV * bh, 128, "a2"))) return rc;
   if (D == 128) {
     // one CTA per branch; the two CTAs of a query tile form a cluster and exchange A2 through distributed shared memory
     if ((rc = set_smem(da::diffattn_fwd128_branch_kernel<BF, DROP>, da::fwd128::SMEM_BYTES, p->device))) return rc;
@@ -320,14 +325,9 @@ int fwd_impl(const DiffAttnParams* p) {
     attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 2;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    DA_CUDA(cudaLaunchKernelEx(&cfg, da::diffattn_fwd128_branch_kernel<BF, DROP>, mq1, mq2, mk1, mk2, mv, a));
+    DA_CUDA(cudaLaunchKernelEx(&cfg, da::diffattn_fwd128_branch_kernel<BF, DROP>, mq1, mq2, mk1, mk2, mv, my, ma2, a));
     return DIFFATTN_OK;
   }
-  // outputs leave through TMA stores: dense [B*H, N, 2D] maps with 128-row boxes
-  CUtensorMap my, ma2;
-  const long long bh = (long long)p->B * p->H;
-  if ((rc = make_map<BF>(&my, p->y, DV, p->N, (int)bh, 1, DV, (int64_t)p->N * DV, (int64_t)p->N * DV * bh, 128, "y"))) return rc;
-  if ((rc = make_map<BF>(&ma2, p->a2, DV, p->N, (int)bh, 1, DV, (int64_t)p->N * DV, (int64_t)p->N * DV * bh, 128, "a2"))) return rc;
   CUtensorMap myg = my;      // only read by the kernel when a gain is given
   if (p->gain && (rc = make_map<BF>(&myg, p->y_gained, DV, p->N, (int)bh, 1, DV, (int64_t)p->N * DV, (int64_t)p->N * DV * bh, 128, "y_gained"))) return rc;
   dim3 grid((p->N + 127) / 128, p->B * p->H);

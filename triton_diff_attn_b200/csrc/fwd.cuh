@@ -90,16 +90,20 @@ struct DropRow {                 // dropout of one query row: this row's half of
   int row_odd;
 };
 
-// t_s: this thread's lane and the sub-tile's score columns in TMEM; t_o, O_COLS: the branch's accumulator; nv: visible columns of
-// this row (the rest get -inf, probability 0); wait_m / publish_m: hand-over of the running maximum; wait_pv: P_b V of
-// sub-tile t-1 has completed (false: a bounded wait gave up).
-template <bool BF, bool DROP, int O_COLS, class WaitM, class PublishM, class WaitPv>
-__device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, uint32_t t_o, int t, int nv, float sl2, volatile float* m_row,
-                                                const DropRow& dr, WaitM wait_m, PublishM publish_m, WaitPv wait_pv) {
+// t_s: this thread's lane and the sub-tile's score columns in TMEM; t_p: where its probabilities go (two per column; may be
+// t_s); t_o, O_COLS: the branch's accumulator; nv: visible columns of this row (the rest get -inf, probability 0); loaded:
+// the scores are in registers; wait_m / publish_m: hand-over of the running maximum; wait_pv: P_b V of
+// sub-tile t-1 has completed; mid: runs half way through the exponentials; p_free: the
+// columns behind t_p may be overwritten (both false: a bounded wait gave up).
+template <bool BF, bool DROP, int O_COLS, class Loaded, class WaitM, class PublishM, class WaitPv, class Mid, class PFree>
+__device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, uint32_t t_p, uint32_t t_o, int t, int nv, float sl2,
+                                                volatile float* m_row, const DropRow& dr, Loaded loaded, WaitM wait_m, PublishM publish_m,
+                                                WaitPv wait_pv, Mid mid, PFree p_free) {
   uint32_t sr[64];
   tmem_ld32(t_s, sr);
   tmem_ld32(t_s + 32, sr + 32);
   tc_wait_ld();
+  loaded();
   if (nv < 64) {
 #pragma unroll
     for (int i = 0; i < 64; ++i)
@@ -142,6 +146,7 @@ __device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, 
   f32x2 sum2[2] = {pk2(0.f, 0.f), pk2(0.f, 0.f)};
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
+    if (i == 16) mid();
     const f32x2 x = fma2(pk2u(sr[2 * i], sr[2 * i + 1]), sl2_2, neg_2);
     float x0, x1;
     up2(x, x0, x1);
@@ -157,10 +162,11 @@ __device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, 
     for (int i = 0; i < 32; ++i)
       sr[i] &= drop_pair_mask(drop_hash(dr.key, dr.row2, uint32_t(t * 32 + i)), dr.row_odd, dr.thresh);
   }
-  tmem_st32(t_s, sr);
+  const bool ok = p_free();
+  tmem_st32(t_p, sr);
   tc_wait_st();
   tc_fence_before();
-  return true;
+  return ok;
 }
 
 }  // namespace da

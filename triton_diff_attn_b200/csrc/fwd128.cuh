@@ -1,55 +1,54 @@
 // Differential-attention forward for head dim D = 128 (value width 256), sm_100a.
 //
 // Two 256-wide accumulators do not fit in TMEM next to the score buffers, so the two branches run in the two CTAs of a
-// thread-block cluster (blockIdx.z = branch).  Same softmax scheme as the D <= 64 kernel (fwd.cuh, fwd64.cuh): scores
-// in two alternating 64-column TMEM buffers, one exp pass per sub-tile against the stale running maximum, P written
-// over its scores as the TMEM A operand of P V.  Streamed tiles are 64 rows: {K_b, V}.  At the end branch 2 hands its
+// thread-block cluster (blockIdx.z = branch): with a single branch the whole accumulator fits and nothing is computed twice
+// (12 units of B*H*N^2*D and 2 N^2 exponentials per head).  Softmax as in the D <= 64 kernel (softmax_subtile in fwd.cuh):
+// two warpgroups on alternate 64-column sub-tiles, half a pass apart.  TMEM also holds the probabilities apart from the scores
+// (S(t+2) is computed as soon as S(t) is in registers) and Q, the A operand of the score MMAs.  At the end branch 2 hands its
 // A2 = O_2 / l_2 in fp32 to branch 1 through distributed shared memory, and branch 1 forms y and rstd.
-// (An earlier form kept both branches in one CTA and made two passes over the keys, one per 128-column half of V, with
-// the probabilities recomputed in the second: 16 units of B*H*N^2*D and 4 N^2 exponentials per head; it measured
-// 1.97 ms against 1.4 ms for this form at B2 H8 N8192 D128.  A form without the cluster -- branch 1 writes A1 as 16-bit
-// values into y, a second kernel combines -- was as fast but lost accuracy where A1 - lambda A2 cancels: with bf16
-// tensors, lambda 0.8, a causal mask and rms_norm two of 400 seeded cases left the tolerance.  The same
-// one-branch-per-CTA form at head dim 64 -- S and O take 256 TMEM columns and 90 KB of shared memory, so two CTAs share
-// an SM -- measured 0.84 ms against 0.81 ms for the D <= 64 kernel of fwd64.cuh at B4 H16 N4096 D64: there nothing is
-// computed twice to begin with.)
+// What bounds it: the tensor pipe needs 768 clocks per sub-tile (S 256, P V 512), and at B2 H8 N8192 D128 it executes
+// 1377 TFLOP/s sustained, the rate a plain cuBLAS loop reaches under the 1 kW cap.  Against one softmax warpgroup with P over
+// its scores and Q in shared memory: 1.44 -> 1.20 ms there, 0.206 -> 0.160 ms at B1 H8 N4096 causal; both warpgroups in phase 1.29.
+// (An earlier form kept both branches in one CTA and made two passes over the keys, with the probabilities recomputed in
+// the second: 1.97 ms.  A form without the cluster -- branch 1 writes A1 as 16-bit values into y, a second kernel
+// combines -- lost accuracy where A1 - lambda A2 cancels: with bf16 tensors, lambda 0.8, a causal mask and rms_norm two of 400
+// seeded cases left the tolerance.)
 #pragma once
 #include "fwd.cuh"
 #include "sm100.cuh"
 
 namespace da {
 
-// ------------------------------------------------------------------------------------------------
-// One branch per CTA (blockIdx.z; the two CTAs of a query tile are one cluster), one pass: with a single branch the
-// whole 256-wide accumulator fits in TMEM next to the score buffers, so nothing is computed twice (12 units of
-// B*H*N^2*D and 2 N^2 exponentials per head).
-// TMEM: S two 64-column buffers [0,128) | O [128,384).  Warps 0-3 softmax (thread = query row), 4 TMA, 5 MMA issuer.
-// ------------------------------------------------------------------------------------------------
 namespace fwd128 {
-constexpr int BM = 128, SUB = 64, HD = 128, DV = 256, ST = 3;
+constexpr int BM = 128, SUB = 64, HD = 128, DV = 256;
+constexpr int KS = 4, VS = 3;                   // ring depths: K is requested two sub-tiles ahead of V
 constexpr int Q_BYTES = BM * HD * 2;            // 32 KB: two boxes [128 x 64]
 constexpr int K_BYTES = SUB * HD * 2;           // 16 KB: two boxes [64 x 64]
 constexpr int V_BYTES = SUB * DV * 2;           // 32 KB: four boxes [64 x 64]
-constexpr int STAGE_BYTES = K_BYTES + V_BYTES;  // 48 KB
-constexpr int OFF_Q = 0, OFF_STAGE = Q_BYTES;
-constexpr int OFF_MISC = OFF_STAGE + ST * STAGE_BYTES;      // 176 KB
-constexpr int MISC_BYTES = 1024;
+constexpr int OFF_Q = 0, OFF_K = Q_BYTES, OFF_V = OFF_K + KS * K_BYTES;
+constexpr int OFF_MISC = OFF_V + VS * V_BYTES;              // 192 KB
+// epilogue, rings and Q idle: 64-column tiles of the outputs (16 KB each) from 0, the fp32 exchange tile (128 KB) behind them
+constexpr int OUT_TILE_BYTES = BM * 128;
+constexpr int OFF_OUT = 0, OFF_X = 4 * OUT_TILE_BYTES;
+static_assert(OFF_X + BM * DV * 4 <= OFF_MISC, "epilogue tiles do not fit");
+constexpr int MISC_BYTES = 6144;
 constexpr int SMEM_BYTES = OFF_MISC + MISC_BYTES + 1024;
-// warps 0-3 softmax (thread = query row, all 64 columns of a sub-tile), warp 4 TMA, warp 5 MMA issuer.  (Two softmax
-// warps per lane quarter, 32 columns each, exchanging the row maximum through shared memory and a 64-thread named
-// barrier once per sub-tile, measured 1.49 ms against 1.38 ms at B2 H8 N8192 D128: the exchange costs more than the
-// second warp's help on the exp unit brings.)
-constexpr int NUM_THREADS = 192;
-constexpr int WARP_TMA = 4, WARP_MMA = 5;
-constexpr int T_S = 0, T_O = 128;
+constexpr int NUM_SOFTMAX = 256;
+constexpr int NUM_THREADS = NUM_SOFTMAX + 128;
+constexpr int WARP_TMA = 8, WARP_PV = 9, WARP_S = 10, WARP_TMA_V = 11;
+// TMEM: S two 64-column buffers | P likewise, 16-bit pairs | Q as 16-bit pairs | O
+constexpr int T_S = 0, T_P = 128, T_Q = 192, T_O = 256;
+constexpr int NB_P = 2, NB_SF = 4, NB_M = 6, NB_OUT = 9, NB_START = 11;     // named barriers, + sub-tile parity (1: the softmax warps)
 struct Misc {
-  uint64_t bar_q;
-  uint64_t full[ST], empty[ST];
-  uint64_t s_full[2], p_full[2];
-  uint64_t o_done, o_full;
+  uint64_t bar_q, q_ready;
+  uint64_t k_full[KS], k_empty[KS], v_full[VS], v_empty[VS];
+  uint64_t s_full[2], pv_done[2], o_full;
   uint64_t peer_ready, peer_data;     // arrivals come from the partner CTA of the cluster (the other branch)
   uint32_t tmem_slot;
   int abort_flag;
+  float m_run[BM];                    // running row maximum
+  float m_end[2][BM], l_end[2][BM];   // maximum and row sum of each warpgroup at the end
+  float ssq[2][BM];
 };
 static_assert(sizeof(Misc) <= MISC_BYTES, "misc area too small");
 }  // namespace fwd128
@@ -58,7 +57,8 @@ template <bool BF, bool DROP>
 __global__ void __launch_bounds__(fwd128::NUM_THREADS, 1)
 diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_constant__ CUtensorMap tm_q2,
                               const __grid_constant__ CUtensorMap tm_k1, const __grid_constant__ CUtensorMap tm_k2,
-                              const __grid_constant__ CUtensorMap tm_v, const FwdArgs args) {
+                              const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_y,
+                              const __grid_constant__ CUtensorMap tm_a2, const FwdArgs args) {
   using namespace fwd128;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -73,18 +73,36 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
   const CUtensorMap* tm_q = br ? &tm_q2 : &tm_q1;
   const CUtensorMap* tm_k = br ? &tm_k2 : &tm_k1;
 
+  auto load_k = [&](int t) {
+    const int s = t % KS;
+    uint8_t* kp = smem + OFF_K + s * K_BYTES;
+    mbar_expect_tx(&misc->k_full[s], K_BYTES);
+    for (int c = 0; c < 2; ++c) tma_load_4d(kp + c * 8192, tm_k, &misc->k_full[s], c * 64, t * SUB, h_idx, b_idx);
+  };
+  auto load_v = [&](int t) {
+    const int s = t % VS;
+    uint8_t* vp = smem + OFF_V + s * V_BYTES;
+    mbar_expect_tx(&misc->v_full[s], V_BYTES);
+    for (int c = 0; c < 4; ++c) tma_load_4d(vp + c * 8192, &tm_v, &misc->v_full[s], c * 64, t * SUB, h_idx, b_idx);
+  };
   if (warp == WARP_TMA && lane == 0) {
     mbar_init(&misc->bar_q, 1);
-    for (int i = 0; i < ST; ++i) { mbar_init(&misc->full[i], 1); mbar_init(&misc->empty[i], 1); }
-    for (int u = 0; u < 2; ++u) { mbar_init(&misc->s_full[u], 1); mbar_init(&misc->p_full[u], 128); }
-    mbar_init(&misc->o_done, 1);
+    mbar_init(&misc->q_ready, NUM_SOFTMAX);
+    for (int i = 0; i < KS; ++i) { mbar_init(&misc->k_full[i], 1); mbar_init(&misc->k_empty[i], 1); }
+    for (int i = 0; i < VS; ++i) { mbar_init(&misc->v_full[i], 1); mbar_init(&misc->v_empty[i], 1); }
+    for (int u = 0; u < 2; ++u) { mbar_init(&misc->s_full[u], 1); mbar_init(&misc->pv_done[u], 1); }
     mbar_init(&misc->o_full, 1);
     mbar_init(&misc->peer_ready, 1);
-    mbar_init(&misc->peer_data, 128);
+    mbar_init(&misc->peer_data, NUM_SOFTMAX);
     misc->abort_flag = 0;
     mbar_init_fence();
+    // the first loads go out before the setup barriers; the first pass over a ring needs no "empty" wait
+    mbar_expect_tx(&misc->bar_q, Q_BYTES);
+    for (int c = 0; c < 2; ++c) tma_load_4d(smem + OFF_Q + c * 16384, tm_q, &misc->bar_q, c * 64, q_tile * BM, h_idx, b_idx);
+    load_k(0); load_k(1); load_v(0); load_v(1);                 // nsub >= 2
+    tma_prefetch_desc(&tm_y); tma_prefetch_desc(&tm_a2);
   }
-  if (warp == WARP_MMA) tmem_alloc(&misc->tmem_slot, 512);
+  if (warp == WARP_PV) tmem_alloc(&misc->tmem_slot, 512);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();          // the partner's mbarriers are initialised before anything arrives on them
@@ -93,267 +111,254 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
 
   if (warp == WARP_TMA) {
     if (elect_one()) {
-      mbar_expect_tx(&misc->bar_q, Q_BYTES);
-      for (int c = 0; c < 2; ++c) tma_load_4d(smem + OFF_Q + c * 16384, tm_q, &misc->bar_q, c * 64, q_tile * BM, h_idx, b_idx);
-      int st = 0;
-      uint32_t par = 1;
-      for (int t = 0; t < nsub; ++t) {
-        uint8_t* sp = smem + OFF_STAGE + st * STAGE_BYTES;
-        if (!mbar_wait(&misc->empty[st], par, abort_flag, 2101, t)) break;
-        mbar_expect_tx(&misc->full[st], STAGE_BYTES);
-        for (int c = 0; c < 2; ++c) tma_load_4d(sp + c * 8192, tm_k, &misc->full[st], c * 64, t * SUB, h_idx, b_idx);
-        for (int c = 0; c < 4; ++c) tma_load_4d(sp + K_BYTES + c * 8192, &tm_v, &misc->full[st], c * 64, t * SUB, h_idx, b_idx);
-        if (++st == ST) { st = 0; par ^= 1; }
+      for (int t = 2; t < nsub; ++t) {
+        if (!mbar_wait(&misc->k_empty[t % KS], ((t / KS) & 1) ^ 1, abort_flag, 2101, t)) break;
+        load_k(t);
       }
     }
-  } else if (warp == WARP_MMA) {
+  } else if (warp == WARP_TMA_V) {
+    // (a producer warp per ring: the score MMAs run two sub-tiles ahead of P V, and with one warp for both rings the next
+    // K waits behind a V whose stage is not free yet: 2.3 ms against 1.4 ms at B2 H8 N8192 D128)
     if (elect_one()) {
-      constexpr uint32_t IDESC_S = make_idesc(BM, SUB, 0, 0, BF);
-      constexpr uint32_t IDESC_O = make_idesc(BM, DV, 0, 1, BF);      // V as MN-major B: four 64-column atoms 8 KB apart
-      const uint32_t q_lo = sdesc_lo(smem_u32(smem + OFF_Q));
-      const uint32_t st_lo0 = sdesc_lo(smem_u32(smem + OFF_STAGE));
-      const uint32_t tb = tmem_base;
-      auto issue_s = [&](uint32_t sp_lo, int u) {
+      for (int t = 2; t < nsub; ++t) {
+        if (!mbar_wait(&misc->v_empty[t % VS], ((t / VS) & 1) ^ 1, abort_flag, 2102, t)) break;
+        load_v(t);
+      }
+    }
+  } else if (warp == WARP_S) {
+    // S(t+2) = Q K^T once the scores of sub-tile t are in registers.  Scores and probabilities have TMEM columns of their
+    // own, so a warpgroup finds its next scores ready when it has stored its probabilities, and the two kinds of MMAs need no
+    // order between them: two issuing warps, so that one's waits run under the other's MMAs (1.198 ms against 1.207 ms
+    // with one warp for both at B2 H8 N8192 D128).
+    constexpr uint32_t IDESC_S = make_idesc(BM, SUB, 0, 0, BF);
+    const uint32_t k_lo0 = sdesc_lo(smem_u32(smem + OFF_K));
+    bool ok = mbar_wait_warp(&misc->q_ready, 0, abort_flag, 2201);
+    for (int t = 0; ok && t < nsub; ++t) {
+      const int ks = t % KS, u = t & 1;
+      ok = mbar_wait_warp(&misc->k_full[ks], (t / KS) & 1, abort_flag, 2202, t);
+      if (!ok) break;
+      if (t >= 2) named_bar_sync(NB_SF + u, 160);
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k)
-          mma_ss_lo(tb + T_S + u * SUB, q_lo + (k / 4) * (16384 >> 4) + (k % 4) * 2, sp_lo + (k / 4) * (8192 >> 4) + (k % 4) * 2, IDESC_S, k > 0);
+          mma_ts_lo(tmem_base + T_S + u * SUB, tmem_base + T_Q + k * 8, k_lo0 + ks * (K_BYTES >> 4) + (k / 4) * (8192 >> 4) + (k % 4) * 2, IDESC_S, k > 0);
         mma_commit(&misc->s_full[u]);
-      };
-      bool ok = mbar_wait(&misc->bar_q, 0, abort_flag, 2201);
-      ok = ok && mbar_wait(&misc->full[0], 0, abort_flag, 2202);
-      if (ok) {
-        tc_fence_after();
-        issue_s(st_lo0, 0);
-        int st = 0;
-        uint32_t par = 0;
-        for (int t = 0; t < nsub; ++t) {
-          const int u = t & 1;
-          const uint32_t sp_lo = st_lo0 + st * (STAGE_BYTES >> 4);
-          const uint32_t v_lo = sp_lo + (K_BYTES >> 4) + ((8192u >> 4) << 16) - (1u << 16);
-          int st_n = st + 1;
-          uint32_t par_n = par;
-          if (st_n == ST) { st_n = 0; par_n ^= 1; }
-          if (t + 1 < nsub) {
-            if (!mbar_wait(&misc->full[st_n], par_n, abort_flag, 2203, t)) break;
-            tc_fence_after();
-            issue_s(st_lo0 + st_n * (STAGE_BYTES >> 4), u ^ 1);
-          }
-          if (!mbar_wait(&misc->p_full[u], (t >> 1) & 1, abort_flag, 2204, t)) break;
-          tc_fence_after();
-#pragma unroll
-          for (int k = 0; k < SUB / 16; ++k)
-            mma_ts_lo(tb + T_O, tb + T_S + u * SUB + k * 8, v_lo + k * (2048 >> 4), IDESC_O, (t > 0 || k > 0));
-          mma_commit(&misc->o_done);
-          mma_commit(&misc->empty[st]);
-          if (t == nsub - 1) mma_commit(&misc->o_full);
-          st = st_n;
-          par = par_n;
-        }
+        mma_commit(&misc->k_empty[ks]);
       }
+      __syncwarp();
     }
+  } else if (warp == WARP_PV) {
+    // O += P(t) V(t)
+    constexpr uint32_t IDESC_O = make_idesc(BM, DV, 0, 1, BF);      // V as MN-major B: four 64-column atoms 8 KB apart
+    const uint32_t v_lo0 = sdesc_lo(smem_u32(smem + OFF_V), 8192);
+    for (int t = 0; t < nsub; ++t) {
+      const int vs = t % VS, u = t & 1;
+      if (!mbar_wait_warp(&misc->v_full[vs], (t / VS) & 1, abort_flag, 2203, t)) break;
+      named_bar_sync(NB_P + u, 160);
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < SUB / 16; ++k)
+          mma_ts_lo(tmem_base + T_O, tmem_base + T_P + u * (SUB / 2) + k * 8, v_lo0 + vs * (V_BYTES >> 4) + k * (2048 >> 4), IDESC_O, (t > 0 || k > 0));
+        mma_commit(&misc->pv_done[u]);
+        mma_commit(&misc->v_empty[vs]);
+      }
+      __syncwarp();
+    }
+    if (elect_one()) mma_commit(&misc->o_full);
   } else {
-    const int row = warp * 32 + lane;
-    const uint32_t lane_base = uint32_t(warp * 32) << 16;
-    const uint32_t t_s0 = tmem_base + lane_base + T_S;
+    const int u = warp >> 2;                                // sub-tile parity of this warpgroup
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
     const uint32_t t_o = tmem_base + lane_base + T_O;
     const float sl2 = args.sm_scale * 1.4426950408889634f;
-    const f32x2 sl2_2 = pk2(sl2, sl2);
     const size_t grow = size_t(bh) * args.n + size_t(q_tile) * BM + row;
-    const uint32_t dkey = DROP ? drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), uint32_t(br)) : 0u;
-    const uint32_t drow2 = uint32_t(q_tile * BM + row) >> 1;
-    const int drow_odd = row & 1;
-    bool ok = true;
-    float m_run = -INFINITY, l_run = 0.f;
-    for (int t = 0; t < nsub; ++t) {
-      const uint32_t t_s = t_s0 + (t & 1) * SUB;
-      if (!mbar_wait(&misc->s_full[t & 1], (t >> 1) & 1, abort_flag, 2301 + br, t)) { ok = false; break; }
-      tc_fence_after();
-      uint32_t sr[SUB];
-      tmem_ld32(t_s + 0, sr);
-      tmem_ld32(t_s + 32, sr + 32);
-      tc_wait_ld();
-      {
-        int nv = args.n - t * SUB;             // visible key columns of this row in this sub-tile; the rest get -inf
-        if (args.causal) nv = min(nv, q_tile * BM + row - t * SUB + 1);
-        if (nv < SUB) {
+    // Q into TMEM, the A operand of S = Q K^T: this thread's row, the 64 columns of box u (128 bytes, swizzled in 16-byte
+    // chunks) -> 32 columns.  The score MMAs then read only K from shared memory (with both operands there an N = 64 step
+    // takes 48 clocks of shared-memory bandwidth for 32 of tensor time).
+    bool ok = mbar_wait_warp(&misc->bar_q, 0, abort_flag, 2300);
+    {
+      uint32_t qv[32];
+      const uint8_t* qrow = smem + OFF_Q + u * 16384 + row * 128;
 #pragma unroll
-          for (int i = 0; i < SUB; ++i)
-            if (i >= nv) sr[i] = 0xff800000u;
-        }
+      for (int c = 0; c < 8; ++c) {
+        const uint4 v = *reinterpret_cast<const uint4*>(qrow + ((c ^ (row & 7)) << 4));
+        qv[4 * c] = v.x; qv[4 * c + 1] = v.y; qv[4 * c + 2] = v.z; qv[4 * c + 3] = v.w;
       }
-      // one pass against the stale running maximum, the sub-tile's own maximum alongside (see fwd64.cuh)
-      float neg = -m_run * sl2;
-      f32x2 sum2[2] = {pk2(0.f, 0.f), pk2(0.f, 0.f)};
-      float mx[4];
-      uint32_t pk[SUB / 2];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) mx[c] = __uint_as_float(sr[c]);
-      if (t > 0) {
-#pragma unroll
-        for (int i = 0; i < SUB / 2; ++i) {
-          float x0, x1;
-          up2(fma2(pk2u(sr[2 * i], sr[2 * i + 1]), sl2_2, pk2(neg, neg)), x0, x1);
-          const float p0 = ex2(x0), p1 = ex2(x1);
-          sum2[i & 1] = add2(sum2[i & 1], pk2(p0, p1));
-          pk[i] = pack2<BF>(p0, p1);
-          mx[i & 3] = max3(mx[i & 3], __uint_as_float(sr[2 * i]), __uint_as_float(sr[2 * i + 1]));
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < SUB / 2; ++i)
-          mx[i & 3] = max3(mx[i & 3], __uint_as_float(sr[2 * i]), __uint_as_float(sr[2 * i + 1]));
-      }
-      const float m_new = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      const bool need = (t == 0) || ((m_new - m_run) * sl2 > 8.f);
-      if (__any_sync(0xffffffffu, need)) {
-        if (t > 0) {
-          // O must be quiescent: wait for P V of the previous sub-tile, then rescale it
-          if (!mbar_wait(&misc->o_done, (t - 1) & 1, abort_flag, 2305 + br, t)) { ok = false; break; }
-          tc_fence_after();
-          const float scale = need ? ex2((m_run - m_new) * sl2) : 1.f;
-          l_run *= scale;
-#pragma unroll
-          for (int c = 0; c < DV / 32; ++c) {
-            uint32_t o[32];
-            tmem_ld32(t_o + c * 32, o);
-            tc_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * scale);
-            tmem_st32(t_o + c * 32, o);
-          }
-        }
-        if (need) m_run = m_new;
-        neg = -m_run * sl2;
-        sum2[0] = sum2[1] = pk2(0.f, 0.f);
-#pragma unroll
-        for (int i = 0; i < SUB / 2; ++i) {
-          float x0, x1;
-          up2(fma2(pk2u(sr[2 * i], sr[2 * i + 1]), sl2_2, pk2(neg, neg)), x0, x1);
-          const float p0 = ex2(x0), p1 = ex2(x1);
-          sum2[i & 1] = add2(sum2[i & 1], pk2(p0, p1));
-          pk[i] = pack2<BF>(p0, p1);
-        }
-      }
-      {
-        float sa, sb;
-        up2(add2(sum2[0], sum2[1]), sa, sb);
-        l_run += sa + sb;                       // the softmax denominator is taken before dropout
-      }
-      if constexpr (DROP) {
-#pragma unroll
-        for (int i = 0; i < SUB / 2; ++i)
-          pk[i] &= drop_pair_mask(drop_hash(dkey, drow2, uint32_t(t * (SUB / 2) + i)), drow_odd, args.drop_thresh);
-      }
-      tmem_st32(t_s, pk);
+      tmem_st32(tmem_base + lane_base + T_Q + u * 32, qv);
       tc_wait_st();
       tc_fence_before();
-      mbar_arrive(&misc->p_full[t & 1]);
+      mbar_arrive(&misc->q_ready);
+    }
+    SoftmaxState st;
+    {
+      const uint32_t t_s = tmem_base + lane_base + T_S + u * SUB, t_p = tmem_base + lane_base + T_P + u * (SUB / 2);
+      DropRow dr;
+      if constexpr (DROP) {
+        dr.key = drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), uint32_t(br));
+        dr.row2 = uint32_t(q_tile * BM + row) >> 1;
+        dr.thresh = args.drop_thresh;
+        dr.row_odd = row & 1;
+      }
+      int t = u;
+      // Warpgroup 1 starts half a pass behind warpgroup 0: in phase, both would be at their exponentials together and
+      // leave the exp unit idle together.
+      if (u == 1) named_bar_sync(NB_START, 256);
+      uint32_t s_ready = 0;             // answer of the early probe (see mbar_probe)
+      for (; ok && t < nsub; t += 2) {
+        ok = s_ready || mbar_wait(&misc->s_full[u], (t >> 1) & 1, abort_flag, 2301 + br, t);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        int nv = args.n - t * SUB;             // visible key columns of this row in this sub-tile
+        if (args.causal) nv = min(nv, q_tile * BM + row - t * SUB + 1);
+        ok = softmax_subtile<BF, DROP, DV>(
+                 st, t_s, t_p, t_o, t, nv, sl2, &misc->m_run[row], dr,
+                 [&] { if (t + 2 < nsub) { tc_fence_before(); named_bar_arrive(NB_SF + u, 160); } },
+                 [&] { named_bar_sync(NB_M + (u ^ 1), 256); }, [&] { if (t + 1 < nsub) named_bar_arrive(NB_M + u, 256); },
+                 [&] { return mbar_wait_warp(&misc->pv_done[u ^ 1], ((t - 1) >> 1) & 1, abort_flag, 2305 + br, t); },
+                 [&] {
+                   if (t == 0) named_bar_arrive(NB_START, 256);
+                   if (t + 2 < nsub) s_ready = mbar_probe(&misc->s_full[u], ((t + 2) >> 1) & 1);
+                 },
+                 [&] { return t < 2 || mbar_wait_warp(&misc->pv_done[u], ((t - 2) >> 1) & 1, abort_flag, 2303 + br, t); });
+        named_bar_arrive(NB_P + u, 160);
+        if (!ok) { t += 2; break; }
+      }
+      // a warp whose wait gave up stands in for the named-barrier arrivals it will no longer make
+      if (!ok && t == 0) named_bar_arrive(NB_START, 256);
+      for (; t < nsub; t += 2) {
+        if (t + 2 < nsub) named_bar_arrive(NB_SF + u, 160);
+        if (t > 0) named_bar_arrive(NB_M + (u ^ 1), 256);
+        if (t + 1 < nsub) named_bar_arrive(NB_M + u, 256);
+        named_bar_arrive(NB_P + u, 160);
+      }
     }
 
     // ---- epilogue.  The two CTAs of a cluster hold A1 = O_1 / l_1 (branch 1) and A2 = O_2 / l_2 (branch 2) of the same 128
     // query rows.  Branch 2 writes a2 and hands its A2 in fp32 to branch 1 through distributed shared memory (into branch
-    // 1's key/value ring, idle by then); branch 1 forms y = RMSNorm(A1 - lambda A2) (1 - lambda_init) and rstd.
-    // Every thread runs every barrier; only the global writes depend on `ok`.
-    ok = mbar_wait(&misc->o_full, 0, abort_flag, 2311 + br) && ok;
+    // 1's rings, idle by then); branch 1 forms y = RMSNorm(A1 - lambda A2) (1 - lambda_init) and rstd.  Warpgroup u has
+    // value columns [128 u, 128 u + 128).  Every thread runs every barrier; only the global writes depend on `ok`.
+    ok = mbar_wait_warp(&misc->o_full, 0, abort_flag, 2311 + br) && ok;
     tc_fence_after();
-    const float inv_l = (DROP ? args.drop_scale : 1.f) / l_run;
+    misc->m_end[u][row] = st.m;
+    misc->l_end[u][row] = st.l;
+    named_bar_sync(1, NUM_SOFTMAX);
+    const float ma = misc->m_end[0][row], mb = misc->m_end[1][row], m_fin = fmaxf(ma, mb);
+    const float l_fin = misc->l_end[0][row] * ex2((ma - m_fin) * sl2) + misc->l_end[1][row] * ex2((mb - m_fin) * sl2);
+    const float inv_l = (DROP ? args.drop_scale : 1.f) / l_fin;
     const bool live = ok && !*abort_flag && (q_tile * BM + row < args.n);
+    uint8_t* out = smem + OFF_OUT + 2 * u * OUT_TILE_BYTES;      // this warpgroup's two 64-column tiles
+    // stores the warpgroup's two tiles once all its threads have written them
+    auto store_tiles = [&](const CUtensorMap* map, uint8_t* tiles) {
+      fence_proxy_async_smem();
+      named_bar_sync(NB_OUT + u, 128);
+      if ((warp & 3) == 0 && elect_one()) {
+        if (!*abort_flag)
+          for (int c = 0; c < 2; ++c) tma_store_4d(tiles + c * OUT_TILE_BYTES, map, (2 * u + c) * 64, q_tile * BM, bh, 0);
+        tma_store_commit();
+        tma_store_wait_read();
+      }
+    };
     // exchange tile: 64 chunks of four floats per row, chunk-major (chunk c of row r at (c * 128 + r) * 16 bytes), so that
     // the 32 rows of a warp touch consecutive 16-byte words
-    uint8_t* xtile = smem + OFF_STAGE;
+    uint8_t* xtile = smem + OFF_X;
     if (br == 1) {
       const uint32_t x_remote = cluster_map(smem_u32(xtile), 0);
-      ok = mbar_wait_cluster(&misc->peer_ready, 0, abort_flag, 2313) && ok;       // branch 1's ring is idle
-      __half* dst = args.a2 + grow * DV;
+      ok = mbar_wait_cluster(&misc->peer_ready, 0, abort_flag, 2313) && ok;       // branch 1's rings are idle
 #pragma unroll
-      for (int c = 0; c < DV / 32; ++c) {
+      for (int c = 0; c < 4; ++c) {
         uint32_t o[32];
-        tmem_ld32(t_o + c * 32, o);
+        tmem_ld32(t_o + u * 128 + c * 32, o);
         tc_wait_ld();
         float f[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(o[i]) * inv_l;
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-          cluster_st_v4(x_remote + uint32_t(((c * 8 + i) * BM + row) * 16), f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
-        if (live) {
+          cluster_st_v4(x_remote + uint32_t(((u * 32 + c * 8 + i) * BM + row) * 16), f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            *reinterpret_cast<uint4*>(dst + c * 32 + 8 * i) =
-                make_uint4(pack2<BF>(f[8 * i + 0], f[8 * i + 1]), pack2<BF>(f[8 * i + 2], f[8 * i + 3]),
-                           pack2<BF>(f[8 * i + 4], f[8 * i + 5]), pack2<BF>(f[8 * i + 6], f[8 * i + 7]));
-        }
+        for (int i = 0; i < 4; ++i)
+          st_swizzled_chunk(out + (c >> 1) * OUT_TILE_BYTES, row, (c & 1) * 4 + i,
+                            make_uint4(pack2<BF>(f[8 * i + 0], f[8 * i + 1]), pack2<BF>(f[8 * i + 2], f[8 * i + 3]),
+                                       pack2<BF>(f[8 * i + 4], f[8 * i + 5]), pack2<BF>(f[8 * i + 6], f[8 * i + 7])));
       }
       cluster_mbar_arrive(cluster_map(smem_u32(&misc->peer_data), 0));
-      if (live) args.lse2[grow] = m_run * args.sm_scale + logf(l_run);
+      store_tiles(&tm_a2, out);
+      if (live && u == 0) args.lse2[grow] = m_fin * args.sm_scale + logf(l_fin);
     } else {
       if (threadIdx.x == 0) cluster_mbar_arrive(cluster_map(smem_u32(&misc->peer_ready), 1));
       const float lam = load_lambda(args.lambda_ptr, args.lambda_dtype);
       ok = mbar_wait_cluster(&misc->peer_data, 0, abort_flag, 2314) && ok;
-      const bool live0 = live && ok && !*abort_flag;
-      const float4* xrow = reinterpret_cast<const float4*>(xtile) + row;
-      // first pass: sum of squares of A = A1 - lambda A2 (the accumulator and the exchange tile are read again below);
-      // without rms_norm only rstd needs it, and it is gathered in the second pass
-      float ssq = 0.f;
-#pragma unroll
-      for (int c = 0; c < DV / 32; ++c) {
-        if (!args.rms_norm) break;
+      const float4* xrow = reinterpret_cast<const float4*>(xtile) + u * 32 * BM + row;
+      // A = A1 - lambda A2 of one 32-column chunk (the accumulator and the exchange tile are read twice with rms_norm)
+      auto load_a = [&](int c, float (&a)[32]) {
         uint32_t o[32];
-        tmem_ld32(t_o + c * 32, o);
+        tmem_ld32(t_o + u * 128 + c * 32, o);
         tc_wait_ld();
+        float ssq = 0.f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const float4 z = xrow[(c * 8 + i) * BM];
-          const float a0 = __uint_as_float(o[4 * i + 0]) * inv_l - lam * z.x, a1 = __uint_as_float(o[4 * i + 1]) * inv_l - lam * z.y;
-          const float a2 = __uint_as_float(o[4 * i + 2]) * inv_l - lam * z.z, a3 = __uint_as_float(o[4 * i + 3]) * inv_l - lam * z.w;
-          ssq += (a0 * a0 + a1 * a1) + (a2 * a2 + a3 * a3);
+          const float zz[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            a[4 * i + k] = __uint_as_float(o[4 * i + k]) * inv_l - lam * zz[k];
+            ssq += a[4 * i + k] * a[4 * i + k];
+          }
         }
+        return ssq;
+      };
+      float ys = 1.f, ssq = 0.f;
+      auto row_rstd = [&] {
+        misc->ssq[u][row] = ssq;
+        named_bar_sync(1, NUM_SOFTMAX);
+        return rsqrtf((misc->ssq[0][row] + misc->ssq[1][row]) * (1.f / DV) + args.eps);
+      };
+      float rstd = 0.f;
+      if (args.rms_norm) {
+        for (int c = 0; c < 4; ++c) {
+          float a[32];
+          ssq += load_a(c, a);
+        }
+        rstd = row_rstd();
+        ys = args.out_scale * rstd;
       }
-      const float ys = args.rms_norm ? args.out_scale * rsqrtf(ssq * (1.f / DV) + args.eps) : 1.f;
-      float ssq2 = 0.f;
 #pragma unroll
-      for (int c = 0; c < DV / 32; ++c) {
-        uint32_t o[32];
-        tmem_ld32(t_o + c * 32, o);
-        tc_wait_ld();
-        float f[32];
+      for (int c = 0; c < 4; ++c) {
+        float a[32];
+        const float s2 = load_a(c, a);
+        if (!args.rms_norm) ssq += s2;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float4 z = xrow[(c * 8 + i) * BM];
-          const float a0 = __uint_as_float(o[4 * i + 0]) * inv_l - lam * z.x, a1 = __uint_as_float(o[4 * i + 1]) * inv_l - lam * z.y;
-          const float a2 = __uint_as_float(o[4 * i + 2]) * inv_l - lam * z.z, a3 = __uint_as_float(o[4 * i + 3]) * inv_l - lam * z.w;
-          ssq2 += (a0 * a0 + a1 * a1) + (a2 * a2 + a3 * a3);
-          f[4 * i + 0] = a0 * ys; f[4 * i + 1] = a1 * ys; f[4 * i + 2] = a2 * ys; f[4 * i + 3] = a3 * ys;
-        }
-        if (live0) {
+        for (int i = 0; i < 4; ++i) {
+          float f[8];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int col = c * 32 + 8 * i;
-            *reinterpret_cast<uint4*>(args.y + grow * DV + col) =
-                make_uint4(pack2<BF>(f[8 * i + 0], f[8 * i + 1]), pack2<BF>(f[8 * i + 2], f[8 * i + 3]),
-                           pack2<BF>(f[8 * i + 4], f[8 * i + 5]), pack2<BF>(f[8 * i + 6], f[8 * i + 7]));
-            if (args.gain) {
-              const float4 g0 = __ldg(reinterpret_cast<const float4*>(args.gain + col));
-              const float4 g1 = __ldg(reinterpret_cast<const float4*>(args.gain + col + 4));
-              *reinterpret_cast<uint4*>(args.yg + grow * DV + col) =
-                  make_uint4(pack2<BF>(f[8 * i + 0] * g0.x, f[8 * i + 1] * g0.y), pack2<BF>(f[8 * i + 2] * g0.z, f[8 * i + 3] * g0.w),
-                             pack2<BF>(f[8 * i + 4] * g1.x, f[8 * i + 5] * g1.y), pack2<BF>(f[8 * i + 6] * g1.z, f[8 * i + 7] * g1.w));
-            }
+          for (int k = 0; k < 8; ++k) f[k] = a[8 * i + k] * ys;
+          st_swizzled_chunk(out + (c >> 1) * OUT_TILE_BYTES, row, (c & 1) * 4 + i,
+                            make_uint4(pack2<BF>(f[0], f[1]), pack2<BF>(f[2], f[3]), pack2<BF>(f[4], f[5]), pack2<BF>(f[6], f[7])));
+          if (args.gain && live && ok) {
+            const int col = u * 128 + c * 32 + 8 * i;
+            const float4 g0 = __ldg(reinterpret_cast<const float4*>(args.gain + col)), g1 = __ldg(reinterpret_cast<const float4*>(args.gain + col + 4));
+            *reinterpret_cast<uint4*>(args.yg + grow * DV + col) =
+                make_uint4(pack2<BF>(f[0] * g0.x, f[1] * g0.y), pack2<BF>(f[2] * g0.z, f[3] * g0.w), pack2<BF>(f[4] * g1.x, f[5] * g1.y), pack2<BF>(f[6] * g1.z, f[7] * g1.w));
           }
         }
       }
-      if (live0) {
-        args.lse1[grow] = m_run * args.sm_scale + logf(l_run);
-        args.rstd[grow] = rsqrtf(ssq2 * (1.f / DV) + args.eps);
+      if (!args.rms_norm) rstd = row_rstd();
+      store_tiles(&tm_y, out);
+      if (live && ok && !*abort_flag && u == 0) {
+        args.lse1[grow] = m_fin * args.sm_scale + logf(l_fin);
+        args.rstd[grow] = rstd;
       }
     }
   }
 
   // neither CTA leaves while its partner may still arrive on its barriers or write into its shared memory
-  cluster_sync_all();
   tc_fence_before();
+  cluster_sync_all();
   __syncthreads();
-  if (warp == WARP_MMA) {
+  if (warp == WARP_PV) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }

@@ -228,9 +228,9 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
         int nv = args.n - t * SUB;                  // visible key columns: up to the sequence end, up to the diagonal
         if (args.causal) nv = min(nv, q_tile * BM + row - t * SUB + 1);
         ok = softmax_subtile<BF, DROP, DV>(
-            st, t_s, t_o, t, nv, sl2, &misc->m_run[br][row], dr, [&] { named_bar_sync(NB_M + br * 2 + (u ^ 1), 256); },
+            st, t_s, t_s, t_o, t, nv, sl2, &misc->m_run[br][row], dr, [] {}, [&] { named_bar_sync(NB_M + br * 2 + (u ^ 1), 256); },
             [&] { if (t + 1 < nsub) named_bar_arrive(NB_M + br * 2 + u, 256); },
-            [&] { return mbar_wait_warp(&misc->pv_done[br][u ^ 1], ((t - 1) >> 1) & 1, abort_flag, 305 + br, t); });
+            [&] { return mbar_wait_warp(&misc->pv_done[br][u ^ 1], ((t - 1) >> 1) & 1, abort_flag, 305 + br, t); }, [] {}, [] { return true; });
         named_bar_arrive(NB_P + br * 2 + u, 160);
         if (!ok) { t += 2; break; }
       }
