@@ -420,11 +420,13 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
     const float sl2 = args.sm_scale * 1.4426950408889634f;
     const float sg = load_lambda(args.lambda_ptr, args.lambda_dtype) < 0.f ? 1.f : -1.f;   // -sign(lambda)
     // dropout: this thread owns key column kv_tile*BKV + row; a hash covers two consecutive query rows of it
-    const uint32_t dkey1 = DROP ? drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 0u) : 0u;
-    const uint32_t dkey2 = DROP ? drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 1u) : 0u;
-    const uint32_t dcol2 = uint32_t(kv_tile * BKV + row) >> 1;
-    const int dcol_odd = row & 1;
-    const float dscale = DROP ? args.drop_scale : 1.f;
+    DropWalk dw1, dw2;
+    if constexpr (DROP) {
+      const uint32_t col2 = uint32_t(kv_tile * BKV + row) >> 1;
+      dw1 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 0u), col2, row & 1, args.drop_thresh);
+      dw2 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 1u), col2, row & 1, args.drop_thresh);
+    }
+    const f32x2 dscale_2 = pk2(args.drop_scale, args.drop_scale), sgd_2 = pk2(sg * args.drop_scale, sg * args.drop_scale);     // DROP only
     const f32x2 sl2_2 = pk2(sl2, sl2), sg_2 = pk2(sg, sg);
     bool ok = true;
     uint32_t s_ready = 0;            // answers of the early probes (see mbar_probe)
@@ -469,19 +471,13 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
         float pcv[2], d1v[2], d2v[2];
         if constexpr (DROP) {
           // dropped positions contribute neither to dV nor to dP; kept ones carry the factor 1/(1-p)
-          const uint32_t drow2 = uint32_t((i0 + i) * (BQ / 2) + g * 8 + jj);
-          const uint32_t h1 = drop_hash(dkey1, drow2, dcol2), h2 = drop_hash(dkey2, drow2, dcol2);
-          const float p1v[2] = {p10, p11}, p2v[2] = {p20, p21};
-          const float nz[2] = {sb.x, sb.y}, nw[2] = {sb.z, sb.w};
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const float dpv = __uint_as_float(dp[2 * jj + u]);
-            const float k1 = drop_keep(h1, 2 * u + dcol_odd, args.drop_thresh) ? dscale : 0.f;
-            const float k2 = drop_keep(h2, 2 * u + dcol_odd, args.drop_thresh) ? sg * dscale : 0.f;
-            pcv[u] = fmaf(k2, p2v[u], k1 * p1v[u]);
-            d1v[u] = p1v[u] * fmaf(k1, dpv, nz[u]);
-            d2v[u] = p2v[u] * fmaf(k2, dpv, nw[u]);
-          }
+          const uint32_t f1 = drop_at_row(dw1, uint32_t((i0 + i) * (BQ / 2) + g * 8), jj), f2 = drop_at_row(dw2, uint32_t((i0 + i) * (BQ / 2) + g * 8), jj);
+          const uint32_t m10 = drop_mask_first(f1), m11 = drop_mask_second(f1), m20 = drop_mask_first(f2), m21 = drop_mask_second(f2);
+          const uint32_t dp0 = dp[2 * jj], dp1 = dp[2 * jj + 1];
+          up2(fma2(sgd_2, pk2u(__float_as_uint(p20) & m20, __float_as_uint(p21) & m21),
+                   mul2(dscale_2, pk2u(__float_as_uint(p10) & m10, __float_as_uint(p11) & m11))), pcv[0], pcv[1]);
+          up2(mul2(pk2(p10, p11), fma2(dscale_2, pk2u(dp0 & m10, dp1 & m11), pk2(sb.x, sb.y))), d1v[0], d1v[1]);
+          up2(mul2(pk2(p20, p21), fma2(sgd_2, pk2u(dp0 & m20, dp1 & m21), pk2(sb.z, sb.w))), d2v[0], d2v[1]);
         } else {
           const f32x2 p1_2 = pk2(p10, p11), p2_2 = pk2(p20, p21), dp_2 = pk2u(dp[2 * jj], dp[2 * jj + 1]);
           up2(fma2(sg_2, p2_2, p1_2), pcv[0], pcv[1]);
@@ -753,11 +749,11 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
     const float neg_l = br ? sv.y : sv.x;
     const float neg_e = br ? sv.w : sv.z;
     const float sg = (br && !(lam < 0.f)) ? -1.f : 1.f;      // branch 2: -sign(lambda) (|lambda| sits in neg_l, the sign in e)
-    const uint32_t dkey = DROP ? drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), uint32_t(br)) : 0u;
-    const uint32_t drow2 = uint32_t(q_tile * BM + row) >> 1;
-    const int drow_odd = row & 1;
+    DropWalk dw;
+    if constexpr (DROP)
+      dw = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), uint32_t(br)), uint32_t(q_tile * BM + row) >> 1, row & 1, args.drop_thresh);
     const float sgs = DROP ? sg * args.drop_scale : sg;
-    const f32x2 sl2_2 = pk2(sl2, sl2), negl_2 = pk2(neg_l, neg_l), sg_2 = pk2(sg, sg), nege_2 = pk2(neg_e, neg_e);
+    const f32x2 sl2_2 = pk2(sl2, sl2), negl_2 = pk2(neg_l, neg_l), sg_2 = pk2(sgs, sgs), nege_2 = pk2(neg_e, neg_e);
     bool ok = true;
     for (int t = 0; t < nsub; ++t) {
       const int u = t & 1;
@@ -786,17 +782,16 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
         float x0, x1;
         up2(fma2(pk2u(s[2 * i], s[2 * i + 1]), sl2_2, negl_2), x0, x1);
         const float p0 = ex2(x0), p1 = ex2(x1);
+        uint32_t d0 = dp[2 * i], d1 = dp[2 * i + 1];
         if constexpr (DROP) {
           // dP reaches a probability only where it was kept, with the factor 1/(1-p)
-          const uint32_t hh = drop_hash(dkey, drow2, uint32_t(t * (SUB / 2) + half * 16 + i));
-          const float g0 = drop_keep(hh, 2 * drow_odd, args.drop_thresh) ? sgs : 0.f;
-          const float g1 = drop_keep(hh, 2 * drow_odd + 1, args.drop_thresh) ? sgs : 0.f;
-          s[i] = pack2<BF>(p0 * fmaf(g0, __uint_as_float(dp[2 * i]), neg_e), p1 * fmaf(g1, __uint_as_float(dp[2 * i + 1]), neg_e));
-        } else {
-          float r0, r1;
-          up2(mul2(pk2(p0, p1), fma2(pk2u(dp[2 * i], dp[2 * i + 1]), sg_2, nege_2)), r0, r1);
-          s[i] = pack2<BF>(r0, r1);
+          const uint32_t f = drop_at_col(dw, uint32_t(t * (SUB / 2) + half * 16), i);
+          d0 &= drop_mask_first(f);
+          d1 &= drop_mask_second(f);
         }
+        float r0, r1;
+        up2(mul2(pk2(p0, p1), fma2(pk2u(d0, d1), sg_2, nege_2)), r0, r1);
+        s[i] = pack2<BF>(r0, r1);
       }
       tmem_st16(t_s, s);
       tc_wait_st();

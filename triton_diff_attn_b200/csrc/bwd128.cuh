@@ -191,12 +191,15 @@ diffattn_bwd_side128_kernel(const __grid_constant__ CUtensorMap tm_x0, const __g
       neg_l = br ? sv.y : sv.x;
       neg_e = br ? sv.w : sv.z;
     }
-    const f32x2 sl2_2 = pk2(sl2, sl2), sg_2 = pk2(sg, sg);
+    const f32x2 sl2_2 = pk2(sl2, sl2);
     // dropout: `own` is this thread's fixed coordinate (query row on the query side, key column on the key side)
-    const uint32_t dkey = DROP ? drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), uint32_t(br)) : 0u;
-    const uint32_t down2 = uint32_t(tile * BM + row) >> 1;
-    const int down_odd = row & 1;
+    DropWalk dw;
+    if constexpr (DROP) {
+      const uint32_t key = drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), uint32_t(br)), own2 = uint32_t(tile * BM + row) >> 1;
+      dw = QSIDE ? drop_walk_row(key, own2, row & 1, args.drop_thresh) : drop_walk_col(key, own2, row & 1, args.drop_thresh);
+    }
     const float sgs = DROP ? sg * args.drop_scale : sg;
+    const f32x2 sgs_2 = pk2(sgs, sgs);
     bool ok = mbar_wait(&misc->bar_xy, 0, abort_flag, 1300 + g);
     {
       // Y into TMEM: this thread's row, the 64 columns of box g (128 bytes, swizzled in 16-byte chunks) -> 32 columns
@@ -264,15 +267,15 @@ diffattn_bwd_side128_kernel(const __grid_constant__ CUtensorMap tm_x0, const __g
         float x0, x1, v0, v1;
         up2(fma2(pk2u(s[2 * i], s[2 * i + 1]), sl2_2, nl_2), x0, x1);
         const f32x2 p_2 = pk2(ex2(x0), ex2(x1));
-        f32x2 sge_2 = sg_2;
+        uint32_t t0w = tt[2 * i], t1w = tt[2 * i + 1];
         if constexpr (DROP) {
           // streamed index of this pair: key columns on the query side, query rows on the key side
-          const uint32_t str2 = uint32_t((QSIDE ? t : t0 + t) * (SUB / 2) + g * 8 + i);
-          const uint32_t hh = QSIDE ? drop_hash(dkey, down2, str2) : drop_hash(dkey, str2, down2);
-          sge_2 = pk2(drop_keep(hh, QSIDE ? 2 * down_odd : down_odd, args.drop_thresh) ? sgs : 0.f,
-                      drop_keep(hh, QSIDE ? 2 * down_odd + 1 : 2 + down_odd, args.drop_thresh) ? sgs : 0.f);
+          const uint32_t str2 = uint32_t((QSIDE ? t : t0 + t) * (SUB / 2) + g * 8);
+          const uint32_t f = QSIDE ? drop_at_col(dw, str2, i) : drop_at_row(dw, str2, i);
+          t0w &= drop_mask_first(f);
+          t1w &= drop_mask_second(f);
         }
-        up2(mul2(p_2, fma2(sge_2, pk2u(tt[2 * i], tt[2 * i + 1]), ne_2)), v0, v1);
+        up2(mul2(p_2, fma2(sgs_2, pk2u(t0w, t1w), ne_2)), v0, v1);
         ds[i] = pack2<BF>(v0, v1);
       }
       asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
@@ -480,10 +483,13 @@ diffattn_bwd_dv128_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gri
     const uint32_t tb = tmem_base + lane_base;
     const float sl2 = args.sm_scale * 1.4426950408889634f;
     const float sg = load_lambda(args.lambda_ptr, args.lambda_dtype) < 0.f ? 1.f : -1.f;   // -sign(lambda)
-    const uint32_t dkey1 = DROP ? drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 0u) : 0u;
-    const uint32_t dkey2 = DROP ? drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 1u) : 0u;
-    const uint32_t dcol2 = uint32_t(kv_tile * BKV + row) >> 1;
-    const int dcol_odd = row & 1;
+    DropWalk dw1, dw2;
+    if constexpr (DROP) {
+      const uint32_t col2 = uint32_t(kv_tile * BKV + row) >> 1;
+      dw1 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 0u), col2, row & 1, args.drop_thresh);
+      dw2 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 1u), col2, row & 1, args.drop_thresh);
+    }
+    const f32x2 dscale_2 = pk2(args.drop_scale, args.drop_scale), sgd_2 = pk2(sg * args.drop_scale, sg * args.drop_scale);     // DROP only
     const f32x2 sl2_2 = pk2(sl2, sl2), sg_2 = pk2(sg, sg);
     bool ok = mbar_wait(&misc->bar_kv, 0, abort_flag, 1600 + g);
     {
@@ -533,12 +539,14 @@ diffattn_bwd_dv128_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gri
         up2(fma2(pk2u(s2[2 * jj], s2[2 * jj + 1]), sl2_2, pk2(sa.z, sa.w)), x20, x21);
         const f32x2 p1_2 = pk2(ex2(x10), ex2(x11)), p2_2 = pk2(ex2(x20), ex2(x21));
         if constexpr (DROP) {
-          const uint32_t drow2 = uint32_t((i0 + i) * (BQ / 2) + g * 8 + jj);
-          const uint32_t h1 = drop_hash(dkey1, drow2, dcol2), h2 = drop_hash(dkey2, drow2, dcol2);
-          const float ds1 = args.drop_scale, ds2 = sg * args.drop_scale;
-          const f32x2 k1_2 = pk2(drop_keep(h1, dcol_odd, args.drop_thresh) ? ds1 : 0.f, drop_keep(h1, 2 + dcol_odd, args.drop_thresh) ? ds1 : 0.f);
-          const f32x2 k2_2 = pk2(drop_keep(h2, dcol_odd, args.drop_thresh) ? ds2 : 0.f, drop_keep(h2, 2 + dcol_odd, args.drop_thresh) ? ds2 : 0.f);
-          up2(fma2(k2_2, p2_2, mul2(k1_2, p1_2)), v0, v1);
+          const uint32_t r0 = uint32_t((i0 + i) * (BQ / 2) + g * 8);
+          const uint32_t f1 = drop_at_row(dw1, r0, jj), f2 = drop_at_row(dw2, r0, jj);
+          float p10, p11, p20, p21;
+          up2(p1_2, p10, p11);
+          up2(p2_2, p20, p21);
+          const f32x2 k1_2 = pk2u(__float_as_uint(p10) & drop_mask_first(f1), __float_as_uint(p11) & drop_mask_second(f1));
+          const f32x2 k2_2 = pk2u(__float_as_uint(p20) & drop_mask_first(f2), __float_as_uint(p21) & drop_mask_second(f2));
+          up2(fma2(sgd_2, k2_2, mul2(dscale_2, k1_2)), v0, v1);
         } else {
           up2(fma2(sg_2, p2_2, p1_2), v0, v1);
         }

@@ -308,11 +308,13 @@ diffattn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __g
     const float sg = load_lambda(args.lambda_ptr, args.lambda_dtype) < 0.f ? 1.f : -1.f;   // -sign(lambda)
     const bool kv_valid = kv_tile * BKV + row < args.n;    // key rows past the sequence end take no part in dQ
     // dropout: this thread owns key column kv_tile*BKV + row; a hash covers two consecutive query rows of it
-    const uint32_t dkey1 = DROP ? drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 0u) : 0u;
-    const uint32_t dkey2 = DROP ? drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 1u) : 0u;
-    const uint32_t dcol2 = uint32_t(kv_tile * BKV + row) >> 1;
-    const int dcol_odd = row & 1;
-    const float dscale = DROP ? args.drop_scale : 1.f;
+    DropWalk dw1, dw2;
+    if constexpr (DROP) {
+      const uint32_t col2 = uint32_t(kv_tile * BKV + row) >> 1;
+      dw1 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 0u), col2, row & 1, args.drop_thresh);
+      dw2 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 1u), col2, row & 1, args.drop_thresh);
+    }
+    const f32x2 dscale_2 = pk2(args.drop_scale, args.drop_scale), sgd_2 = pk2(sg * args.drop_scale, sg * args.drop_scale);     // DROP only
     uint8_t* const pc_row = smem + OFF_PC + row * 128;
     const int ch0 = ((g * 2) ^ (row & 7)) << 4, ch1 = ((g * 2 + 1) ^ (row & 7)) << 4;
     const f32x2 sl2_2 = pk2(sl2, sl2), sg_2 = pk2(sg, sg);
@@ -363,19 +365,13 @@ diffattn_bwd_fused64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __g
         float pcv[2], d1v[2], d2v[2];
         if constexpr (DROP) {
           // dropped positions contribute neither to dV nor to dP; kept ones carry the factor 1/(1-p)
-          const uint32_t drow2 = uint32_t(qt * (BQ / 2) + g * 8 + jj);
-          const uint32_t h1 = drop_hash(dkey1, drow2, dcol2), h2 = drop_hash(dkey2, drow2, dcol2);
-          const float p1v[2] = {p10, p11}, p2v[2] = {p20, p21};
-          const float nz[2] = {sb.x, sb.y}, nw[2] = {sb.z, sb.w};
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const float dpv = __uint_as_float(dp[2 * jj + u]);
-            const float k1 = drop_keep(h1, 2 * u + dcol_odd, args.drop_thresh) ? dscale : 0.f;
-            const float k2 = drop_keep(h2, 2 * u + dcol_odd, args.drop_thresh) ? sg * dscale : 0.f;
-            pcv[u] = fmaf(k2, p2v[u], k1 * p1v[u]);
-            d1v[u] = p1v[u] * fmaf(k1, dpv, nz[u]);
-            d2v[u] = p2v[u] * fmaf(k2, dpv, nw[u]);
-          }
+          const uint32_t f1 = drop_at_row(dw1, uint32_t(qt * (BQ / 2) + g * 8), jj), f2 = drop_at_row(dw2, uint32_t(qt * (BQ / 2) + g * 8), jj);
+          const uint32_t m10 = drop_mask_first(f1), m11 = drop_mask_second(f1), m20 = drop_mask_first(f2), m21 = drop_mask_second(f2);
+          const uint32_t dp0 = dp[2 * jj], dp1 = dp[2 * jj + 1];
+          up2(fma2(sgd_2, pk2u(__float_as_uint(p20) & m20, __float_as_uint(p21) & m21),
+                   mul2(dscale_2, pk2u(__float_as_uint(p10) & m10, __float_as_uint(p11) & m11))), pcv[0], pcv[1]);
+          up2(mul2(pk2(p10, p11), fma2(dscale_2, pk2u(dp0 & m10, dp1 & m11), pk2(sb.x, sb.y))), d1v[0], d1v[1]);
+          up2(mul2(pk2(p20, p21), fma2(sgd_2, pk2u(dp0 & m20, dp1 & m21), pk2(sb.z, sb.w))), d2v[0], d2v[1]);
         } else {
           const f32x2 p1_2 = pk2(p10, p11), p2_2 = pk2(p20, p21), dp_2 = pk2u(dp[2 * jj], dp[2 * jj + 1]);
           up2(fma2(sg_2, p2_2, p1_2), pcv[0], pcv[1]);

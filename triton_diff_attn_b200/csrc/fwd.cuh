@@ -85,10 +85,6 @@ __device__ __forceinline__ float max3(float a, float b, float c) { return fmaxf(
 struct SoftmaxState {
   float m = -INFINITY, l = 0.f;
 };
-struct DropRow {                 // dropout of one query row: this row's half of every 2 x 2 block hash (see sm100.cuh)
-  uint32_t key, row2, thresh;
-  int row_odd;
-};
 
 // t_s: this thread's lane and the sub-tile's score columns in TMEM; t_p: where its probabilities go (two per column; may be
 // t_s); t_o, O_COLS: the branch's accumulator; nv: visible columns of this row (the rest get -inf, probability 0); loaded:
@@ -97,7 +93,7 @@ struct DropRow {                 // dropout of one query row: this row's half of
 // columns behind t_p may be overwritten (both false: a bounded wait gave up).
 template <bool BF, bool DROP, int O_COLS, class Loaded, class WaitM, class PublishM, class WaitPv, class Mid, class PFree>
 __device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, uint32_t t_p, uint32_t t_o, int t, int nv, float sl2,
-                                                volatile float* m_row, const DropRow& dr, Loaded loaded, WaitM wait_m, PublishM publish_m,
+                                                volatile float* m_row, const DropWalk& dr, Loaded loaded, WaitM wait_m, PublishM publish_m,
                                                 WaitPv wait_pv, Mid mid, PFree p_free) {
   uint32_t sr[64];
   tmem_ld32(t_s, sr);
@@ -160,7 +156,7 @@ __device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, 
   if constexpr (DROP) {
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-      sr[i] &= drop_pair_mask(drop_hash(dr.key, dr.row2, uint32_t(t * 32 + i)), dr.row_odd, dr.thresh);
+      sr[i] &= drop_mask_pair(drop_at_col(dr, uint32_t(t * 32), i));
   }
   const bool ok = p_free();
   tmem_st32(t_p, sr);

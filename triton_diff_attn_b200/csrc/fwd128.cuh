@@ -194,13 +194,9 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
     SoftmaxState st;
     {
       const uint32_t t_s = tmem_base + lane_base + T_S + u * SUB, t_p = tmem_base + lane_base + T_P + u * (SUB / 2);
-      DropRow dr;
-      if constexpr (DROP) {
-        dr.key = drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), uint32_t(br));
-        dr.row2 = uint32_t(q_tile * BM + row) >> 1;
-        dr.thresh = args.drop_thresh;
-        dr.row_odd = row & 1;
-      }
+      DropWalk dr;
+      if constexpr (DROP)
+        dr = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), uint32_t(br)), uint32_t(q_tile * BM + row) >> 1, row & 1, args.drop_thresh);
       int t = u;
       // Warpgroup 1 starts half a pass behind warpgroup 0: in phase, both would be at their exponentials together and
       // leave the exp unit idle together.

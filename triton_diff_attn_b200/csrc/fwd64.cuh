@@ -213,13 +213,9 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
     {
       const uint32_t t_s = tmem_base + lane_base + br * 128 + u * SUB;
       const uint32_t t_o = tmem_base + lane_base + T_O + br * 128;
-      DropRow dr;
-      if constexpr (DROP) {
-        dr.key = drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), uint32_t(br));
-        dr.row2 = uint32_t(q_tile * BM + row) >> 1;
-        dr.thresh = args.drop_thresh;
-        dr.row_odd = row & 1;
-      }
+      DropWalk dr;
+      if constexpr (DROP)
+        dr = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), uint32_t(br)), uint32_t(q_tile * BM + row) >> 1, row & 1, args.drop_thresh);
       int t = u;
       for (; t < nsub; t += 2) {
         ok = mbar_wait_warp(&misc->s_full[br][u], (t >> 1) & 1, abort_flag, 301 + br, t);

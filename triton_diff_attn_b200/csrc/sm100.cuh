@@ -434,14 +434,38 @@ __host__ __device__ __forceinline__ uint32_t mix32(uint32_t h) {
 __host__ __device__ __forceinline__ uint32_t drop_key(uint32_t seed_lo, uint32_t seed_hi, uint32_t bh, uint32_t branch) {
   return mix32(seed_lo ^ mix32(seed_hi + 0x9E3779B9U * (2u * bh + branch + 1u)));
 }
-__device__ __forceinline__ uint32_t drop_hash(uint32_t key, uint32_t row2, uint32_t col2) {
-  return mix32(((row2 << 16) | col2) ^ key);
+// A thread walks along one row or one column, so everything that does not change on its way is folded up front: mix32's
+// first step only mixes the upper half of its argument into the lower one, and becomes one xor per hash.  The two decisions
+// of a hash are compared together: byte b of a 16-bit lane that also holds 0x8000 keeps bit 15 after the subtraction of
+// the threshold iff b >= threshold, and prmt's sign replication turns that bit into a mask.  About 11 instructions per pair
+// instead of 20 (12 with two 32-bit masks).  B2 H16 N2048 D64, p = 0.1: forward 245 -> 170 us, dK/dV 247 -> 217, dQ 228 -> 176.
+struct DropWalk {
+  uint32_t base, sel, sub;     // folded key and fixed coordinate; which two bytes of a hash are this thread's; threshold in both lanes
+};
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
 }
-__device__ __forceinline__ bool drop_keep(uint32_t h, int byte, uint32_t thresh) { return ((h >> (8 * byte)) & 0xffu) >= thresh; }
-// mask for one packed pair of 16-bit probabilities of ONE row (columns 2c, 2c+1): bytes 2*(row&1), 2*(row&1)+1
-__device__ __forceinline__ uint32_t drop_pair_mask(uint32_t h, int row_odd, uint32_t thresh) {
-  const uint32_t f = row_odd ? (h >> 16) : (h & 0xffffu);
-  return ((f & 0xffu) >= thresh ? 0x0000ffffu : 0u) | (f >= (thresh << 8) ? 0xffff0000u : 0u);
+__device__ __forceinline__ DropWalk drop_walk_row(uint32_t key, uint32_t row2, int row_odd, uint32_t thresh) {      // decisions: columns 2c, 2c+1
+  const uint32_t w = (row2 << 16) ^ key;
+  return DropWalk{w ^ (w >> 16), row_odd ? 0x4342u : 0x4140u, thresh * 0x00010001u};
 }
+__device__ __forceinline__ DropWalk drop_walk_col(uint32_t key, uint32_t col2, int col_odd, uint32_t thresh) {      // decisions: rows 2r, 2r+1
+  const uint32_t w = col2 ^ key;
+  return DropWalk{w ^ (w >> 16), col_odd ? 0x4341u : 0x4240u, thresh * 0x00010001u};
+}
+__device__ __forceinline__ uint32_t drop_flags(const DropWalk& w, uint32_t h) {      // the rest of mix32, then the two comparisons
+  h *= 0x7feb352dU; h ^= h >> 15; h *= 0x846ca68bU; h ^= h >> 16;
+  return prmt(h, 0x80808080u, w.sel) - w.sub;
+}
+// flags of block column c0 + i of a row walk, block row r0 + i of a column walk (c0, r0: multiples of a power of two above i)
+__device__ __forceinline__ uint32_t drop_at_col(const DropWalk& w, uint32_t c0, uint32_t i) { return drop_flags(w, (w.base ^ c0) ^ i); }
+__device__ __forceinline__ uint32_t drop_at_row(const DropWalk& w, uint32_t r0, uint32_t i) {
+  return drop_flags(w, (w.base ^ (r0 * 0x00010001u)) ^ (i * 0x00010001u));
+}
+__device__ __forceinline__ uint32_t drop_mask_first(uint32_t flags) { return prmt(flags, flags, 0x9999u); }     // 32-bit masks
+__device__ __forceinline__ uint32_t drop_mask_second(uint32_t flags) { return prmt(flags, flags, 0xBBBBu); }
+__device__ __forceinline__ uint32_t drop_mask_pair(uint32_t flags) { return prmt(flags, flags, 0xBB99u); }      // one packed 16-bit pair
 
 }  // namespace da
