@@ -563,38 +563,48 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
 }
 
 // ------------------------------------------------------------------------------------------------
-// 3. dQ1, dQ2: one CTA = 128 query rows; key/value tiles of 128 rows stream by and are consumed in
-// sub-tiles of 64 rows.  TMEM: S1 two 64-column buffers [0,128), S2 [128,256), dP [256,384),
-// dQ1 [384,448), dQ2 [448,512).  Thread = query row; four warpgroups: two per branch, each forming
-// dS_b = +-P_b (dP - E_b) for 32 of the 64 columns of a sub-tile and writing it as fp16 over the first 16 of its
-// own columns (TMEM A-operand of dS_b K_b).  The MMAs of sub-tile t+1 are issued before
-// the issuer waits for dS(t), so the warpgroups always find their next scores ready.
+// 3. dQ1, dQ2: one CTA = 128 query rows; key/value tiles of 128 rows stream by.  TMEM: S1 [0,128), S2 [128,256),
+// dP [256,384), dQ1 [384,448), dQ2 [448,512).  Thread = query row.
+//
+// Score tiles are 128 columns wide: an M = 128, N = 128 step reads 8 KB of operands in its 64 clocks where two N = 64 steps
+// read 12 KB in 96, and the tensor pipe with its operand reads is what bounds this kernel.  That leaves one buffer per score
+// tile, and each is refilled while the pass that used it is still running: a warpgroup forms dS_b = +-P_b (dP - E_b)
+// of BOTH branches for 32 of the 128 columns, branch 1 first, and writes each as 16-bit over the first 16 of its own score
+// columns (TMEM A-operand of dS_b K_b); dP is read once and stays in registers for both.  So dP(j+1) is issued as soon as
+// dP(j) is in registers, S1(j+1) behind dQ1(j) under branch 2, S2(j+1) behind dQ2(j) under branch 1 of the next tile.
+// The warpgroups of columns 64.. (team 1) run half a branch behind the others, so that one team's exponentials
+// cover the other's waits, loads and stores.
+// B4 H16 N4096 D64: 0.81 -> 0.77 ms (1.9 GHz), 0.935 -> 0.889 ms sustained under the power cap; B8 H16 N2048 D32 418 -> 375 us.
+// (64-column sub-tiles in two buffers, the teams on alternate sub-tiles and the same piecewise refill: 0.950 ms sustained, 390 us.)
 // ------------------------------------------------------------------------------------------------
-// (Separate ring barriers for the V part of a stage, free half a tile before the K part, measured no change here:
-// this kernel does not wait for its loads.  The D = 128 kernels did, see bwd128.cuh.)
 namespace dq64 {
-constexpr int BM = 128, BN = 128, SUB = 64, HD = 64, DV = 128, ST = 2;
+constexpr int BM = 128, BN = 128, HD = 64, DV = 128, KS = 3, VS = 2;
 constexpr int Q_BYTES = BM * HD * 2;        // 16 KB
 constexpr int DA_BYTES = BM * DV * 2;       // 32 KB
 constexpr int K_BYTES = BN * HD * 2;        // 16 KB
 constexpr int V_BYTES = BN * DV * 2;        // 32 KB
-constexpr int STAGE_BYTES = 2 * K_BYTES + V_BYTES;   // 64 KB
 constexpr int OFF_Q1 = 0, OFF_Q2 = Q_BYTES, OFF_DA = 2 * Q_BYTES;
-constexpr int OFF_STAGE = OFF_DA + DA_BYTES;         // 64 KB
-constexpr int OFF_MISC = OFF_STAGE + ST * STAGE_BYTES;
+constexpr int OFF_K = OFF_DA + DA_BYTES;             // 64 KB; stage s: K1 at +s*2*K_BYTES, K2 right after
+constexpr int OFF_V = OFF_K + KS * 2 * K_BYTES;      // 160 KB
+constexpr int OFF_MISC = OFF_V + VS * V_BYTES;       // 224 KB
 constexpr int MISC_BYTES = 1024;
 constexpr int SMEM_BYTES = OFF_MISC + MISC_BYTES + 1024;
-constexpr int NWG = 4;                      // warpgroup w: branch w>>1, columns [32(w&1), 32(w&1)+32) of each sub-tile
+static_assert(SMEM_BYTES <= 227 * 1024, "more shared memory than an SM gives one CTA");
+constexpr int NWG = 4;                      // warpgroup w: columns [32w, 32w+32) of each tile
 constexpr int NUM_THREADS = NWG * 128 + 64;
 constexpr int WARP_TMA = NWG * 4, WARP_MMA = NWG * 4 + 1;
 constexpr int T_S1 = 0, T_S2 = 128, T_DP = 256, T_DQ1 = 384, T_DQ2 = 448;
+// Named barriers: all warpgroups arrive, the MMA warp syncs.  (An mbarrier wait costs the issuer 150-300 clocks while MMAs
+// saturate shared memory; a named barrier a tenth of that.)  NB_START: team 1 waits for team 0's first half branch.
+constexpr int NB_DP = 1, NB_DS1 = 2, NB_DS2 = 3, NB_START = 4, NB_THREADS = NWG * 128 + 32;
 struct Misc {
   uint64_t bar_q;
-  uint64_t full[ST], empty[ST];
-  uint64_t s_full[2][2], ds_full[2][2], acc_full;   // [branch][buffer]
+  uint64_t k_full[KS], k_empty[KS], v_full[VS], v_empty[VS];
+  uint64_t s_full[2], acc_full;   // [branch]; branch 1 stands for dP too
   uint32_t tmem_slot;
   int abort_flag;
 };
+static_assert(sizeof(Misc) <= MISC_BYTES, "misc area too small");
 }  // namespace dq64
 
 template <bool BF, bool DROP>
@@ -614,35 +624,40 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
   const int b_idx = bh / args.h, h_idx = bh % args.h;
   const int nkv_all = args.n_pad / BN;
   const int nkv = (args.causal && q_tile + 1 < nkv_all) ? q_tile + 1 : nkv_all;   // causal: stop at the diagonal tile
-  const int nsub = 2 * nkv;
 
+  // key / value tile j into its ring slot
+  auto load_k = [&](int j) {
+    const int st = j % KS;
+    uint8_t* sp = smem + OFF_K + st * 2 * K_BYTES;
+    mbar_expect_tx(&misc->k_full[st], 2 * K_BYTES);
+    tma_load_4d(sp, &tm_k1, &misc->k_full[st], 0, j * BN, h_idx, b_idx);
+    tma_load_4d(sp + K_BYTES, &tm_k2, &misc->k_full[st], 0, j * BN, h_idx, b_idx);
+  };
+  auto load_v = [&](int j) {
+    const int st = j % VS;
+    uint8_t* sp = smem + OFF_V + st * V_BYTES;
+    mbar_expect_tx(&misc->v_full[st], V_BYTES);
+    tma_load_4d(sp, &tm_v, &misc->v_full[st], 0, j * BN, h_idx, b_idx);
+    tma_load_4d(sp + V_BYTES / 2, &tm_v, &misc->v_full[st], 64, j * BN, h_idx, b_idx);
+  };
   if (warp == WARP_TMA && lane == 0) {
     mbar_init(&misc->bar_q, 1);
-    for (int i = 0; i < ST; ++i) { mbar_init(&misc->full[i], 1); mbar_init(&misc->empty[i], 1); }
-    for (int b = 0; b < 2; ++b)
-      for (int u = 0; u < 2; ++u) { mbar_init(&misc->s_full[b][u], 1); mbar_init(&misc->ds_full[b][u], 256); }
+    for (int i = 0; i < KS; ++i) { mbar_init(&misc->k_full[i], 1); mbar_init(&misc->k_empty[i], 1); }
+    for (int i = 0; i < VS; ++i) { mbar_init(&misc->v_full[i], 1); mbar_init(&misc->v_empty[i], 1); }
+    for (int b = 0; b < 2; ++b) mbar_init(&misc->s_full[b], 1);
     mbar_init(&misc->acc_full, 1);
     misc->abort_flag = 0;
     mbar_init_fence();
-  }
-  // key/value stage j (tile j) into ring slot j % ST
-  auto load_stage = [&](int j) {
-    const int st = j % ST;
-    uint8_t* sp = smem + OFF_STAGE + st * STAGE_BYTES;
-    mbar_expect_tx(&misc->full[st], STAGE_BYTES);
-    tma_load_4d(sp, &tm_k1, &misc->full[st], 0, j * BN, h_idx, b_idx);
-    tma_load_4d(sp + K_BYTES, &tm_k2, &misc->full[st], 0, j * BN, h_idx, b_idx);
-    tma_load_4d(sp + 2 * K_BYTES, &tm_v, &misc->full[st], 0, j * BN, h_idx, b_idx);
-    tma_load_4d(sp + 2 * K_BYTES + V_BYTES / 2, &tm_v, &misc->full[st], 64, j * BN, h_idx, b_idx);
-  };
-  if (warp == WARP_TMA && lane == 0) {
-    // the resident tiles and the first pass over the ring are requested before the CTA-wide setup barrier
+    // the resident tiles and the first pass over the rings are requested before the CTA-wide setup barrier
     mbar_expect_tx(&misc->bar_q, 2 * Q_BYTES + DA_BYTES);
-    tma_load_4d(smem + OFF_Q1, &tm_q1, &misc->bar_q, 0, q_tile * BM, h_idx, b_idx);
-    tma_load_4d(smem + OFF_Q2, &tm_q2, &misc->bar_q, 0, q_tile * BM, h_idx, b_idx);
     tma_load_4d(smem + OFF_DA, &tm_da, &misc->bar_q, 0, q_tile * BM, bh, 0);
     tma_load_4d(smem + OFF_DA + DA_BYTES / 2, &tm_da, &misc->bar_q, 64, q_tile * BM, bh, 0);
-    for (int j = 0; j < ST && j < nkv; ++j) load_stage(j);
+    tma_load_4d(smem + OFF_Q1, &tm_q1, &misc->bar_q, 0, q_tile * BM, h_idx, b_idx);
+    tma_load_4d(smem + OFF_Q2, &tm_q2, &misc->bar_q, 0, q_tile * BM, h_idx, b_idx);
+    for (int j = 0; j < KS && j < nkv; ++j) {
+      if (j < VS) load_v(j);
+      load_k(j);
+    }
   }
   if (warp == WARP_MMA) tmem_alloc(&misc->tmem_slot, 512);
   tc_fence_before();
@@ -652,140 +667,133 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
 
   if (warp == WARP_TMA) {
     if (elect_one()) {
-      for (int j = ST; j < nkv; ++j) {
-        if (!mbar_wait(&misc->empty[j % ST], ((j / ST) & 1) ^ 1, abort_flag, 701, j)) break;
-        load_stage(j);
+      for (int j = VS; j < nkv; ++j) {
+        if (!mbar_wait(&misc->v_empty[j % VS], ((j / VS) & 1) ^ 1, abort_flag, 701, j)) break;
+        load_v(j);
+        if (j < KS) continue;
+        if (!mbar_wait(&misc->k_empty[j % KS], ((j / KS) & 1) ^ 1, abort_flag, 702, j)) break;
+        load_k(j);
       }
     }
   } else if (warp == WARP_MMA) {
-    // One elected thread issues every MMA; descriptors advance by 32-bit adds (see sm100.cuh).  (Three issuing warps
-    // as in the dK/dV kernel were measured here in two forms: split by kind (S | dP | dQ, which needs a committed
-    // mbarrier between the dQ and the S issuer because the score buffers are recycled on the tensor pipe's issue
-    // order): 1.00 against 0.92 ms; split by branch (S_b and dQ_b | dP, which keeps that order): 0.98 ms.  Both
-    // slower: the single issuer stays.  So did two issuing warps, one per branch (S_b and dQ_b, dP of alternate sub-tiles,
-    // no barrier between the two): 0.944 against 0.912 ms -- although the elementwise warps that share a scheduler with
-    // the single issuer finish every sub-tile 130-300 clocks after the others.)
-    if (elect_one()) {
-      constexpr uint32_t IDESC_S = make_idesc(BM, SUB, 0, 0, BF);    // S = Q K^T, dP = dA V^T
-      const uint32_t IDESC_DQ = make_idesc(BM, args.d, 0, 1, BF);    // dQ += dS K   (K MN-major); head dim 32: 32 columns
-      const int kd = args.d >> 4;       // 16-deep MMA steps over the head dim: head dim 32 skips the zero padding
-      constexpr uint32_t HALF = (SUB * 128) >> 4;
-      const uint32_t q1_lo = sdesc_lo(smem_u32(smem + OFF_Q1)), q2_lo = sdesc_lo(smem_u32(smem + OFF_Q2));
-      const uint32_t da_lo = sdesc_lo(smem_u32(smem + OFF_DA));
-      const uint32_t st_lo0 = sdesc_lo(smem_u32(smem + OFF_STAGE));
-      const uint32_t tb = tmem_base;
-      // scores of a 64-row sub-tile into buffer u: S1 and dP (commit -> branch 1), then S2 (commit -> branch 2)
-      auto issue_scores = [&](uint32_t sp_lo, int u) {
+    // One warp issues every MMA.  Every trip makes its barrier calls whether or not a wait gave up, so no warpgroup is left
+    // without its partner.
+    constexpr uint32_t IDESC_S = make_idesc(BM, BN, 0, 0, BF);     // S = Q K^T, dP = dA V^T
+    const uint32_t IDESC_DQ = make_idesc(BM, args.d, 0, 1, BF);    // dQ += dS K   (K MN-major); head dim 32: 32 columns
+    const int kd = args.d >> 4;       // 16-deep MMA steps over the head dim: head dim 32 skips the zero padding
+    const uint32_t q_lo = sdesc_lo(smem_u32(smem + OFF_Q1)), da_lo = sdesc_lo(smem_u32(smem + OFF_DA));
+    const uint32_t k_lo0 = sdesc_lo(smem_u32(smem + OFF_K)), v_lo0 = sdesc_lo(smem_u32(smem + OFF_V));
+    const uint32_t tb = tmem_base;
+    auto issue_dp = [&](int vs) {
+      const uint32_t v_lo = v_lo0 + vs * (V_BYTES >> 4);
 #pragma unroll
-        for (int k = 0; k < HD / 16; ++k)
-          if (k < kd) mma_ss_lo(tb + T_S1 + u * SUB, q1_lo + k * 2, sp_lo + u * HALF + k * 2, IDESC_S, k > 0);
+      for (int k = 0; k < DV / 16; ++k)
+        if (k < 2 * kd)
+          mma_ss_lo(tb + T_DP, da_lo + (k / 4) * ((DA_BYTES / 2) >> 4) + (k % 4) * 2, v_lo + (k / 4) * ((V_BYTES / 2) >> 4) + (k % 4) * 2, IDESC_S,
+                    k > 0);
+      mma_commit(&misc->v_empty[vs]);
+    };
+    auto issue_s = [&](int br, int ks) {
+      const uint32_t k_lo = k_lo0 + ks * ((2 * K_BYTES) >> 4) + br * (K_BYTES >> 4);
 #pragma unroll
-        for (int k = 0; k < DV / 16; ++k)
-          if (k < 2 * kd)
-            mma_ss_lo(tb + T_DP + u * SUB, da_lo + (k / 4) * ((DA_BYTES / 2) >> 4) + (k % 4) * 2,
-                      sp_lo + ((2 * K_BYTES) >> 4) + (k / 4) * ((V_BYTES / 2) >> 4) + u * HALF + (k % 4) * 2, IDESC_S, k > 0);
-        mma_commit(&misc->s_full[0][u]);
+      for (int k = 0; k < HD / 16; ++k)
+        if (k < kd) mma_ss_lo(tb + (br ? T_S2 : T_S1), q_lo + br * (Q_BYTES >> 4) + k * 2, k_lo + k * 2, IDESC_S, k > 0);
+      mma_commit(&misc->s_full[br]);
+    };
+    auto issue_dq = [&](int br, int ks, uint32_t first) {
+      const uint32_t k_lo = k_lo0 + ks * ((2 * K_BYTES) >> 4) + br * (K_BYTES >> 4);
 #pragma unroll
-        for (int k = 0; k < HD / 16; ++k)
-          if (k < kd) mma_ss_lo(tb + T_S2 + u * SUB, q2_lo + k * 2, sp_lo + (K_BYTES >> 4) + u * HALF + k * 2, IDESC_S, k > 0);
-        mma_commit(&misc->s_full[1][u]);
-      };
-      auto issue_dq = [&](int br, uint32_t sp_lo, int u, uint32_t first) {
-#pragma unroll
-        for (int k = 0; k < SUB / 16; ++k)
-          mma_ts_lo(tb + (br ? T_DQ2 : T_DQ1), tb + (br ? T_S2 : T_S1) + u * SUB + (k / 2) * 32 + (k % 2) * 8,
-                    sp_lo + br * (K_BYTES >> 4) + u * HALF + k * (2048 >> 4), IDESC_DQ, k > 0 ? 1u : first);
-      };
-      bool ok = mbar_wait(&misc->bar_q, 0, abort_flag, 801);
-      ok = ok && mbar_wait(&misc->full[0], 0, abort_flag, 802);
-      if (ok) {
-        tc_fence_after();
-        issue_scores(st_lo0, 0);
-        int st = 0;
-        uint32_t st_par = 0;
-        for (int j = 0; j < nkv; ++j) {
-          const uint32_t sp_lo = st_lo0 + st * (STAGE_BYTES >> 4);
-          const uint32_t ph = j & 1;
-          int st_n = st + 1;
-          uint32_t par_n = st_par;
-          if (st_n == ST) { st_n = 0; par_n ^= 1; }
-          // ---- sub-tile 2j (buffer 0): scores of 2j+1 first
-          issue_scores(sp_lo, 1);
-          if (!mbar_wait(&misc->ds_full[0][0], ph, abort_flag, 804, j)) break;
-          tc_fence_after();
-          issue_dq(0, sp_lo, 0, j > 0);
-          if (!mbar_wait(&misc->ds_full[1][0], ph, abort_flag, 805, j)) break;
-          tc_fence_after();
-          issue_dq(1, sp_lo, 0, j > 0);
-          // ---- sub-tile 2j+1 (buffer 1): scores of 2j+2 (next tile) first
-          if (j + 1 < nkv) {
-            if (!mbar_wait(&misc->full[st_n], par_n, abort_flag, 803, j)) break;
-            tc_fence_after();
-            issue_scores(st_lo0 + st_n * (STAGE_BYTES >> 4), 0);
-          }
-          if (!mbar_wait(&misc->ds_full[0][1], ph, abort_flag, 806, j)) break;
-          tc_fence_after();
-          issue_dq(0, sp_lo, 1, 1);
-          if (!mbar_wait(&misc->ds_full[1][1], ph, abort_flag, 807, j)) break;
-          tc_fence_after();
-          issue_dq(1, sp_lo, 1, 1);
-          mma_commit(&misc->empty[st]);
-          st = st_n;
-          st_par = par_n;
-        }
-        mma_commit(&misc->acc_full);
-      }
+      for (int k = 0; k < BN / 16; ++k)
+        mma_ts_lo(tb + (br ? T_DQ2 : T_DQ1), tb + (br ? T_S2 : T_S1) + (k / 2) * 32 + (k % 2) * 8, k_lo + k * (2048 >> 4), IDESC_DQ,
+                  k > 0 ? 1u : first);
+    };
+    bool ok = mbar_wait_warp(&misc->bar_q, 0, abort_flag, 801);
+    ok = ok && mbar_wait_warp(&misc->v_full[0], 0, abort_flag, 802);
+    ok = ok && mbar_wait_warp(&misc->k_full[0], 0, abort_flag, 803);
+    tc_fence_after();
+    if (ok && elect_one()) {
+      issue_dp(0);
+      issue_s(0, 0);
+      issue_s(1, 0);
     }
+    __syncwarp();
+    int ks = 0;                        // K ring slot of tile j
+    uint32_t k_par = 0;                // parity of its pass over the ring
+    for (int j = 0; j < nkv; ++j) {
+      const bool more = j + 1 < nkv;
+      const int vs_n = (j + 1) % VS;
+      int ks_n = ks + 1;
+      if (ks_n == KS) { ks_n = 0; k_par ^= 1; }
+      if (more) {                      // tile j + 1 has landed (waited for under the warpgroups' pass)
+        ok = ok && mbar_wait_warp(&misc->v_full[vs_n], ((j + 1) / VS) & 1, abort_flag, 804, j);
+        ok = ok && mbar_wait_warp(&misc->k_full[ks_n], k_par, abort_flag, 805, j);
+      }
+      named_bar_sync(NB_DP, NB_THREADS);                               // dP(j) is in registers
+      tc_fence_after();
+      if (ok && more && elect_one()) issue_dp(vs_n);
+      __syncwarp();
+      named_bar_sync(NB_DS1, NB_THREADS);                              // dS1(j) written
+      tc_fence_after();
+      if (ok && elect_one()) {
+        issue_dq(0, ks, j > 0);
+        if (more) issue_s(0, ks_n);
+      }
+      __syncwarp();
+      named_bar_sync(NB_DS2, NB_THREADS);                              // dS2(j) written
+      tc_fence_after();
+      if (ok && elect_one()) {
+        issue_dq(1, ks, j > 0);
+        mma_commit(&misc->k_empty[ks]);
+        if (more) issue_s(1, ks_n);
+      }
+      __syncwarp();
+      ks = ks_n;
+    }
+    if (ok && elect_one()) mma_commit(&misc->acc_full);
   } else {
-    const int br = warp >> 3;                      // branch
-    const int half = (warp >> 2) & 1;              // which 32 of the 64 columns of a sub-tile
+    const int g = warp >> 2;                       // columns [32g, 32g + 32) of every tile
     const int row = (warp & 3) * 32 + lane;
     const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
     const uint32_t tb = tmem_base + lane_base;
     const float sl2 = args.sm_scale * 1.4426950408889634f;
     const float lam = load_lambda(args.lambda_ptr, args.lambda_dtype);
-    const size_t grow = size_t(bh) * args.n + size_t(q_tile) * BM + row;
     const float4 sv = stat_row(args.stats, size_t(bh) * args.n_pad + size_t(q_tile) * BM + row);
-    const float neg_l = br ? sv.y : sv.x;
-    const float neg_e = br ? sv.w : sv.z;
-    const float sg = (br && !(lam < 0.f)) ? -1.f : 1.f;      // branch 2: -sign(lambda) (|lambda| sits in neg_l, the sign in e)
-    DropWalk dw;
-    if constexpr (DROP)
-      dw = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), uint32_t(br)), uint32_t(q_tile * BM + row) >> 1, row & 1, args.drop_thresh);
-    const float sgs = DROP ? sg * args.drop_scale : sg;
-    const f32x2 sl2_2 = pk2(sl2, sl2), negl_2 = pk2(neg_l, neg_l), sg_2 = pk2(sgs, sgs), nege_2 = pk2(neg_e, neg_e);
+    const float sg = lam < 0.f ? 1.f : -1.f;       // branch 2: -sign(lambda) (|lambda| sits in its statistics, the sign in e)
+    DropWalk dw1, dw2;
+    if constexpr (DROP) {
+      const uint32_t row2 = uint32_t(q_tile * BM + row) >> 1;
+      dw1 = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 0u), row2, row & 1, args.drop_thresh);
+      dw2 = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 1u), row2, row & 1, args.drop_thresh);
+    }
+    const float dscale = DROP ? args.drop_scale : 1.f;
+    const f32x2 sl2_2 = pk2(sl2, sl2);
+    // (once a wait has given up the loop goes on without waiting, on whatever TMEM holds, and syncs on the named barriers
+    // instead of only arriving: nobody is left waiting and nobody runs ahead)
     bool ok = true;
-    for (int t = 0; t < nsub; ++t) {
-      const int u = t & 1;
-      // own 32 columns; the fp16 result goes to the first 16 of them (the other warpgroup's columns are untouched)
-      const uint32_t t_s = tb + (br ? T_S2 : T_S1) + u * SUB + half * 32;
-      const uint32_t t_dp = tb + T_DP + u * SUB + half * 32;
-      if (!mbar_wait(&misc->s_full[br][u], (t >> 1) & 1, abort_flag, 901 + br, t)) { ok = false; break; }
-      tc_fence_after();
-      uint32_t s[32], dp[32];
-      tmem_ld32(t_s, s);
-      tmem_ld32(t_dp, dp);
-      tc_wait_ld();
-      {
-        // key columns past the sequence end or (causal) right of the diagonal: score -inf, probability 0
-        const int c_first = t * SUB + half * 32;
-        int nv = args.n - c_first;
-        if (args.causal) nv = min(nv, q_tile * BM + row - c_first + 1);
-        if (nv < 32) {
+    auto hand_over = [&](int id) {
+      tc_fence_before();
+      if (ok) named_bar_arrive(id, NB_THREADS);
+      else named_bar_sync(id, NB_THREADS);
+    };
+    const uint32_t t_s1 = tb + T_S1 + g * 32, t_s2 = tb + T_S2 + g * 32, t_dp = tb + T_DP + g * 32;
+    // own 32 columns of one branch: dS over the first 16 of them
+    auto branch = [&](uint32_t* s, const uint32_t* dp, int nv, int j, float neg_l, float neg_e, float sgn, const DropWalk& dw, auto mid) {
+      if (nv < 32) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (i >= nv) s[i] = 0xff800000u;
-        }
+        for (int i = 0; i < 32; ++i)
+          if (i >= nv) s[i] = 0xff800000u;
       }
+      const f32x2 negl_2 = pk2(neg_l, neg_l), nege_2 = pk2(neg_e, neg_e), sg_2 = pk2(sgn * dscale, sgn * dscale);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
+        if (i == 8) mid();
         float x0, x1;
         up2(fma2(pk2u(s[2 * i], s[2 * i + 1]), sl2_2, negl_2), x0, x1);
         const float p0 = ex2(x0), p1 = ex2(x1);
         uint32_t d0 = dp[2 * i], d1 = dp[2 * i + 1];
         if constexpr (DROP) {
           // dP reaches a probability only where it was kept, with the factor 1/(1-p)
-          const uint32_t f = drop_at_col(dw, uint32_t(t * (SUB / 2) + half * 16), i);
+          const uint32_t f = drop_at_col(dw, uint32_t(j * (BN / 2) + g * 16), i);
           d0 &= drop_mask_first(f);
           d1 &= drop_mask_second(f);
         }
@@ -793,21 +801,45 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
         up2(mul2(pk2(p0, p1), fma2(pk2u(d0, d1), sg_2, nege_2)), r0, r1);
         s[i] = pack2<BF>(r0, r1);
       }
-      tmem_st16(t_s, s);
+    };
+    if (g >= 2) named_bar_sync(NB_START, NWG * 128);
+    for (int j = 0; j < nkv; ++j) {
+      // key columns past the sequence end or (causal) right of the diagonal: score -inf, probability 0
+      const int c_first = j * BN + g * 32;
+      int nv = args.n - c_first;
+      if (args.causal) nv = min(nv, q_tile * BM + row - c_first + 1);
+      uint32_t s[32], dp[32];
+      ok = ok && mbar_wait_warp(&misc->s_full[0], j & 1, abort_flag, 901, j);
+      tc_fence_after();
+      tmem_ld32(t_dp, dp);
+      tmem_ld32(t_s1, s);
+      tc_wait_ld();
+      hand_over(NB_DP);
+      branch(s, dp, nv, j, sv.x, sv.z, 1.f, dw1, [&] { if (j == 0 && g < 2) named_bar_arrive(NB_START, NWG * 128); });
+      tmem_st16(t_s1, s);
       tc_wait_st();
-      tc_fence_before();
-      mbar_arrive(&misc->ds_full[br][u]);
+      hand_over(NB_DS1);
+      ok = ok && mbar_wait_warp(&misc->s_full[1], j & 1, abort_flag, 902, j);
+      tc_fence_after();
+      tmem_ld32(t_s2, s);
+      tc_wait_ld();
+      branch(s, dp, nv, j, sv.y, sv.w, sg, dw2, [] {});
+      tmem_st16(t_s2, s);
+      tc_wait_st();
+      hand_over(NB_DS2);
     }
-    ok = ok && mbar_wait(&misc->acc_full, 0, abort_flag, 911 + br);
+    ok = ok && mbar_wait(&misc->acc_full, 0, abort_flag, 911);
     tc_fence_after();
+    const int u = g >> 1, half = g & 1;            // this warpgroup stores columns [32 half, 32 half + 32) of dQ of branch u
     uint32_t acc[32];
-    tmem_ld32(tb + (br ? T_DQ2 : T_DQ1) + half * 32, acc);
+    tmem_ld32(tb + (u ? T_DQ2 : T_DQ1) + half * 32, acc);
     tc_wait_ld();
     // (32 columns per thread: direct 16-byte stores; a shared-memory tile and a TMA store, as the other two
     // kernels use for their wider rows, measured 4 % slower here)
     if (ok && !*abort_flag && half * 32 < args.d && q_tile * BM + row < args.n) {
       const float sc = args.sm_scale;
-      uint4* p = reinterpret_cast<uint4*>((br ? args.dq2 : args.dq1) + grow * args.d + half * 32);
+      const size_t grow = size_t(bh) * args.n + size_t(q_tile) * BM + row;
+      uint4* p = reinterpret_cast<uint4*>((u ? args.dq2 : args.dq1) + grow * args.d + half * 32);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         uint4 v;
