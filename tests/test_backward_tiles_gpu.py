@@ -30,3 +30,45 @@ def test_gradients_at_tile_edges(d, n, causal, p):
         # the repository's fp16 bound.  (A single token is left to the parity tests: its score gradients are zero up to the
         # 16-bit rounding of the saved outputs, so they have no relative error.)
         assert m["rel_l2"] <= 1e-3, (name, m)
+
+
+@pytest.mark.parametrize("b,h,n,d", [(1, 1, 64, 64), (2, 5, 200, 32), (3, 7, 640, 64), (1, 3, 300, 128), (2, 20, 512, 128)])
+def test_overlapping_kernels_equal_separate_ones(b, h, n, d):
+    """In one call the backward's kernels start before the one ahead of them has ended; issued one stage at a time they do not.
+    Several calls follow each other on the stream with fresh inputs in the same buffers, smaller and larger than the chip."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import triton_diff_attn_b200 as pkg
+    from triton_diff_attn_b200 import _lib
+    dev = torch.device("cuda", 0)
+    ins = [t.to(dev) for t in oracle.make_inputs(b, h, n, d, 77)]
+    q1, q2, k1, k2, v, dy = ins
+    lam = torch.tensor([0.5], device=dev)
+    saved = [torch.empty_like(v), torch.empty_like(v)] + [torch.empty((b, h, n), device=dev) for _ in range(3)]
+    grads = [torch.empty_like(t) for t in (q1, q2, k1, k2, v)]
+    dlam = torch.zeros(1, device=dev)
+    p = _lib.new_params()
+    pkg.layers._fill_common(p, q1, q2, k1, k2, v, lam, 0.2, True, saved)
+    ws = torch.empty(_lib.lib.diffattn_workspace_bytes(p), dtype=torch.uint8, device=dev)
+    p.dy, p.dlambda, p.workspace, p.workspace_bytes = dy.data_ptr(), dlam.data_ptr(), ws.data_ptr(), ws.numel()
+    p.dq1, p.dq2, p.dk1, p.dk2, p.dv = (t.data_ptr() for t in grads)
+
+    def rounds(step):
+        out = []
+        for i in range(4):
+            for t, fresh in zip(ins, oracle.make_inputs(b, h, n, d, 200 + i)):
+                t.copy_(fresh)
+            _lib.check(_lib.lib.diffattn_fwd(p), "fwd")
+            step()
+            out += [g.clone() for g in grads]      # right behind the call: whoever follows it must see every gradient complete
+        return out
+
+    def separate():
+        for stage in (_lib.STAGE_PRE, _lib.STAGE_DKDV, _lib.STAGE_DQ):
+            _lib.check(_lib.lib.diffattn_bwd_stages(p, stage), "stage")
+            torch.cuda.synchronize()
+
+    want = rounds(separate)
+    got = rounds(lambda: _lib.check(_lib.lib.diffattn_bwd(p), "bwd"))
+    pkg.device_status(0)
+    assert all(torch.equal(a, w) for a, w in zip(got, want))

@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(256) diffattn_bwd_pre_kernel(const BwdArgs arg
   // as good or better (0.062 ms each).
   constexpr int PRE_ROWS = VPL == 4 ? 2 : 4;
   constexpr int DV = 32 * VPL;
+  griddep_launch();      // the first tensor-core kernel may set itself up; it waits for this one before it reads dA or the statistics
   constexpr float LOG2E = 1.4426950408889634f;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -95,6 +96,14 @@ __global__ void __launch_bounds__(256) diffattn_bwd_pre_kernel(const BwdArgs arg
       z[t] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
 
+  // rows N..n_pad-1 of every (batch, head) in `stats`: neutral values (see BwdArgs::n_pad)
+  if (const int pad = args.n_pad - args.n) {
+    const long long total = args.rows / args.n * pad;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+      const long long bh_i = i / pad;
+      stat_store(args.stats, bh_i * args.n_pad + args.n + (i - bh_i * pad), make_float4(-INFINITY, -INFINITY, 0.f, 0.f));
+    }
+  }
   // PRE_ROWS rows per warp and trip: all their loads are issued before the first reduction, which keeps that many
   // times the bytes in flight per warp (one row per trip ran at 26 % of the DRAM rate: the shuffles of a row's two
   // reductions sat between its loads and the next row's).
@@ -204,16 +213,6 @@ __global__ void __launch_bounds__(256) diffattn_bwd_pre_kernel(const BwdArgs arg
   }
 }
 
-// rows N..n_pad-1 of every (batch, head) in `stats`: neutral values (see BwdArgs::n_pad)
-__global__ void diffattn_bwd_padstats_kernel(const BwdArgs args, int bh_total) {
-  const int pad = args.n_pad - args.n;
-  const long long total = (long long)bh_total * pad;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long bh_i = i / pad;
-    stat_store(args.stats, bh_i * args.n_pad + args.n + (i - bh_i * pad), make_float4(-INFINITY, -INFINITY, 0.f, 0.f));
-  }
-}
-
 // ------------------------------------------------------------------------------------------------
 // 2. dK1, dK2, dV: one CTA = 128 key/value rows of one (batch, head); query tiles of 64 stream by.
 // TMEM: dV [0,128) dK1 [128,192) dK2 [192,256) | scores S1^T [256,320) S2^T [320,384) dP^T [384,448) |
@@ -315,6 +314,8 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
       tma_load_4d(smem + OFF_K2, &tm_k2, &misc->bar_kv, 0, kv_tile * BKV, h_idx, b_idx);
       tma_load_4d(smem + OFF_V, &tm_v, &misc->bar_kv, 0, kv_tile * BKV, h_idx, b_idx);
       tma_load_4d(smem + OFF_V + V_BYTES / 2, &tm_v, &misc->bar_kv, 64, kv_tile * BKV, h_idx, b_idx);
+      griddep_wait();        // dA and the statistics come from the preprocess kernel
+      griddep_launch();      // the dQ kernel depends on nothing else: it may fill the SMs that this grid's last wave leaves idle
       for (int i = 0; i < nq; ++i) {
         const int st = i % ST;
         uint8_t* sp = smem + OFF_STAGE + st * STAGE_BYTES;
@@ -857,6 +858,8 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+  // whoever waits for this grid waits for the one before it too
+  if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) griddep_wait();
 }
 
 }  // namespace da

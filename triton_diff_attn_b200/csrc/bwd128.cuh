@@ -98,6 +98,8 @@ diffattn_bwd_side128_kernel(const __grid_constant__ CUtensorMap tm_x0, const __g
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&misc->tmem_slot);
 
+  // (launched after the dV kernel's every CTA has seen the preprocess kernel complete: nothing to wait for here)
+  if (!QSIDE && threadIdx.x == 0) griddep_launch();
   if (warp == WARP_TMA) {
     if (elect_one()) {
       mbar_expect_tx(&misc->bar_xy, X_BYTES + Y_BYTES);
@@ -311,6 +313,8 @@ diffattn_bwd_side128_kernel(const __grid_constant__ CUtensorMap tm_x0, const __g
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+  // whoever waits for this grid waits for the one before it too
+  if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) griddep_wait();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -398,6 +402,8 @@ diffattn_bwd_dv128_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gri
         tma_load_4d(smem + OFF_K1 + c * 16384, &tm_k1, &misc->bar_kv, c * 64, kv_tile * BKV, h_idx, b_idx);
         tma_load_4d(smem + OFF_K2 + c * 16384, &tm_k2, &misc->bar_kv, c * 64, kv_tile * BKV, h_idx, b_idx);
       }
+      griddep_wait();        // dA and the statistics come from the preprocess kernel
+      griddep_launch();      // the side kernels depend on nothing else
       int qs = 0, as = 0, ts = 0;
       uint32_t qpar = 1, apar = 1, tpar = 1;
       for (int i = 0; i < nq; ++i) {
