@@ -72,3 +72,38 @@ def test_overlapping_kernels_equal_separate_ones(b, h, n, d):
     got = rounds(lambda: _lib.check(_lib.lib.diffattn_bwd(p), "bwd"))
     pkg.device_status(0)
     assert all(torch.equal(a, w) for a, w in zip(got, want))
+
+
+@pytest.mark.parametrize("b,h,n,d,causal,p,gain", [
+    (10, 16, 33, 64, False, 0.0, False),      # one tile per head, just more items than SMs
+    (16, 20, 100, 64, True, 0.25, True),      # one tile per head, three rounds
+    (5, 16, 200, 32, False, 0.0, True),       # two tiles; head dim 32 (one dV store)
+    (5, 20, 385, 64, True, 0.0, False),       # four tiles of unequal cost, backward rounds
+    (3, 25, 300, 64, False, 0.25, True),      # an odd number of tiles: the rings change slots from item to item
+    (4, 40, 257, 32, True, 0.0, True),        # more heads than a causal group holds in one round
+    (2, 80, 129, 64, False, 0.0, True),
+])
+def test_several_tiles_per_cta(b, h, n, d, causal, p, gain):
+    """With more tiles than SMs a CTA works on one tile after the other: outputs and gradients of every head against the oracle."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import triton_diff_attn_b200 as pkg
+    q1, q2, k1, k2, v, dy = oracle.make_inputs(b, h, n, d, 50 + n)
+    # (dropout without the output norm: under a causal mask the first rows keep a key or none, A_1 - lambda A_2 can all but vanish there,
+    # and the norm's 1 / rms then amplifies the 16-bit rounding of the operands in any implementation)
+    lam, seed, rms = torch.tensor([0.5]), 99, p == 0.0
+    g = torch.linspace(0.5, 1.5, 2 * d) if gain else None
+    extra = {"dropout_threshold": pkg.layers.dropout_threshold(p), "dropout_seed": seed} if p else {}
+    want = oracle.backward_closed_form(q1, q2, k1, k2, v, lam, dy, 0.2, rms, causal=causal, gain=g, **extra)
+    dev = torch.device("cuda", 0)
+    leaves = [t.to(dev).requires_grad_(True) for t in (q1, q2, k1, k2, v)]
+    for _ in range(2):
+        y = pkg.MultiheadDiffAttnKernel(*leaves, lam.to(dev), 0.2, rms, causal=causal, dropout_p=p, dropout_seed=seed,
+                                        gain=g.to(dev) if gain else None)
+        grads = torch.autograd.grad(y, leaves, dy.to(dev))
+    pkg.device_status(0)
+    wy = oracle.forward(q1, q2, k1, k2, v, lam, 0.2, rms, causal=causal, gain=g, **extra)["y_gained" if gain else "y"]
+    for name, got, ref in [("y", y.detach(), wy)] + [(k, t, want[k]) for k, t in zip(("dq1", "dq2", "dk1", "dk2", "dv"), grads)]:
+        # the repository's fp16 bound, for each head: a wrong tile must not hide among the others
+        err = (got.float().cpu() - ref.float()).flatten(2).norm(dim=2)
+        assert bool((err <= 2e-3 * ref.float().flatten(2).norm(dim=2)).all()), (name, float((err / ref.float().flatten(2).norm(dim=2)).max()))

@@ -48,6 +48,8 @@ struct BwdArgs {
   float* dq_acc;        // NULL, or workspace fp32 [2][B*H][n_pad][64]: partial sums of dQ1, dQ2 of the single-pass kernel
                         // (bwd_fused64.cuh); zeroed by the preprocess kernel, converted by the finishing kernel
   long long dq_acc_f4;  // its size in float4 units
+  WorkArgs qwork;       // D <= 64: the query tiles of a persistent dQ CTA
+  WorkArgs kwork;       // D <= 64: the key tiles of a persistent dK/dV CTA
 };
 
 // Row statistics, interleaved by pairs of rows so that a kernel that walks two neighbouring rows (the key-side
@@ -214,7 +216,7 @@ __global__ void __launch_bounds__(256) diffattn_bwd_pre_kernel(const BwdArgs arg
 }
 
 // ------------------------------------------------------------------------------------------------
-// 2. dK1, dK2, dV: one CTA = 128 key/value rows of one (batch, head); query tiles of 64 stream by.
+// 2. dK1, dK2, dV: a CTA works on 128 key/value rows of one (batch, head) at a time; query tiles of 64 stream by.
 // TMEM: dV [0,128) dK1 [128,192) dK2 [192,256) | scores S1^T [256,320) S2^T [320,384) dP^T [384,448) |
 // fp16 A-operands dS1^T [448,480) dS2^T [480,512).  Thread = key row; four warpgroups, warpgroup g handles
 // query columns [16g, 16g+16) (more resident warps per scheduler hide the exp-unit and TMEM latencies).  The warpgroups pull their scores into registers and release the score columns at once,
@@ -243,6 +245,7 @@ constexpr int Q_BYTES = BQ * HD * 2;        // 8 KB
 constexpr int DA_BYTES = BQ * DV * 2;       // 16 KB, two boxes of 8 KB
 constexpr int STAT_BYTES = BQ * 16;         // 1 KB
 constexpr int STAGE_BYTES = 2 * Q_BYTES + DA_BYTES + STAT_BYTES;   // 33 KB
+static_assert(STAGE_BYTES % 1024 == 0 && STAGE_BYTES >= V_BYTES && V_BYTES == 2 * K_BYTES && ST == 3, "two ring slots take the epilogue's tiles");
 constexpr int PC_BYTES = BKV * BQ * 2;      // 16 KB per buffer
 constexpr int OFF_K1 = 0, OFF_K2 = K_BYTES, OFF_V = 2 * K_BYTES;
 constexpr int OFF_PC = OFF_V + V_BYTES;                            // 64 KB
@@ -253,13 +256,16 @@ constexpr int SMEM_BYTES = OFF_MISC + MISC_BYTES + 1024;
 constexpr int NWG = 4;                      // elementwise warpgroups; warpgroup g owns query columns [16g, 16g+16)
 constexpr int NUM_THREADS = NWG * 128 + 128;                      // + TMA warp and three MMA-issuing warps, one per scheduler
 constexpr int WARP_TMA = NWG * 4, WARP_MMA = NWG * 4 + 1;         // issuers: WARP_MMA (S^T), +1 (dP^T), +2 (dV, dK)
+// Named barriers: output operands of a tile written (+ tile & 1), its scores in registers, the accumulators of a key tile in
+// registers, its gradients in shared memory.  (A wait on an mbarrier costs an
+// issuer 110-300 clocks even when the phase is long complete, a named barrier a tenth.)
+constexpr int NB_E = 1, NB_SFREE = 3, NB_ACC = 4, NB_STORE = 5;
+constexpr int NB_E_THREADS = NWG * 128 + 32, NB_SFREE_THREADS = NWG * 128 + 64;
 constexpr int T_DV = 0, T_DK1 = 128, T_DK2 = 192, T_S1 = 256, T_S2 = 320, T_DP = 384, T_DS1 = 448, T_DS2 = 480;
 struct Misc {
-  uint64_t bar_kv;
+  uint64_t bar_kv, kv_empty;
   uint64_t full[ST], empty[ST];
   uint64_t s_full;      // scores of a tile written (MMA -> warpgroups)
-  uint64_t s_free;      // scores of a tile are in registers (one arrival per elementwise thread)
-  uint64_t e_done;      // dS^T in TMEM and Pc in shared memory written (one arrival per elementwise thread)
   uint64_t mma_done;    // dV/dK MMAs of a tile completed (operand buffers reusable)
   uint64_t acc_full;
   uint32_t tmem_slot;
@@ -267,7 +273,7 @@ struct Misc {
 };
 }  // namespace dkdv64
 
-template <bool BF, bool DROP>
+template <bool BF, bool DROP, bool LIST>
 __global__ void __launch_bounds__(dkdv64::NUM_THREADS, 1)
 diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_constant__ CUtensorMap tm_q2,
                            const __grid_constant__ CUtensorMap tm_k1, const __grid_constant__ CUtensorMap tm_k2,
@@ -280,20 +286,23 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
   Misc* misc = reinterpret_cast<Misc*>(smem + OFF_MISC);
   volatile int* abort_flag = &misc->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kv_tile = blockIdx.x, bh = blockIdx.y;
-  const int b_idx = bh / args.h, h_idx = bh % args.h;
+  // Persistent: this CTA works on the key tiles of its WorkList one after the other; rings and barriers run on from one to the
+  // next (each role counts along by itself), so the next tile's operands arrive and its first scores are computed under this
+  // tile's last pass and epilogue, and the gradients leave under the next tile's first passes.
+  // Against one CTA per tile: B8 H16 N512 D64 63 -> 58 us, causal 49 -> 42, B32 H16 N128 D64 35 -> 29, B4 H16 N4096 unchanged.
+  // (With dK1 and dK2 staged in the Pc buffers one more ring slot could be refilled early, B32 H16 N128 25 us, but the wait that
+  // the first Pc stores then need sat in the loop over the query tiles and cost it 4 %.)
+  WorkList<LIST> work(args.kwork);
   // the last query tiles may reach past N (zero dA, neutral statistics); under the causal mask only query tiles
-  // from the diagonal on see these keys: tiles i0 .. nq_all-1, visited with the local index i (tile i0 + i)
+  // from the diagonal on see a key tile: tiles i0 .. nq_all-1, visited with the local index i (tile i0 + i)
   const int nq_all = args.n_pad / BQ;
-  const int i0 = args.causal ? kv_tile * (BKV / BQ) : 0;
-  const int nq = nq_all - i0;
+  auto first_q = [&](int kv_tile) { return args.causal ? kv_tile * (BKV / BQ) : 0; };
 
   if (warp == WARP_TMA && lane == 0) {
     mbar_init(&misc->bar_kv, 1);
+    mbar_init(&misc->kv_empty, 2);
     for (int i = 0; i < ST; ++i) { mbar_init(&misc->full[i], 1); mbar_init(&misc->empty[i], 1); }
     mbar_init(&misc->s_full, 2);
-    mbar_init(&misc->s_free, NWG * 128);
-    mbar_init(&misc->e_done, NWG * 128);
     mbar_init(&misc->mma_done, 1);
     mbar_init(&misc->acc_full, 1);
     misc->abort_flag = 0;
@@ -308,110 +317,151 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
   // (Requesting the resident tiles and the first ring pass before the setup barrier, as the forward and the dQ
   // kernel do, measured 3 % slower here.)
   if (warp == WARP_TMA) {
-    if (elect_one()) {
-      mbar_expect_tx(&misc->bar_kv, 2 * K_BYTES + V_BYTES);
-      tma_load_4d(smem + OFF_K1, &tm_k1, &misc->bar_kv, 0, kv_tile * BKV, h_idx, b_idx);
-      tma_load_4d(smem + OFF_K2, &tm_k2, &misc->bar_kv, 0, kv_tile * BKV, h_idx, b_idx);
-      tma_load_4d(smem + OFF_V, &tm_v, &misc->bar_kv, 0, kv_tile * BKV, h_idx, b_idx);
-      tma_load_4d(smem + OFF_V + V_BYTES / 2, &tm_v, &misc->bar_kv, 64, kv_tile * BKV, h_idx, b_idx);
-      griddep_wait();        // dA and the statistics come from the preprocess kernel
-      griddep_launch();      // the dQ kernel depends on nothing else: it may fill the SMs that this grid's last wave leaves idle
-      for (int i = 0; i < nq; ++i) {
-        const int st = i % ST;
-        uint8_t* sp = smem + OFF_STAGE + st * STAGE_BYTES;
-        if (!mbar_wait(&misc->empty[st], ((i / ST) & 1) ^ 1, abort_flag, 401, i)) break;
-        mbar_expect_tx(&misc->full[st], STAGE_BYTES);
-        tma_load_4d(sp, &tm_q1, &misc->full[st], 0, (i0 + i) * BQ, h_idx, b_idx);
-        tma_load_4d(sp + Q_BYTES, &tm_q2, &misc->full[st], 0, (i0 + i) * BQ, h_idx, b_idx);
-        tma_load_4d(sp + 2 * Q_BYTES, &tm_da, &misc->full[st], 0, (i0 + i) * BQ, bh, 0);
-        tma_load_4d(sp + 2 * Q_BYTES + DA_BYTES / 2, &tm_da, &misc->full[st], 64, (i0 + i) * BQ, bh, 0);
-        bulk_load_1d(sp + 2 * Q_BYTES + DA_BYTES, args.stats + (size_t(bh) * args.n_pad + size_t(i0 + i) * BQ), STAT_BYTES,
-                     &misc->full[st]);
+    bool ok = true;
+    int st = 0, it = 0;
+    uint32_t par = 1;                    // parity of an "empty" wait of the ring (the first pass never waits)
+    WorkItem last{0, 0};
+    // Gradients leave through the TMA engine, from the ring slots that the next tile fills second (dK1, dK2) and third (dV).
+    // The engine clips at the tensor's bounds: key rows past the sequence end and, for head dim 32, the padding columns are not
+    // written.
+    auto store = [&](int second) {
+      named_bar_sync(NB_STORE, NB_E_THREADS);
+      if (elect_one()) {
+        if (!*abort_flag) {
+          const uint8_t* dk = smem + OFF_STAGE + second * STAGE_BYTES;
+          const uint8_t* dv = smem + OFF_STAGE + (second + 1) % ST * STAGE_BYTES;
+          tma_store_4d(dv, &tm_dv, 0, last.tile * BKV, last.bh, 0);
+          if (args.d > 32) tma_store_4d(dv + V_BYTES / 2, &tm_dv, 64, last.tile * BKV, last.bh, 0);
+          tma_store_4d(dk, &tm_dk1, 0, last.tile * BKV, last.bh, 0);
+          tma_store_4d(dk + K_BYTES, &tm_dk2, 0, last.tile * BKV, last.bh, 0);
+          tma_store_commit();
+          tma_store_wait_read();
+        }
       }
+      __syncwarp();
+    };
+    for (; work.valid(); ++it, work.next()) {
+      const WorkItem wi = work.item();
+      const int b_idx = wi.bh / args.h, h_idx = wi.bh % args.h, i0 = first_q(wi.tile), nq = nq_all - i0;
+      if (it > 0) ok = ok && mbar_wait_warp(&misc->kv_empty, (it - 1) & 1, abort_flag, 402, it);
+      if (ok && elect_one()) {
+        mbar_expect_tx(&misc->bar_kv, 2 * K_BYTES + V_BYTES);
+        tma_load_4d(smem + OFF_K1, &tm_k1, &misc->bar_kv, 0, wi.tile * BKV, h_idx, b_idx);
+        tma_load_4d(smem + OFF_K2, &tm_k2, &misc->bar_kv, 0, wi.tile * BKV, h_idx, b_idx);
+        tma_load_4d(smem + OFF_V, &tm_v, &misc->bar_kv, 0, wi.tile * BKV, h_idx, b_idx);
+        tma_load_4d(smem + OFF_V + V_BYTES / 2, &tm_v, &misc->bar_kv, 64, wi.tile * BKV, h_idx, b_idx);
+        if (it == 0) {
+          tma_prefetch_desc(&tm_dv); tma_prefetch_desc(&tm_dk1); tma_prefetch_desc(&tm_dk2);
+          griddep_wait();        // dA and the statistics come from the preprocess kernel
+          griddep_launch();      // the dQ kernel depends on nothing else: it may fill the SMs that this grid's last wave leaves idle
+        }
+      }
+      __syncwarp();
+      for (int i = 0; i < nq; ++i) {
+        if (i == 1 && it > 0) store(st);     // (every tile has at least two query tiles)
+        ok = ok && mbar_wait_warp(&misc->empty[st], par, abort_flag, 401, i);
+        if (ok && elect_one()) {
+          uint8_t* sp = smem + OFF_STAGE + st * STAGE_BYTES;
+          mbar_expect_tx(&misc->full[st], STAGE_BYTES);
+          tma_load_4d(sp, &tm_q1, &misc->full[st], 0, (i0 + i) * BQ, h_idx, b_idx);
+          tma_load_4d(sp + Q_BYTES, &tm_q2, &misc->full[st], 0, (i0 + i) * BQ, h_idx, b_idx);
+          tma_load_4d(sp + 2 * Q_BYTES, &tm_da, &misc->full[st], 0, (i0 + i) * BQ, wi.bh, 0);
+          tma_load_4d(sp + 2 * Q_BYTES + DA_BYTES / 2, &tm_da, &misc->full[st], 64, (i0 + i) * BQ, wi.bh, 0);
+          bulk_load_1d(sp + 2 * Q_BYTES + DA_BYTES, args.stats + (size_t(wi.bh) * args.n_pad + size_t(i0 + i) * BQ), STAT_BYTES, &misc->full[st]);
+        }
+        __syncwarp();
+        if (++st == ST) { st = 0; par ^= 1; }
+      }
+      last = wi;
     }
+    store((st + 1) % ST);
   } else if (warp == WARP_MMA || warp == WARP_MMA + 1) {
     // ---- score issuers: warp WARP_MMA issues S1^T and S2^T of every tile, warp WARP_MMA + 1 issues dP^T.
     // MMA issue is spread over three warps on three schedulers (these two and the output issuer below): one warp
     // issuing all 32 MMAs of a tile takes ~300 clocks per tile from the elementwise warps of its scheduler, and
     // every tile waits for that slowest quarter.  One elected thread per warp; descriptors advance by 32-bit adds.
-    if (elect_one()) {
-      const bool is_dp = warp == WARP_MMA + 1;
-      constexpr uint32_t IDESC_S = make_idesc(BKV, BQ, 0, 0, BF);     // S^T = K Q^T, dP^T = V dA^T
-      const uint32_t k1_lo = sdesc_lo(smem_u32(smem + OFF_K1)), k2_lo = sdesc_lo(smem_u32(smem + OFF_K2));
-      const uint32_t v_lo = sdesc_lo(smem_u32(smem + OFF_V));
-      const uint32_t st_lo0 = sdesc_lo(smem_u32(smem + OFF_STAGE));
-      const uint32_t tb = tmem_base;
-      const int kd = args.d >> 4;       // 16-deep MMA steps over the head dim (value width: twice as many): head dim 32 skips the zero padding
-      auto issue_scores = [&](uint32_t sp_lo) {
-        if (!is_dp) {
+    // (Every trip makes its barrier calls whether or not a wait gave up: nobody is left without a partner.)
+    const bool is_dp = warp == WARP_MMA + 1;
+    constexpr uint32_t IDESC_S = make_idesc(BKV, BQ, 0, 0, BF);     // S^T = K Q^T, dP^T = V dA^T
+    const uint32_t k1_lo = sdesc_lo(smem_u32(smem + OFF_K1)), k2_lo = sdesc_lo(smem_u32(smem + OFF_K2));
+    const uint32_t v_lo = sdesc_lo(smem_u32(smem + OFF_V));
+    const uint32_t st_lo0 = sdesc_lo(smem_u32(smem + OFF_STAGE));
+    const uint32_t tb = tmem_base;
+    const int kd = args.d >> 4;       // 16-deep MMA steps over the head dim (value width: twice as many): head dim 32 skips the zero padding
+    auto issue_scores = [&](uint32_t sp_lo) {
+      if (!is_dp) {
 #pragma unroll
-          for (int k = 0; k < HD / 16; ++k)
-            if (k < kd) mma_ss_lo(tb + T_S1, k1_lo + k * 2, sp_lo + k * 2, IDESC_S, k > 0);
+        for (int k = 0; k < HD / 16; ++k)
+          if (k < kd) mma_ss_lo(tb + T_S1, k1_lo + k * 2, sp_lo + k * 2, IDESC_S, k > 0);
 #pragma unroll
-          for (int k = 0; k < HD / 16; ++k)
-            if (k < kd) mma_ss_lo(tb + T_S2, k2_lo + k * 2, sp_lo + (Q_BYTES >> 4) + k * 2, IDESC_S, k > 0);
-        } else {
+        for (int k = 0; k < HD / 16; ++k)
+          if (k < kd) mma_ss_lo(tb + T_S2, k2_lo + k * 2, sp_lo + (Q_BYTES >> 4) + k * 2, IDESC_S, k > 0);
+      } else {
 #pragma unroll
-          for (int k = 0; k < DV / 16; ++k)
-            if (k < 2 * kd)
-              mma_ss_lo(tb + T_DP, v_lo + (k / 4) * ((V_BYTES / 2) >> 4) + (k % 4) * 2,
-                        sp_lo + ((2 * Q_BYTES) >> 4) + (k / 4) * ((DA_BYTES / 2) >> 4) + (k % 4) * 2, IDESC_S, k > 0);
-        }
-        mma_commit(&misc->s_full);        // two arrivals per tile: this warp's and the other score issuer's
-      };
-      bool ok = mbar_wait(&misc->bar_kv, 0, abort_flag, 501);
-      ok = ok && mbar_wait(&misc->full[0], 0, abort_flag, 502);
-      if (ok) {
+        for (int k = 0; k < DV / 16; ++k)
+          if (k < 2 * kd)
+            mma_ss_lo(tb + T_DP, v_lo + (k / 4) * ((V_BYTES / 2) >> 4) + (k % 4) * 2,
+                      sp_lo + ((2 * Q_BYTES) >> 4) + (k / 4) * ((DA_BYTES / 2) >> 4) + (k % 4) * 2, IDESC_S, k > 0);
+      }
+      mma_commit(&misc->s_full);        // two arrivals per tile: this warp's and the other score issuer's
+    };
+    bool ok = true;
+    int st = 0;
+    uint32_t par = 0;
+    for (int it = 0; work.valid(); ++it, work.next()) {
+      const int nq = nq_all - first_q(work.item().tile);
+      ok = ok && mbar_wait_warp(&misc->bar_kv, it & 1, abort_flag, 501, it);
+      for (int i = 0; i < nq; ++i) {
+        ok = ok && mbar_wait_warp(&misc->full[st], par, abort_flag, 502, i);      // under the warpgroups' pass over the tile before
+        if (it > 0 || i > 0) named_bar_sync(NB_SFREE, NB_SFREE_THREADS);          // the scores before these are in registers
         tc_fence_after();
-        issue_scores(st_lo0);
-        int st = 0;
-        uint32_t st_par = 0;
-        for (int i = 0; i + 1 < nq; ++i) {
-          int st_n = st + 1;
-          uint32_t par_n = st_par;
-          if (st_n == ST) { st_n = 0; par_n ^= 1; }
-          if (!mbar_wait(&misc->full[st_n], par_n, abort_flag, 503, i)) break;
-          if (!mbar_wait(&misc->s_free, i & 1, abort_flag, 504, i)) break;    // scores(i) are in registers
-          tc_fence_after();
-          issue_scores(st_lo0 + st_n * (STAGE_BYTES >> 4));
-          st = st_n;
-          st_par = par_n;
+        if (ok && elect_one()) {
+          issue_scores(st_lo0 + st * (STAGE_BYTES >> 4));
+          if (i == nq - 1) mma_commit(&misc->kv_empty);
         }
+        __syncwarp();
+        if (++st == ST) { st = 0; par ^= 1; }
       }
     }
+    named_bar_sync(NB_SFREE, NB_SFREE_THREADS);
   } else if (warp == WARP_MMA + 2) {
     // ---- output issuer: dV += Pc^T dA, dK_b += dS_b^T Q_b of tile i once the warpgroups have written their operands
-    if (elect_one()) {
-      // head dim 32: only the real 64 value columns / 32 head columns are produced
-      const uint32_t IDESC_DV = make_idesc(BKV, 2 * args.d, 0, 1, BF);    // dV += Pc^T dA   (Pc K-major smem, dA MN-major)
-      const uint32_t IDESC_DK = make_idesc(BKV, args.d, 0, 1, BF);        // dK += dS^T Q    (dS^T in TMEM, Q MN-major)
-      const uint32_t pc_lo0 = sdesc_lo(smem_u32(smem + OFF_PC));
-      const uint32_t st_lo0 = sdesc_lo(smem_u32(smem + OFF_STAGE));
-      constexpr uint32_t DA_MN_LBO = ((DA_BYTES / 2) >> 4) << 16;   // dA as MN-major B: 64-column atoms 8 KB apart
-      const uint32_t tb = tmem_base;
-      int st = 0;
+    // head dim 32: only the real 64 value columns / 32 head columns are produced
+    const uint32_t IDESC_DV = make_idesc(BKV, 2 * args.d, 0, 1, BF);    // dV += Pc^T dA   (Pc K-major smem, dA MN-major)
+    const uint32_t IDESC_DK = make_idesc(BKV, args.d, 0, 1, BF);        // dK += dS^T Q    (dS^T in TMEM, Q MN-major)
+    const uint32_t pc_lo0 = sdesc_lo(smem_u32(smem + OFF_PC));
+    const uint32_t st_lo0 = sdesc_lo(smem_u32(smem + OFF_STAGE));
+    constexpr uint32_t DA_MN_LBO = ((DA_BYTES / 2) >> 4) << 16;   // dA as MN-major B: 64-column atoms 8 KB apart
+    const uint32_t tb = tmem_base;
+    int st = 0;
+    for (int it = 0; work.valid(); ++it, work.next()) {
+      const int nq = nq_all - first_q(work.item().tile);
       for (int i = 0; i < nq; ++i) {
         const uint32_t sp_lo = st_lo0 + st * (STAGE_BYTES >> 4);
         const uint32_t pc_lo = pc_lo0 + (i % PCBUF) * (PC_BYTES >> 4);
-        // e_done(i) implies that stage i was loaded and that the score MMAs reading it have completed
-        if (!mbar_wait(&misc->e_done, i & 1, abort_flag, 505, i)) break;
+        // operands of tile i written: stage i was loaded and the score MMAs reading it have completed
+        if (it > 0 && i == 0) named_bar_sync(NB_ACC, NB_E_THREADS);      // the accumulators of the key tile before are in registers
+        named_bar_sync(NB_E + (i & 1), NB_E_THREADS);
         tc_fence_after();
-        const uint32_t first = i > 0;
+        if (elect_one()) {
+          const uint32_t first = i > 0;
 #pragma unroll
-        for (int k = 0; k < BQ / 16; ++k)
-          mma_ss_lo(tb + T_DV, pc_lo + k * 2, sp_lo + ((2 * Q_BYTES) >> 4) + DA_MN_LBO - (1u << 16) + k * (2048 >> 4), IDESC_DV,
-                    k > 0 ? 1u : first);
+          for (int k = 0; k < BQ / 16; ++k)
+            mma_ss_lo(tb + T_DV, pc_lo + k * 2, sp_lo + ((2 * Q_BYTES) >> 4) + DA_MN_LBO - (1u << 16) + k * (2048 >> 4), IDESC_DV,
+                      k > 0 ? 1u : first);
 #pragma unroll
-        for (int k = 0; k < BQ / 16; ++k)
-          mma_ts_lo(tb + T_DK1, tb + T_DS1 + k * 8, sp_lo + k * (2048 >> 4), IDESC_DK, k > 0 ? 1u : first);
+          for (int k = 0; k < BQ / 16; ++k)
+            mma_ts_lo(tb + T_DK1, tb + T_DS1 + k * 8, sp_lo + k * (2048 >> 4), IDESC_DK, k > 0 ? 1u : first);
 #pragma unroll
-        for (int k = 0; k < BQ / 16; ++k)
-          mma_ts_lo(tb + T_DK2, tb + T_DS2 + k * 8, sp_lo + (Q_BYTES >> 4) + k * (2048 >> 4), IDESC_DK, k > 0 ? 1u : first);
-        mma_commit(&misc->mma_done);
-        mma_commit(&misc->empty[st]);
+          for (int k = 0; k < BQ / 16; ++k)
+            mma_ts_lo(tb + T_DK2, tb + T_DS2 + k * 8, sp_lo + (Q_BYTES >> 4) + k * (2048 >> 4), IDESC_DK, k > 0 ? 1u : first);
+          mma_commit(&misc->mma_done);
+          mma_commit(&misc->empty[st]);
+          if (i == nq - 1) mma_commit(&misc->acc_full);
+        }
+        __syncwarp();
         if (++st == ST) st = 0;
       }
-      mma_commit(&misc->acc_full);
     }
   } else {
     const int g = warp >> 2;                       // warpgroup: query columns [16g, 16g+16) of every tile
@@ -420,138 +470,143 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
     const uint32_t tb = tmem_base + lane_base;
     const float sl2 = args.sm_scale * 1.4426950408889634f;
     const float sg = load_lambda(args.lambda_ptr, args.lambda_dtype) < 0.f ? 1.f : -1.f;   // -sign(lambda)
-    // dropout: this thread owns key column kv_tile*BKV + row; a hash covers two consecutive query rows of it
-    DropWalk dw1, dw2;
-    if constexpr (DROP) {
-      const uint32_t col2 = uint32_t(kv_tile * BKV + row) >> 1;
-      dw1 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 0u), col2, row & 1, args.drop_thresh);
-      dw2 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 1u), col2, row & 1, args.drop_thresh);
-    }
     const f32x2 dscale_2 = pk2(args.drop_scale, args.drop_scale), sgd_2 = pk2(sg * args.drop_scale, sg * args.drop_scale);     // DROP only
     const f32x2 sl2_2 = pk2(sl2, sl2), sg_2 = pk2(sg, sg);
+    // (once a wait has given up the loop goes on without waiting, on whatever TMEM holds, and syncs on the named barriers
+    // instead of only arriving: nobody is left waiting and nobody runs ahead)
     bool ok = true;
+    auto hand_over = [&](int id, int threads) {
+      tc_fence_before();
+      if (ok) named_bar_arrive(id, threads);
+      else named_bar_sync(id, threads);
+    };
     uint32_t s_ready = 0;            // answers of the early probes (see mbar_probe)
-    for (int i = 0; i < nq; ++i) {
-      const int st = i % ST;
-      const float4* stats = reinterpret_cast<const float4*>(smem + OFF_STAGE + st * STAGE_BYTES + 2 * Q_BYTES + DA_BYTES) + g * 16;
-      if (!s_ready && !mbar_wait(&misc->s_full, i & 1, abort_flag, 601 + g, i)) { ok = false; break; }
-      tc_fence_after();
-      uint32_t s1[16], s2[16], dp[16];
-      tmem_ld16(tb + T_S1 + g * 16, s1);
-      tmem_ld16(tb + T_S2 + g * 16, s2);
-      tmem_ld16(tb + T_DP + g * 16, dp);
-      tc_wait_ld();
-      tc_fence_before();
-      mbar_arrive(&misc->s_free);
-      if (args.causal) {
-        // this thread's key row sees query columns >= its own index only: the first c0 columns of its 16 are hidden
-        const int c0 = kv_tile * BKV + row - ((i0 + i) * BQ + g * 16);
-        if (c0 > 0) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (j < c0) { s1[j] = 0xff800000u; s2[j] = 0xff800000u; }
-        }
-      }
-      uint32_t pc[8], d1[8], d2[8];
-      // statistics of the next DA_PF / 2 column pairs (see lds_v4): {x0, x1, y0, y1} and {z0, z1, w0, w1}, negated
-      float4 sva[DA_PF / 2], svb[DA_PF / 2];
-#pragma unroll
-      for (int j = 0; j < DA_PF / 2; ++j) { sva[j] = lds_v4(stats + 2 * j); svb[j] = lds_v4(stats + 2 * j + 1); }
-#pragma unroll
-      for (int jj = 0; jj < 8; ++jj) {
-        const float4 sa = sva[jj % (DA_PF / 2)], sb = svb[jj % (DA_PF / 2)];
-        if (jj + DA_PF / 2 < 8) {
-          sva[jj % (DA_PF / 2)] = lds_v4(stats + 2 * (jj + DA_PF / 2));
-          svb[jj % (DA_PF / 2)] = lds_v4(stats + 2 * (jj + DA_PF / 2) + 1);
-        }
-        float x10, x11, x20, x21;
-        up2(fma2(pk2u(s1[2 * jj], s1[2 * jj + 1]), sl2_2, pk2(sa.x, sa.y)), x10, x11);
-        up2(fma2(pk2u(s2[2 * jj], s2[2 * jj + 1]), sl2_2, pk2(sa.z, sa.w)), x20, x21);
-        const float p10 = ex2(x10), p11 = ex2(x11);
-        const float p20 = ex2(x20), p21 = ex2(x21);     // |lam| P2
-        float pcv[2], d1v[2], d2v[2];
-        if constexpr (DROP) {
-          // dropped positions contribute neither to dV nor to dP; kept ones carry the factor 1/(1-p)
-          const uint32_t f1 = drop_at_row(dw1, uint32_t((i0 + i) * (BQ / 2) + g * 8), jj), f2 = drop_at_row(dw2, uint32_t((i0 + i) * (BQ / 2) + g * 8), jj);
-          const uint32_t m10 = drop_mask_first(f1), m11 = drop_mask_second(f1), m20 = drop_mask_first(f2), m21 = drop_mask_second(f2);
-          const uint32_t dp0 = dp[2 * jj], dp1 = dp[2 * jj + 1];
-          up2(fma2(sgd_2, pk2u(__float_as_uint(p20) & m20, __float_as_uint(p21) & m21),
-                   mul2(dscale_2, pk2u(__float_as_uint(p10) & m10, __float_as_uint(p11) & m11))), pcv[0], pcv[1]);
-          up2(mul2(pk2(p10, p11), fma2(dscale_2, pk2u(dp0 & m10, dp1 & m11), pk2(sb.x, sb.y))), d1v[0], d1v[1]);
-          up2(mul2(pk2(p20, p21), fma2(sgd_2, pk2u(dp0 & m20, dp1 & m21), pk2(sb.z, sb.w))), d2v[0], d2v[1]);
-        } else {
-          const f32x2 p1_2 = pk2(p10, p11), p2_2 = pk2(p20, p21), dp_2 = pk2u(dp[2 * jj], dp[2 * jj + 1]);
-          up2(fma2(sg_2, p2_2, p1_2), pcv[0], pcv[1]);
-          up2(mul2(p1_2, add2(dp_2, pk2(sb.x, sb.y))), d1v[0], d1v[1]);
-          up2(mul2(p2_2, fma2(sg_2, dp_2, pk2(sb.z, sb.w))), d2v[0], d2v[1]);
-        }
-        pc[jj] = pack2<BF>(pcv[0], pcv[1]);
-        d1[jj] = pack2<BF>(d1v[0], d1v[1]);
-        d2[jj] = pack2<BF>(d2v[0], d2v[1]);
-      }
-      // The dS^T columns are free once the output MMAs of tile i-1 have completed (mma_done); the Pc buffer of this
-      // tile was last read by tile i-2, whose completion the previous trip waited for.  So the Pc stores and their
-      // proxy fence go first, under the latency of an early look at mma_done (see mbar_probe).
-      static_assert(PCBUF == 2, "the Pc buffer of tile i must be the one tile i-2 used");
-      const uint32_t md_ready = i > 0 ? mbar_probe(&misc->mma_done, (i - 1) & 1) : 1u;
-      // Pc tile [128 key rows][64 query columns] fp16, 128-byte rows, 16-byte chunks XOR-swizzled by row
+    int st = 0;
+    for (; work.valid(); work.next()) {
       {
-        uint8_t* prow = smem + OFF_PC + (i % PCBUF) * PC_BYTES + row * 128;
+        // (nq is even, so the per-tile barriers' phases have parity i & 1 in every key tile)
+        const WorkItem wi = work.item();
+        const int kv_tile = wi.tile, i0 = first_q(kv_tile), nq = nq_all - i0;
+        // dropout: this thread owns key column kv_tile*BKV + row; a hash covers two consecutive query rows of it
+        DropWalk dw1, dw2;
+        if constexpr (DROP) {
+          const uint32_t col2 = uint32_t(kv_tile * BKV + row) >> 1;
+          dw1 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(wi.bh), 0u), col2, row & 1, args.drop_thresh);
+          dw2 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(wi.bh), 1u), col2, row & 1, args.drop_thresh);
+        }
+        for (int i = 0; i < nq; ++i) {
+          const float4* stats = reinterpret_cast<const float4*>(smem + OFF_STAGE + st * STAGE_BYTES + 2 * Q_BYTES + DA_BYTES) + g * 16;
+          if (!__all_sync(0xffffffffu, s_ready)) ok = ok && mbar_wait_warp(&misc->s_full, i & 1, abort_flag, 601 + g, i);
+          tc_fence_after();
+          uint32_t s1[16], s2[16], dp[16];
+          tmem_ld16(tb + T_S1 + g * 16, s1);
+          tmem_ld16(tb + T_S2 + g * 16, s2);
+          tmem_ld16(tb + T_DP + g * 16, dp);
+          tc_wait_ld();
+          hand_over(NB_SFREE, NB_SFREE_THREADS);
+          if (args.causal) {
+            // this thread's key row sees query columns >= its own index only: the first c0 columns of its 16 are hidden
+            const int c0 = row - (i * BQ + g * 16);          // kv_tile * BKV = i0 * BQ
+            if (c0 > 0) {
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int chunk = (g * 2 + c) ^ (row & 7);
-          *reinterpret_cast<uint4*>(prow + chunk * 16) = make_uint4(pc[4 * c], pc[4 * c + 1], pc[4 * c + 2], pc[4 * c + 3]);
+              for (int j = 0; j < 16; ++j)
+                if (j < c0) { s1[j] = 0xff800000u; s2[j] = 0xff800000u; }
+            }
+          }
+          uint32_t pc[8], d1[8], d2[8];
+          // statistics of the next DA_PF / 2 column pairs (see lds_v4): {x0, x1, y0, y1} and {z0, z1, w0, w1}, negated
+          float4 sva[DA_PF / 2], svb[DA_PF / 2];
+#pragma unroll
+          for (int j = 0; j < DA_PF / 2; ++j) { sva[j] = lds_v4(stats + 2 * j); svb[j] = lds_v4(stats + 2 * j + 1); }
+#pragma unroll
+          for (int jj = 0; jj < 8; ++jj) {
+            const float4 sa = sva[jj % (DA_PF / 2)], sb = svb[jj % (DA_PF / 2)];
+            if (jj + DA_PF / 2 < 8) {
+              sva[jj % (DA_PF / 2)] = lds_v4(stats + 2 * (jj + DA_PF / 2));
+              svb[jj % (DA_PF / 2)] = lds_v4(stats + 2 * (jj + DA_PF / 2) + 1);
+            }
+            float x10, x11, x20, x21;
+            up2(fma2(pk2u(s1[2 * jj], s1[2 * jj + 1]), sl2_2, pk2(sa.x, sa.y)), x10, x11);
+            up2(fma2(pk2u(s2[2 * jj], s2[2 * jj + 1]), sl2_2, pk2(sa.z, sa.w)), x20, x21);
+            const float p10 = ex2(x10), p11 = ex2(x11);
+            const float p20 = ex2(x20), p21 = ex2(x21);     // |lam| P2
+            float pcv[2], d1v[2], d2v[2];
+            if constexpr (DROP) {
+              // dropped positions contribute neither to dV nor to dP; kept ones carry the factor 1/(1-p)
+              const uint32_t f1 = drop_at_row(dw1, uint32_t((i0 + i) * (BQ / 2) + g * 8), jj), f2 = drop_at_row(dw2, uint32_t((i0 + i) * (BQ / 2) + g * 8), jj);
+              const uint32_t m10 = drop_mask_first(f1), m11 = drop_mask_second(f1), m20 = drop_mask_first(f2), m21 = drop_mask_second(f2);
+              const uint32_t dp0 = dp[2 * jj], dp1 = dp[2 * jj + 1];
+              up2(fma2(sgd_2, pk2u(__float_as_uint(p20) & m20, __float_as_uint(p21) & m21),
+                       mul2(dscale_2, pk2u(__float_as_uint(p10) & m10, __float_as_uint(p11) & m11))), pcv[0], pcv[1]);
+              up2(mul2(pk2(p10, p11), fma2(dscale_2, pk2u(dp0 & m10, dp1 & m11), pk2(sb.x, sb.y))), d1v[0], d1v[1]);
+              up2(mul2(pk2(p20, p21), fma2(sgd_2, pk2u(dp0 & m20, dp1 & m21), pk2(sb.z, sb.w))), d2v[0], d2v[1]);
+            } else {
+              const f32x2 p1_2 = pk2(p10, p11), p2_2 = pk2(p20, p21), dp_2 = pk2u(dp[2 * jj], dp[2 * jj + 1]);
+              up2(fma2(sg_2, p2_2, p1_2), pcv[0], pcv[1]);
+              up2(mul2(p1_2, add2(dp_2, pk2(sb.x, sb.y))), d1v[0], d1v[1]);
+              up2(mul2(p2_2, fma2(sg_2, dp_2, pk2(sb.z, sb.w))), d2v[0], d2v[1]);
+            }
+            pc[jj] = pack2<BF>(pcv[0], pcv[1]);
+            d1[jj] = pack2<BF>(d1v[0], d1v[1]);
+            d2[jj] = pack2<BF>(d2v[0], d2v[1]);
+          }
+          // The dS^T columns are free once the output MMAs of tile i-1 have completed (mma_done); the Pc buffer of this
+          // tile was last read by tile i-2, whose completion the previous trip waited for.  So the Pc stores and their
+          // proxy fence go first, under the latency of an early look at mma_done (see mbar_probe).
+          static_assert(PCBUF == 2, "the Pc buffer of tile i must be the one tile i-2 used");
+          const uint32_t md_ready = i > 0 ? mbar_probe(&misc->mma_done, (i - 1) & 1) : 1u;
+          // Pc tile [128 key rows][64 query columns] fp16, 128-byte rows, 16-byte chunks XOR-swizzled by row
+          {
+            uint8_t* prow = smem + OFF_PC + (i % PCBUF) * PC_BYTES + row * 128;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              const int chunk = (g * 2 + c) ^ (row & 7);
+              *reinterpret_cast<uint4*>(prow + chunk * 16) = make_uint4(pc[4 * c], pc[4 * c + 1], pc[4 * c + 2], pc[4 * c + 3]);
+            }
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          if (i > 0) {
+            if (!__all_sync(0xffffffffu, md_ready)) ok = ok && mbar_wait_warp(&misc->mma_done, (i - 1) & 1, abort_flag, 605 + g, i);
+            tc_fence_after();
+          }
+          s_ready = i + 1 < nq ? mbar_probe(&misc->s_full, (i + 1) & 1) : 0u;
+          // 8 packed columns per warpgroup: the 32x32b.x8 shape
+          asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                       ::"r"(tb + T_DS1 + g * 8), "r"(d1[0]), "r"(d1[1]), "r"(d1[2]), "r"(d1[3]), "r"(d1[4]), "r"(d1[5]), "r"(d1[6]), "r"(d1[7]) : "memory");
+          asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                       ::"r"(tb + T_DS2 + g * 8), "r"(d2[0]), "r"(d2[1]), "r"(d2[2]), "r"(d2[3]), "r"(d2[4]), "r"(d2[5]), "r"(d2[6]), "r"(d2[7]) : "memory");
+          tc_wait_st();
+          hand_over(NB_E + (i & 1), NB_E_THREADS);
+          if (++st == ST) st = 0;
         }
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      if (i > 0) {
-        if (!md_ready && !mbar_wait(&misc->mma_done, (i - 1) & 1, abort_flag, 605 + g, i)) { ok = false; break; }
-        tc_fence_after();
-      }
-      s_ready = i + 1 < nq ? mbar_probe(&misc->s_full, (i + 1) & 1) : 0u;
-      // 8 packed columns per warpgroup: the 32x32b.x8 shape
-      asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                   ::"r"(tb + T_DS1 + g * 8), "r"(d1[0]), "r"(d1[1]), "r"(d1[2]), "r"(d1[3]), "r"(d1[4]), "r"(d1[5]), "r"(d1[6]), "r"(d1[7]) : "memory");
-      asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                   ::"r"(tb + T_DS2 + g * 8), "r"(d2[0]), "r"(d2[1]), "r"(d2[2]), "r"(d2[3]), "r"(d2[4]), "r"(d2[5]), "r"(d2[6]), "r"(d2[7]) : "memory");
-      tc_wait_st();
-      tc_fence_before();
-      mbar_arrive(&misc->e_done);
-    }
-    ok = ok && mbar_wait(&misc->acc_full, 0, abort_flag, 611 + g);
-    tc_fence_after();
-    // warpgroup g reads accumulator columns [64g, 64g+64): g = 0,1 -> the two halves of dV, g = 2 -> dK1, g = 3 -> dK2
-    uint32_t acc[64];
-    tmem_ld32(tb + g * 64, acc);
-    tmem_ld32(tb + g * 64 + 32, acc + 32);
-    tc_wait_ld();
-    // The gradients leave through shared memory and the TMA engine (row-per-thread global stores of 16-byte
-    // pieces are several times slower): each warpgroup lays its 64 columns into a swizzled [128][64] tile over
-    // the resident K1 / K2 / V tiles, which no MMA reads any more, and one of its threads stores the tile.
-    // The engine clips at the tensor's bounds: key rows past the sequence end and, for head dim 32, the
-    // padding columns are not written.
-    {
-      const float s = g < 2 ? 1.f : args.sm_scale;
-      uint8_t* tile = smem + ((g + 2) & 3) * K_BYTES;     // g = 0,1 -> the two halves of V; 2 -> K1; 3 -> K2
+      work.forget();
+      ok = ok && mbar_wait_warp(&misc->acc_full, work.round & 1, abort_flag, 611 + g);
+      tc_fence_after();
+      // warpgroup g reads accumulator columns [64g, 64g+64): g = 0,1 -> the two halves of dV, g = 2 -> dK1, g = 3 -> dK2
+      uint32_t acc[64];
+      tmem_ld32(tb + g * 64, acc);
+      tmem_ld32(tb + g * 64 + 32, acc + 32);
+      tc_wait_ld();
+      if (work.has_next()) hand_over(NB_ACC, NB_E_THREADS);
+      // The gradients leave through shared memory and the TMA engine (row-per-thread global stores of 16-byte
+      // pieces are several times slower): each warpgroup lays its 64 columns into a swizzled [128][64] tile over buffers that
+      // no MMA reads any more and the next tile does not fill at once, and the TMA warp stores the tiles.
+      {
+        const float s = g < 2 ? 1.f : args.sm_scale;
+        // g = 0, 1: the halves of dV in the ring slot that is filled third from here; 2, 3: dK1, dK2 in the one filled second
+        uint8_t* tile = smem + OFF_STAGE + (st + (g < 2 ? 2 : 1)) % ST * STAGE_BYTES + (g & 1) * K_BYTES;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        uint4 v;
-        v.x = pack2<BF>(__uint_as_float(acc[8 * i + 0]) * s, __uint_as_float(acc[8 * i + 1]) * s);
-        v.y = pack2<BF>(__uint_as_float(acc[8 * i + 2]) * s, __uint_as_float(acc[8 * i + 3]) * s);
-        v.z = pack2<BF>(__uint_as_float(acc[8 * i + 4]) * s, __uint_as_float(acc[8 * i + 5]) * s);
-        v.w = pack2<BF>(__uint_as_float(acc[8 * i + 6]) * s, __uint_as_float(acc[8 * i + 7]) * s);
-        st_swizzled_chunk(tile, row, i, v);
-      }
-      fence_proxy_async_smem();
-      named_bar_sync(1 + g, 128);
-      const int dv_real = 2 * args.d;
-      if ((warp & 3) == 0 && elect_one()) {
-        if (!*abort_flag && (g != 1 || dv_real > 64)) {
-          const CUtensorMap* map = g < 2 ? &tm_dv : (g == 2 ? &tm_dk1 : &tm_dk2);
-          tma_store_4d(tile, map, g == 1 ? 64 : 0, kv_tile * BKV, bh, 0);
-          tma_store_commit();
-          tma_store_wait_read();
+        for (int i = 0; i < 8; ++i) {
+          uint4 v;
+          v.x = pack2<BF>(__uint_as_float(acc[8 * i + 0]) * s, __uint_as_float(acc[8 * i + 1]) * s);
+          v.y = pack2<BF>(__uint_as_float(acc[8 * i + 2]) * s, __uint_as_float(acc[8 * i + 3]) * s);
+          v.z = pack2<BF>(__uint_as_float(acc[8 * i + 4]) * s, __uint_as_float(acc[8 * i + 5]) * s);
+          v.w = pack2<BF>(__uint_as_float(acc[8 * i + 6]) * s, __uint_as_float(acc[8 * i + 7]) * s);
+          st_swizzled_chunk(tile, row, i, v);
         }
+        fence_proxy_async_smem();
+        hand_over(NB_STORE, NB_E_THREADS);
       }
     }
   }
@@ -564,7 +619,7 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
 }
 
 // ------------------------------------------------------------------------------------------------
-// 3. dQ1, dQ2: one CTA = 128 query rows; key/value tiles of 128 rows stream by.  TMEM: S1 [0,128), S2 [128,256),
+// 3. dQ1, dQ2: a CTA works on 128 query rows at a time; key/value tiles of 128 rows stream by.  TMEM: S1 [0,128), S2 [128,256),
 // dP [256,384), dQ1 [384,448), dQ2 [448,512).  Thread = query row.
 //
 // Score tiles are 128 columns wide: an M = 128, N = 128 step reads 8 KB of operands in its 64 clocks where two N = 64 steps
@@ -596,10 +651,11 @@ constexpr int NUM_THREADS = NWG * 128 + 64;
 constexpr int WARP_TMA = NWG * 4, WARP_MMA = NWG * 4 + 1;
 constexpr int T_S1 = 0, T_S2 = 128, T_DP = 256, T_DQ1 = 384, T_DQ2 = 448;
 // Named barriers: all warpgroups arrive, the MMA warp syncs.  (An mbarrier wait costs the issuer 150-300 clocks while MMAs
-// saturate shared memory; a named barrier a tenth of that.)  NB_START: team 1 waits for team 0's first half branch.
-constexpr int NB_DP = 1, NB_DS1 = 2, NB_DS2 = 3, NB_START = 4, NB_THREADS = NWG * 128 + 32;
+// saturate shared memory; a named barrier a tenth of that.)  NB_START: team 1 waits for team 0's first half branch.  NB_ACC: the
+// accumulators of a tile are in registers.
+constexpr int NB_DP = 1, NB_DS1 = 2, NB_DS2 = 3, NB_START = 4, NB_ACC = 5, NB_THREADS = NWG * 128 + 32;
 struct Misc {
-  uint64_t bar_q;
+  uint64_t bar_q, q_empty;
   uint64_t k_full[KS], k_empty[KS], v_full[VS], v_empty[VS];
   uint64_t s_full[2], acc_full;   // [branch]; branch 1 stands for dP too
   uint32_t tmem_slot;
@@ -608,7 +664,7 @@ struct Misc {
 static_assert(sizeof(Misc) <= MISC_BYTES, "misc area too small");
 }  // namespace dq64
 
-template <bool BF, bool DROP>
+template <bool BF, bool DROP, bool LIST>
 __global__ void __launch_bounds__(dq64::NUM_THREADS, 1)
 diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_constant__ CUtensorMap tm_q2,
                          const __grid_constant__ CUtensorMap tm_k1, const __grid_constant__ CUtensorMap tm_k2,
@@ -620,29 +676,34 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
   Misc* misc = reinterpret_cast<Misc*>(smem + OFF_MISC);
   volatile int* abort_flag = &misc->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // causal: the later a query tile, the more keys it sees -- the heaviest tiles are launched first so that the grid's tail is light
-  const int q_tile = args.causal ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x), bh = blockIdx.y;
-  const int b_idx = bh / args.h, h_idx = bh % args.h;
-  const int nkv_all = args.n_pad / BN;
-  const int nkv = (args.causal && q_tile + 1 < nkv_all) ? q_tile + 1 : nkv_all;   // causal: stop at the diagonal tile
-
+  // Persistent: this CTA works on the tiles of its WorkList one after the other; the rings and barriers run on from tile to tile
+  // (each role counts along by itself), so the next tile's operands arrive and its first scores are computed under this
+  // tile's last pass and epilogue.
+  // Against one CTA per tile: B8 H16 N2048 D32 380 -> 353 us, B8 H16 N512 D64 47 -> 41, B4 H16 N4096 D64 886 -> 871 sustained.
+  WorkList<LIST> work(args.qwork);
   // key / value tile j into its ring slot
-  auto load_k = [&](int j) {
-    const int st = j % KS;
+  auto load_k = [&](int st, int j, int h_idx, int b_idx) {
     uint8_t* sp = smem + OFF_K + st * 2 * K_BYTES;
     mbar_expect_tx(&misc->k_full[st], 2 * K_BYTES);
     tma_load_4d(sp, &tm_k1, &misc->k_full[st], 0, j * BN, h_idx, b_idx);
     tma_load_4d(sp + K_BYTES, &tm_k2, &misc->k_full[st], 0, j * BN, h_idx, b_idx);
   };
-  auto load_v = [&](int j) {
-    const int st = j % VS;
+  auto load_v = [&](int st, int j, int h_idx, int b_idx) {
     uint8_t* sp = smem + OFF_V + st * V_BYTES;
     mbar_expect_tx(&misc->v_full[st], V_BYTES);
     tma_load_4d(sp, &tm_v, &misc->v_full[st], 0, j * BN, h_idx, b_idx);
     tma_load_4d(sp + V_BYTES / 2, &tm_v, &misc->v_full[st], 64, j * BN, h_idx, b_idx);
   };
+  auto load_q = [&](int q_tile, int bh, int h_idx, int b_idx) {
+    mbar_expect_tx(&misc->bar_q, 2 * Q_BYTES + DA_BYTES);
+    tma_load_4d(smem + OFF_DA, &tm_da, &misc->bar_q, 0, q_tile * BM, bh, 0);
+    tma_load_4d(smem + OFF_DA + DA_BYTES / 2, &tm_da, &misc->bar_q, 64, q_tile * BM, bh, 0);
+    tma_load_4d(smem + OFF_Q1, &tm_q1, &misc->bar_q, 0, q_tile * BM, h_idx, b_idx);
+    tma_load_4d(smem + OFF_Q2, &tm_q2, &misc->bar_q, 0, q_tile * BM, h_idx, b_idx);
+  };
   if (warp == WARP_TMA && lane == 0) {
     mbar_init(&misc->bar_q, 1);
+    mbar_init(&misc->q_empty, 1);
     for (int i = 0; i < KS; ++i) { mbar_init(&misc->k_full[i], 1); mbar_init(&misc->k_empty[i], 1); }
     for (int i = 0; i < VS; ++i) { mbar_init(&misc->v_full[i], 1); mbar_init(&misc->v_empty[i], 1); }
     for (int b = 0; b < 2; ++b) mbar_init(&misc->s_full[b], 1);
@@ -650,14 +711,12 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
     misc->abort_flag = 0;
     mbar_init_fence();
     // the resident tiles and the first pass over the rings are requested before the CTA-wide setup barrier
-    mbar_expect_tx(&misc->bar_q, 2 * Q_BYTES + DA_BYTES);
-    tma_load_4d(smem + OFF_DA, &tm_da, &misc->bar_q, 0, q_tile * BM, bh, 0);
-    tma_load_4d(smem + OFF_DA + DA_BYTES / 2, &tm_da, &misc->bar_q, 64, q_tile * BM, bh, 0);
-    tma_load_4d(smem + OFF_Q1, &tm_q1, &misc->bar_q, 0, q_tile * BM, h_idx, b_idx);
-    tma_load_4d(smem + OFF_Q2, &tm_q2, &misc->bar_q, 0, q_tile * BM, h_idx, b_idx);
-    for (int j = 0; j < KS && j < nkv; ++j) {
-      if (j < VS) load_v(j);
-      load_k(j);
+    const WorkItem wi = work.item();
+    const int nkv = key_tiles(args.causal, args.n, wi.tile), b_idx = wi.bh / args.h, h_idx = wi.bh % args.h;
+    load_q(wi.tile, wi.bh, h_idx, b_idx);
+    for (int j = 0; j < VS && j < nkv; ++j) {
+      load_v(j, j, h_idx, b_idx);
+      load_k(j, j, h_idx, b_idx);
     }
   }
   if (warp == WARP_MMA) tmem_alloc(&misc->tmem_slot, 512);
@@ -668,12 +727,29 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
 
   if (warp == WARP_TMA) {
     if (elect_one()) {
-      for (int j = VS; j < nkv; ++j) {
-        if (!mbar_wait(&misc->v_empty[j % VS], ((j / VS) & 1) ^ 1, abort_flag, 701, j)) break;
-        load_v(j);
-        if (j < KS) continue;
-        if (!mbar_wait(&misc->k_empty[j % KS], ((j / KS) & 1) ^ 1, abort_flag, 702, j)) break;
-        load_k(j);
+      bool ok = true;
+      int ks = 0, vs = 0;                 // ring slots; the parity bits are those of an "empty" wait (a first pass never waits)
+      uint32_t k_par = 1, v_par = 1;
+      for (int it = 0; ok && work.valid(); ++it, work.next()) {
+        const WorkItem wi = work.item();
+        const int nkv = key_tiles(args.causal, args.n, wi.tile), b_idx = wi.bh / args.h, h_idx = wi.bh % args.h;
+        if (it > 0) {
+          ok = mbar_wait(&misc->q_empty, (it - 1) & 1, abort_flag, 703, it);
+          if (!ok) break;
+          load_q(wi.tile, wi.bh, h_idx, b_idx);
+        }
+        for (int j = 0; j < nkv; ++j) {
+          if (it > 0 || j >= VS) {
+            ok = mbar_wait(&misc->v_empty[vs], v_par, abort_flag, 701, j);
+            if (!ok) break;
+            load_v(vs, j, h_idx, b_idx);
+            ok = mbar_wait(&misc->k_empty[ks], k_par, abort_flag, 702, j);
+            if (!ok) break;
+            load_k(ks, j, h_idx, b_idx);
+          }
+          if (++ks == KS) { ks = 0; k_par ^= 1; }
+          if (++vs == VS) { vs = 0; v_par ^= 1; }
+        }
       }
     }
   } else if (warp == WARP_MMA) {
@@ -708,49 +784,57 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
         mma_ts_lo(tb + (br ? T_DQ2 : T_DQ1), tb + (br ? T_S2 : T_S1) + (k / 2) * 32 + (k % 2) * 8, k_lo + k * (2048 >> 4), IDESC_DQ,
                   k > 0 ? 1u : first);
     };
-    bool ok = mbar_wait_warp(&misc->bar_q, 0, abort_flag, 801);
-    ok = ok && mbar_wait_warp(&misc->v_full[0], 0, abort_flag, 802);
-    ok = ok && mbar_wait_warp(&misc->k_full[0], 0, abort_flag, 803);
-    tc_fence_after();
-    if (ok && elect_one()) {
-      issue_dp(0);
-      issue_s(0, 0);
-      issue_s(1, 0);
-    }
-    __syncwarp();
-    int ks = 0;                        // K ring slot of tile j
-    uint32_t k_par = 0;                // parity of its pass over the ring
-    for (int j = 0; j < nkv; ++j) {
-      const bool more = j + 1 < nkv;
-      const int vs_n = (j + 1) % VS;
-      int ks_n = ks + 1;
-      if (ks_n == KS) { ks_n = 0; k_par ^= 1; }
-      if (more) {                      // tile j + 1 has landed (waited for under the warpgroups' pass)
-        ok = ok && mbar_wait_warp(&misc->v_full[vs_n], ((j + 1) / VS) & 1, abort_flag, 804, j);
-        ok = ok && mbar_wait_warp(&misc->k_full[ks_n], k_par, abort_flag, 805, j);
-      }
-      named_bar_sync(NB_DP, NB_THREADS);                               // dP(j) is in registers
-      tc_fence_after();
-      if (ok && more && elect_one()) issue_dp(vs_n);
-      __syncwarp();
-      named_bar_sync(NB_DS1, NB_THREADS);                              // dS1(j) written
+    bool ok = true;
+    int ks = 0, vs = 0;                // ring slots of tile j
+    uint32_t k_par = 0, v_par = 0;     // parities of their passes over the rings
+    for (int it = 0; work.valid(); ++it, work.next()) {
+      const int nkv = key_tiles(args.causal, args.n, work.item().tile);
+      ok = ok && mbar_wait_warp(&misc->bar_q, it & 1, abort_flag, 801, it);
+      ok = ok && mbar_wait_warp(&misc->v_full[vs], v_par, abort_flag, 802, it);
+      ok = ok && mbar_wait_warp(&misc->k_full[ks], k_par, abort_flag, 803, it);
       tc_fence_after();
       if (ok && elect_one()) {
-        issue_dq(0, ks, j > 0);
-        if (more) issue_s(0, ks_n);
+        issue_dp(vs);
+        issue_s(0, ks);
+        issue_s(1, ks);
+        if (nkv == 1) mma_commit(&misc->q_empty);
       }
       __syncwarp();
-      named_bar_sync(NB_DS2, NB_THREADS);                              // dS2(j) written
-      tc_fence_after();
-      if (ok && elect_one()) {
-        issue_dq(1, ks, j > 0);
-        mma_commit(&misc->k_empty[ks]);
-        if (more) issue_s(1, ks_n);
+      for (int j = 0; j < nkv; ++j) {
+        const bool more = j + 1 < nkv;
+        int ks_n = ks + 1, vs_n = vs + 1;
+        if (ks_n == KS) { ks_n = 0; k_par ^= 1; }
+        if (vs_n == VS) { vs_n = 0; v_par ^= 1; }
+        if (more) {                      // tile j + 1 has landed (waited for under the warpgroups' pass)
+          ok = ok && mbar_wait_warp(&misc->v_full[vs_n], v_par, abort_flag, 804, j);
+          ok = ok && mbar_wait_warp(&misc->k_full[ks_n], k_par, abort_flag, 805, j);
+        }
+        if (j == 0 && it > 0) named_bar_sync(NB_ACC, NB_THREADS);        // the previous tile's accumulators are in registers
+        named_bar_sync(NB_DP, NB_THREADS);                               // dP(j) is in registers
+        tc_fence_after();
+        if (ok && more && elect_one()) issue_dp(vs_n);
+        __syncwarp();
+        named_bar_sync(NB_DS1, NB_THREADS);                              // dS1(j) written
+        tc_fence_after();
+        if (ok && elect_one()) {
+          issue_dq(0, ks, j > 0);
+          if (more) issue_s(0, ks_n);
+        }
+        __syncwarp();
+        named_bar_sync(NB_DS2, NB_THREADS);                              // dS2(j) written
+        tc_fence_after();
+        if (ok && elect_one()) {
+          issue_dq(1, ks, j > 0);
+          mma_commit(&misc->k_empty[ks]);
+          if (more) issue_s(1, ks_n);
+          if (j == nkv - 2) mma_commit(&misc->q_empty);
+          if (!more) mma_commit(&misc->acc_full);
+        }
+        __syncwarp();
+        ks = ks_n;
+        vs = vs_n;
       }
-      __syncwarp();
-      ks = ks_n;
     }
-    if (ok && elect_one()) mma_commit(&misc->acc_full);
   } else {
     const int g = warp >> 2;                       // columns [32g, 32g + 32) of every tile
     const int row = (warp & 3) * 32 + lane;
@@ -758,14 +842,7 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
     const uint32_t tb = tmem_base + lane_base;
     const float sl2 = args.sm_scale * 1.4426950408889634f;
     const float lam = load_lambda(args.lambda_ptr, args.lambda_dtype);
-    const float4 sv = stat_row(args.stats, size_t(bh) * args.n_pad + size_t(q_tile) * BM + row);
     const float sg = lam < 0.f ? 1.f : -1.f;       // branch 2: -sign(lambda) (|lambda| sits in its statistics, the sign in e)
-    DropWalk dw1, dw2;
-    if constexpr (DROP) {
-      const uint32_t row2 = uint32_t(q_tile * BM + row) >> 1;
-      dw1 = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 0u), row2, row & 1, args.drop_thresh);
-      dw2 = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 1u), row2, row & 1, args.drop_thresh);
-    }
     const float dscale = DROP ? args.drop_scale : 1.f;
     const f32x2 sl2_2 = pk2(sl2, sl2);
     // (once a wait has given up the loop goes on without waiting, on whatever TMEM holds, and syncs on the named barriers
@@ -804,51 +881,69 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
       }
     };
     if (g >= 2) named_bar_sync(NB_START, NWG * 128);
-    for (int j = 0; j < nkv; ++j) {
-      // key columns past the sequence end or (causal) right of the diagonal: score -inf, probability 0
-      const int c_first = j * BN + g * 32;
-      int nv = args.n - c_first;
-      if (args.causal) nv = min(nv, q_tile * BM + row - c_first + 1);
-      uint32_t s[32], dp[32];
-      ok = ok && mbar_wait_warp(&misc->s_full[0], j & 1, abort_flag, 901, j);
+    uint32_t done = 0;                             // key tiles done: the phase of the score barriers
+    for (; work.valid(); work.next()) {
+      {
+        const WorkItem wi = work.item();
+        const int q_tile = wi.tile, bh = wi.bh, nkv = key_tiles(args.causal, args.n, q_tile);
+        const float4 sv = stat_row(args.stats, size_t(bh) * args.n_pad + size_t(q_tile) * BM + row);
+        DropWalk dw1, dw2;
+        if constexpr (DROP) {
+          const uint32_t row2 = uint32_t(q_tile * BM + row) >> 1;
+          dw1 = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 0u), row2, row & 1, args.drop_thresh);
+          dw2 = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 1u), row2, row & 1, args.drop_thresh);
+        }
+        for (int j = 0; j < nkv; ++j, ++done) {
+          // key columns past the sequence end or (causal) right of the diagonal: score -inf, probability 0
+          const int c_first = j * BN + g * 32;
+          int nv = args.n - c_first;
+          if (args.causal) nv = min(nv, q_tile * BM + row - c_first + 1);
+          uint32_t s[32], dp[32];
+          ok = ok && mbar_wait_warp(&misc->s_full[0], done & 1, abort_flag, 901, j);
+          tc_fence_after();
+          tmem_ld32(t_dp, dp);
+          tmem_ld32(t_s1, s);
+          tc_wait_ld();
+          hand_over(NB_DP);
+          branch(s, dp, nv, j, sv.x, sv.z, 1.f, dw1, [&] { if (done == 0 && g < 2) named_bar_arrive(NB_START, NWG * 128); });
+          tmem_st16(t_s1, s);
+          tc_wait_st();
+          hand_over(NB_DS1);
+          ok = ok && mbar_wait_warp(&misc->s_full[1], done & 1, abort_flag, 902, j);
+          tc_fence_after();
+          tmem_ld32(t_s2, s);
+          tc_wait_ld();
+          branch(s, dp, nv, j, sv.y, sv.w, sg, dw2, [] {});
+          tmem_st16(t_s2, s);
+          tc_wait_st();
+          hand_over(NB_DS2);
+        }
+      }
+      work.forget();
+      ok = ok && mbar_wait_warp(&misc->acc_full, work.round & 1, abort_flag, 911);
       tc_fence_after();
-      tmem_ld32(t_dp, dp);
-      tmem_ld32(t_s1, s);
+      const int u = g >> 1, half = g & 1;            // this warpgroup stores columns [32 half, 32 half + 32) of dQ of branch u
+      uint32_t acc[32];
+      tmem_ld32(tb + (u ? T_DQ2 : T_DQ1) + half * 32, acc);
       tc_wait_ld();
-      hand_over(NB_DP);
-      branch(s, dp, nv, j, sv.x, sv.z, 1.f, dw1, [&] { if (j == 0 && g < 2) named_bar_arrive(NB_START, NWG * 128); });
-      tmem_st16(t_s1, s);
-      tc_wait_st();
-      hand_over(NB_DS1);
-      ok = ok && mbar_wait_warp(&misc->s_full[1], j & 1, abort_flag, 902, j);
-      tc_fence_after();
-      tmem_ld32(t_s2, s);
-      tc_wait_ld();
-      branch(s, dp, nv, j, sv.y, sv.w, sg, dw2, [] {});
-      tmem_st16(t_s2, s);
-      tc_wait_st();
-      hand_over(NB_DS2);
-    }
-    ok = ok && mbar_wait(&misc->acc_full, 0, abort_flag, 911);
-    tc_fence_after();
-    const int u = g >> 1, half = g & 1;            // this warpgroup stores columns [32 half, 32 half + 32) of dQ of branch u
-    uint32_t acc[32];
-    tmem_ld32(tb + (u ? T_DQ2 : T_DQ1) + half * 32, acc);
-    tc_wait_ld();
-    // (32 columns per thread: direct 16-byte stores; a shared-memory tile and a TMA store, as the other two
-    // kernels use for their wider rows, measured 4 % slower here)
-    if (ok && !*abort_flag && half * 32 < args.d && q_tile * BM + row < args.n) {
-      const float sc = args.sm_scale;
-      const size_t grow = size_t(bh) * args.n + size_t(q_tile) * BM + row;
-      uint4* p = reinterpret_cast<uint4*>((u ? args.dq2 : args.dq1) + grow * args.d + half * 32);
+      if (work.has_next()) hand_over(NB_ACC);
+      const WorkItem wi = work.item();
+      const int q_tile = wi.tile;
+      // (32 columns per thread: direct 16-byte stores; a shared-memory tile and a TMA store, as the other two
+      // kernels use for their wider rows, measured 4 % slower here)
+      if (ok && !*abort_flag && half * 32 < args.d && q_tile * BM + row < args.n) {
+        const float sc = args.sm_scale;
+        const size_t grow = size_t(wi.bh) * args.n + size_t(q_tile) * BM + row;
+        uint4* p = reinterpret_cast<uint4*>((u ? args.dq2 : args.dq1) + grow * args.d + half * 32);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        uint4 v;
-        v.x = pack2<BF>(__uint_as_float(acc[8 * i + 0]) * sc, __uint_as_float(acc[8 * i + 1]) * sc);
-        v.y = pack2<BF>(__uint_as_float(acc[8 * i + 2]) * sc, __uint_as_float(acc[8 * i + 3]) * sc);
-        v.z = pack2<BF>(__uint_as_float(acc[8 * i + 4]) * sc, __uint_as_float(acc[8 * i + 5]) * sc);
-        v.w = pack2<BF>(__uint_as_float(acc[8 * i + 6]) * sc, __uint_as_float(acc[8 * i + 7]) * sc);
-        p[i] = v;
+        for (int i = 0; i < 4; ++i) {
+          uint4 v;
+          v.x = pack2<BF>(__uint_as_float(acc[8 * i + 0]) * sc, __uint_as_float(acc[8 * i + 1]) * sc);
+          v.y = pack2<BF>(__uint_as_float(acc[8 * i + 2]) * sc, __uint_as_float(acc[8 * i + 3]) * sc);
+          v.z = pack2<BF>(__uint_as_float(acc[8 * i + 4]) * sc, __uint_as_float(acc[8 * i + 5]) * sc);
+          v.w = pack2<BF>(__uint_as_float(acc[8 * i + 6]) * sc, __uint_as_float(acc[8 * i + 7]) * sc);
+          p[i] = v;
+        }
       }
     }
   }

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -150,6 +151,38 @@ int set_smem(K kernel, int bytes, int device) {
   return DIFFATTN_OK;
 }
 
+int sm_count(int device) {
+  if (g_sm_count[device] > 0) return g_sm_count[device];
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) sms = 148;
+  g_sm_count[device] = sms;
+  return sms;
+}
+
+// Tiles of a persistent kernel (see WorkList).  Under a mask, heads are walked together as long as their streamed operands (8 D bytes
+// per row) fit half of the L2 -- or in 32s, where four or five CTAs still share what one of them fetched.  Every group boundary
+// costs up to one heaviest tile of imbalance: B1 H16 N8192 D64 causal forward in groups of 14 and 2 heads 480 us, 16
+// together 440 (a grid of one-tile CTAs in that order: 476).
+da::WorkArgs work_args(const DiffAttnParams* p, bool heavy_last) {
+  da::WorkArgs w;
+  w.tiles = (p->N + 127) / 128;
+  w.heads = p->B * p->H;
+  w.items = w.tiles * w.heads;
+  const long long fit = (60ll << 20) / ((long long)p->N * p->D * 8);
+  const int groups = int((w.heads + std::max(fit, 32ll) - 1) / std::max(fit, 32ll));
+  w.group = p->causal ? (w.heads + groups - 1) / groups : 0;
+  w.heavy_last = heavy_last ? 1 : 0;
+  w.magic = w.tiles > 1 ? uint32_t(((1ull << 32) + w.tiles - 1) / w.tiles) : 0u;
+  return w;
+}
+
+// More items than SMs: one CTA per SM with a list of items, so that all but the first find the SM set up, their operands on the way and
+// the previous result's stores in nobody's way (a CTA alone spends about 12k clocks around its loop over the keys, 13 % of
+// it at N = 4096).  Else a CTA per item: finding the first item in a list costs 1-2 us of cold code (B1 H37 N512 D64 dK/dV 16.7 -> 18.7 us).
+dim3 work_grid(const da::WorkArgs& w, bool list, int device) {
+  return list ? dim3(sm_count(device)) : dim3(w.tiles, w.heads);
+}
+
 // Launch; `early`: the kernel may start while the one before it in the stream is still running (programmatic dependent
 // launch: the kernels say in the code what they wait for).
 template <typename... P, typename... A>
@@ -166,14 +199,6 @@ int launch(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t 
   cfg.numAttrs = early ? 1 : 0;
   DA_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
   return DIFFATTN_OK;
-}
-
-int sm_count(int device) {
-  if (g_sm_count[device] > 0) return g_sm_count[device];
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) sms = 148;
-  g_sm_count[device] = sms;
-  return sms;
 }
 
 // Every tensor must be device (or managed) memory of `device`: a host pointer or another GPU's buffer would make
@@ -348,11 +373,12 @@ int fwd_impl(const DiffAttnParams* p) {
   }
   CUtensorMap myg = my;      // only read by the kernel when a gain is given
   if (p->gain && (rc = make_map<BF>(&myg, p->y_gained, DV, p->N, (int)bh, 1, DV, (int64_t)p->N * DV, (int64_t)p->N * DV * bh, 128, "y_gained"))) return rc;
-  dim3 grid((p->N + 127) / 128, p->B * p->H);
-  if ((rc = set_smem(da::diffattn_fwd64_kernel<BF, DROP>, da::fwd64::SMEM_BYTES, p->device))) return rc;
-  da::diffattn_fwd64_kernel<BF, DROP><<<grid, da::fwd64::NUM_THREADS, da::fwd64::SMEM_BYTES, stream>>>(mq1, mq2, mk1, mk2, mv, my, ma2, myg, a);
-  DA_CUDA(cudaGetLastError());
-  return DIFFATTN_OK;
+  a.work = work_args(p, true);
+  const bool list = a.work.items > sm_count(p->device);
+  auto kernel = list ? da::diffattn_fwd64_kernel<BF, DROP, true> : da::diffattn_fwd64_kernel<BF, DROP, false>;
+  if ((rc = set_smem(kernel, da::fwd64::SMEM_BYTES, p->device))) return rc;
+  return launch(kernel, work_grid(a.work, list, p->device), da::fwd64::NUM_THREADS, da::fwd64::SMEM_BYTES, stream, false, mq1, mq2, mk1, mk2, mv, my, ma2,
+                myg, a);
 }
 
 template <bool BF, bool DROP>
@@ -468,9 +494,12 @@ int bwd_impl(const DiffAttnParams* p, int32_t stages) {
       da::diffattn_bwd_fused64_kernel<BF, DROP><<<grid, da::fused64::NUM_THREADS, da::fused64::SMEM_BYTES, stream>>>(mq1, mq2, mk1, mk2, mv, mda, mdk1, mdk2, mdv, a);
     } else {
       // 2'. dK, dV only (two-kernel form)
-      if ((rc = set_smem(da::diffattn_bwd_dkdv64_kernel<BF, DROP>, da::dkdv64::SMEM_BYTES, p->device))) return rc;
-      if ((rc = launch(da::diffattn_bwd_dkdv64_kernel<BF, DROP>, grid, da::dkdv64::NUM_THREADS, da::dkdv64::SMEM_BYTES, stream, pre, mq1, mq2, mk1, mk2, mv,
-                       mda, mdk1, mdk2, mdv, a))) return rc;
+      a.kwork = work_args(p, false);
+      const bool list = a.kwork.items > sms;
+      auto kernel = list ? da::diffattn_bwd_dkdv64_kernel<BF, DROP, true> : da::diffattn_bwd_dkdv64_kernel<BF, DROP, false>;
+      if ((rc = set_smem(kernel, da::dkdv64::SMEM_BYTES, p->device))) return rc;
+      if ((rc = launch(kernel, work_grid(a.kwork, list, p->device), da::dkdv64::NUM_THREADS, da::dkdv64::SMEM_BYTES, stream, pre, mq1, mq2, mk1, mk2, mv, mda,
+                       mdk1, mdk2, mdv, a))) return rc;
     }
     DA_CUDA(cudaGetLastError());
   }
@@ -489,10 +518,12 @@ int bwd_impl(const DiffAttnParams* p, int32_t stages) {
     if ((rc = make_map<BF>(&mk2, p->k2, D, p->N, p->H, p->B, p->qk_stride_n, p->qk_stride_h, p->qk_stride_b, 128, "k2"))) return rc;
     if ((rc = make_map<BF>(&mv, p->v, DV, p->N, p->H, p->B, p->v_stride_n, p->v_stride_h, p->v_stride_b, 128, "v"))) return rc;
     if ((rc = make_map<BF>(&mda, a.da, DV, p->N, (int)bh, 1, DV, (int64_t)p->N * DV, (int64_t)p->N * DV * bh, 128, "dA"))) return rc;
-    if ((rc = set_smem(da::diffattn_bwd_dq64_kernel<BF, DROP>, da::dq64::SMEM_BYTES, p->device))) return rc;
-    dim3 grid(n_tiles, (unsigned)bh);
-    if ((rc = launch(da::diffattn_bwd_dq64_kernel<BF, DROP>, grid, da::dq64::NUM_THREADS, da::dq64::SMEM_BYTES, stream, dkdv, mq1, mq2, mk1, mk2, mv, mda,
-                     a))) return rc;
+    a.qwork = work_args(p, true);
+    const bool list = a.qwork.items > sms;
+    auto kernel = list ? da::diffattn_bwd_dq64_kernel<BF, DROP, true> : da::diffattn_bwd_dq64_kernel<BF, DROP, false>;
+    if ((rc = set_smem(kernel, da::dq64::SMEM_BYTES, p->device))) return rc;
+    if ((rc = launch(kernel, work_grid(a.qwork, list, p->device), da::dq64::NUM_THREADS, da::dq64::SMEM_BYTES, stream, dkdv, mq1, mq2, mk1, mk2, mv, mda, a)))
+      return rc;
   }
   return DIFFATTN_OK;
 }

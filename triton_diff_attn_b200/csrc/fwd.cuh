@@ -35,7 +35,15 @@ struct FwdArgs {
   float drop_scale;       // 256 / (256 - drop_thresh)
   const float* gain;      // NULL, or fp32 [2D]: learnable gain of the output norm; then yg = y * gain is written too
   __half* yg;             // [B*H, N, 2D] dense (only with gain)
+  WorkArgs work;          // D <= 64: the tiles of a persistent CTA
 };
+
+// key/value tiles of 128 rows that query tile `tile` sees: with a causal mask the tiles right of the diagonal tile are skipped
+// altogether.  (The last tile may reach past N: TMA fills those rows with zeros.)
+__device__ __forceinline__ int key_tiles(int causal, int n, int tile) {
+  const int all = (n + 127) / 128;
+  return (causal && tile + 1 < all) ? tile + 1 : all;
+}
 
 __device__ __forceinline__ float load_lambda(const void* p, int dtype) {
   if (dtype == 0) return __half2float(*reinterpret_cast<const __half*>(p));
@@ -62,7 +70,8 @@ constexpr int OFF_V = OFF_K + KS * 2 * K_BYTES;
 constexpr int OFF_MISC = OFF_V + VS * V_BYTES;           // barriers, coefficients
 constexpr int PRELOAD = 2;                               // key/value tiles requested before the setup barrier (<= KS, VS)
 constexpr int STORE_TILE_BYTES = BM * 128;               // epilogue staging: 128 rows x 64 columns x 2 bytes
-static_assert(6 * STORE_TILE_BYTES <= KS * 2 * K_BYTES, "the y / a2 / gained-y staging tiles reuse the K ring");
+static_assert(4 * STORE_TILE_BYTES <= VS * V_BYTES && 2 * STORE_TILE_BYTES <= 2 * K_BYTES && KS >= 2,
+              "the y / a2 staging tiles reuse the V ring, the gained-y tiles a K stage that the next tile's first load does not fill");
 // TMEM columns: S_b buffer u at 128*b + 64*u; O1 at 256, O2 at 384
 constexpr int T_O = 256;
 
@@ -87,12 +96,12 @@ struct SoftmaxState {
 };
 
 // t_s: this thread's lane and the sub-tile's score columns in TMEM; t_p: where its probabilities go (two per column; may be
-// t_s); t_o, O_COLS: the branch's accumulator; nv: visible columns of this row (the rest get -inf, probability 0); loaded:
+// t_s); t_o, O_COLS: the branch's accumulator; first: sub-tile 0; t: its index, only read with dropout; nv: visible columns of this row (the rest get -inf, probability 0); loaded:
 // the scores are in registers; wait_m / publish_m: hand-over of the running maximum; wait_pv: P_b V of
 // sub-tile t-1 has completed; mid: runs half way through the exponentials; p_free: the
 // columns behind t_p may be overwritten (both false: a bounded wait gave up).
 template <bool BF, bool DROP, int O_COLS, class Loaded, class WaitM, class PublishM, class WaitPv, class Mid, class PFree>
-__device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, uint32_t t_p, uint32_t t_o, int t, int nv, float sl2,
+__device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, uint32_t t_p, uint32_t t_o, bool first, int t, int nv, float sl2,
                                                 volatile float* m_row, const DropWalk& dr, Loaded loaded, WaitM wait_m, PublishM publish_m,
                                                 WaitPv wait_pv, Mid mid, PFree p_free) {
   uint32_t sr[64];
@@ -112,7 +121,7 @@ __device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, 
   for (int i = 2; i < 32; ++i) mx[i & 3] = max3(mx[i & 3], __uint_as_float(sr[2 * i]), __uint_as_float(sr[2 * i + 1]));
   const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
   float m_prev = -INFINITY;
-  if (t > 0) {
+  if (!first) {
     wait_m();
     m_prev = *m_row;
   }
@@ -120,7 +129,7 @@ __device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, 
   const float m = need ? m_tile : m_prev;
   if (need) *m_row = m;
   publish_m();
-  if (__any_sync(0xffffffffu, need) && t > 0) {
+  if (__any_sync(0xffffffffu, need) && !first) {
     if (!wait_pv()) return false;
     tc_fence_after();
     const float scale = need ? ex2((m_prev - m) * sl2) : 1.f;

@@ -210,7 +210,7 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
         int nv = args.n - t * SUB;             // visible key columns of this row in this sub-tile
         if (args.causal) nv = min(nv, q_tile * BM + row - t * SUB + 1);
         ok = softmax_subtile<BF, DROP, DV>(
-                 st, t_s, t_p, t_o, t, nv, sl2, &misc->m_run[row], dr,
+                 st, t_s, t_p, t_o, t == 0, t, nv, sl2, &misc->m_run[row], dr,
                  [&] { if (t + 2 < nsub) { tc_fence_before(); named_bar_arrive(NB_SF + u, 160); } },
                  [&] { named_bar_sync(NB_M + (u ^ 1), 256); }, [&] { if (t + 1 < nsub) named_bar_arrive(NB_M + u, 256); },
                  [&] { return mbar_wait_warp(&misc->pv_done[u ^ 1], ((t - 1) >> 1) & 1, abort_flag, 2305 + br, t); },

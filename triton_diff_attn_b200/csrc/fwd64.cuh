@@ -21,12 +21,13 @@ constexpr int SMEM_BYTES = OFF_MISC + MISC_BYTES + 1024; // +1024 for manual ali
 // a quarter of the exponentials on the FMA pipe 0.80 (the pass is not bound by the exp unit, and it costs power).
 constexpr int NUM_SOFTMAX = 512;
 constexpr int NUM_THREADS = NUM_SOFTMAX + 128;
-constexpr int REGS_LAUNCH = 96, REGS_SOFTMAX = 104, REGS_ROLE = 56;
+constexpr int REGS_LAUNCH = 96, REGS_SOFTMAX = 104, REGS_ROLE = 64;
 static_assert(4 * REGS_SOFTMAX + REGS_ROLE <= 5 * REGS_LAUNCH, "register shares exceed the launch pool of a scheduler");
-constexpr int NB_P = 4, NB_M = 8, NB_KV = 12;     // named barriers, + branch * 2 + parity
-constexpr int WARP_TMA = 16, WARP_ALLOC = 17, WARP_MMA = 18;
+constexpr int NB_ALL = 1, NB_STORE = 2, NB_P = 4, NB_M = 8, NB_KV = 12, NB_O = 13;     // named barriers; STORE + branch; P, M + branch * 2 + parity
+constexpr int WARP_TMA = 16, WARP_ALLOC = 17, WARP_MMA = 18, WARP_STORE = 19;
 struct Misc {
-  uint64_t bar_q;
+  uint64_t bar_q, q_empty;
+  uint64_t stored;           // the epilogue's tiles have left the V ring
   uint64_t k_full[KS], k_empty[KS];
   uint64_t v_full[VS], v_empty[VS];
   uint64_t s_full[2][2];     // [branch][buffer]: S sub-tile written by the MMA
@@ -43,7 +44,7 @@ static_assert(sizeof(Misc) <= MISC_BYTES, "misc area too small");
 }  // namespace fwd64
 
 
-template <bool BF, bool DROP>   // BF: tensors are bf16 instead of fp16; DROP: attention dropout on
+template <bool BF, bool DROP, bool LIST>   // BF: tensors are bf16 instead of fp16; DROP: attention dropout on; LIST: several tiles per CTA
 __global__ void __launch_bounds__(fwd64::NUM_THREADS, 1)
 diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_constant__ CUtensorMap tm_q2,
                       const __grid_constant__ CUtensorMap tm_k1, const __grid_constant__ CUtensorMap tm_k2,
@@ -58,19 +59,16 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  // causal: the later a query tile, the more keys it sees -- the heaviest tiles are launched first so that the grid's tail is light
-  const int q_tile = args.causal ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x);
-  const int bh = blockIdx.y;
-  const int b_idx = bh / args.h;
-  const int h_idx = bh % args.h;
-  // the last tile may reach past N (TMA fills those rows with zeros); with a causal mask the tiles right of
-  // the diagonal tile are skipped altogether
-  const int nkv_all = (args.n + BN - 1) / BN;
-  const int nkv = (args.causal && q_tile + 1 < nkv_all) ? q_tile + 1 : nkv_all;
-  const int nsub = 2 * nkv;          // 64-row sub-tiles
-
+  // Persistent: this CTA works on the tiles of its WorkList one after the other.  The loads of the next tile's Q and K go out
+  // as soon as the last scores of this one are issued, its first scores as soon as the last P V is, and y and a2 leave under
+  // the next tile's first passes.  Every ring and barrier runs on from tile to tile; each role counts along by itself.
+  // Against one CTA per tile: B8 H16 N2048 D32 405 -> 375 us, B8 H16 N512 D64 52 -> 46, B4 H16 N2048 D64 causal 156 -> 144,
+  // B4 H16 N4096 D64 878 -> 862 in a sustained loop.
+  WorkList<LIST> work(args.work);
   if (warp == WARP_TMA && lane == 0) {
     mbar_init(&misc->bar_q, 1);
+    mbar_init(&misc->q_empty, 1);
+    mbar_init(&misc->stored, 1);
     for (int i = 0; i < KS; ++i) { mbar_init(&misc->k_full[i], 1); mbar_init(&misc->k_empty[i], 1); }
     for (int i = 0; i < VS; ++i) { mbar_init(&misc->v_full[i], 1); mbar_init(&misc->v_empty[i], 1); }
     for (int b = 0; b < 2; ++b) {
@@ -82,9 +80,12 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
     mbar_init_fence();
     // The first loads go out before the CTA-wide setup barrier (TMEM allocation, everyone's arrival): the
     // barriers they complete on are initialised above, and the first pass over a ring needs no "empty" wait.
+    const WorkItem wi = work.item();
+    const int nkv = key_tiles(args.causal, args.n, wi.tile);
+    const int b_idx = wi.bh / args.h, h_idx = wi.bh % args.h;
     mbar_expect_tx(&misc->bar_q, 2 * Q_BYTES);
-    tma_load_4d(smem + OFF_Q1, &tm_q1, &misc->bar_q, 0, q_tile * BM, h_idx, b_idx);
-    tma_load_4d(smem + OFF_Q2, &tm_q2, &misc->bar_q, 0, q_tile * BM, h_idx, b_idx);
+    tma_load_4d(smem + OFF_Q1, &tm_q1, &misc->bar_q, 0, wi.tile * BM, h_idx, b_idx);
+    tma_load_4d(smem + OFF_Q2, &tm_q2, &misc->bar_q, 0, wi.tile * BM, h_idx, b_idx);
     for (int j = 0; j < PRELOAD && j < nkv; ++j) {
       mbar_expect_tx(&misc->k_full[j], 2 * K_BYTES);
       tma_load_4d(smem + OFF_K + j * 2 * K_BYTES, &tm_k1, &misc->k_full[j], 0, j * BN, h_idx, b_idx);
@@ -107,62 +108,90 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
     // ------------------------------- TMA producer -------------------------------
     reg_dec<REGS_ROLE>();
     if (elect_one()) {
-      for (int j = PRELOAD; j < nkv; ++j) {
-        const int ks = j % KS, vs = j % VS;
-        if (!mbar_wait(&misc->k_empty[ks], ((j / KS) & 1) ^ 1, abort_flag, 101, j)) break;
-        mbar_expect_tx(&misc->k_full[ks], 2 * K_BYTES);
-        tma_load_4d(smem + OFF_K + ks * 2 * K_BYTES, &tm_k1, &misc->k_full[ks], 0, j * BN, h_idx, b_idx);
-        tma_load_4d(smem + OFF_K + ks * 2 * K_BYTES + K_BYTES, &tm_k2, &misc->k_full[ks], 0, j * BN, h_idx, b_idx);
-        if (!mbar_wait(&misc->v_empty[vs], ((j / VS) & 1) ^ 1, abort_flag, 102, j)) break;
-        mbar_expect_tx(&misc->v_full[vs], V_BYTES);
-        tma_load_4d(smem + OFF_V + vs * V_BYTES, &tm_v, &misc->v_full[vs], 0, j * BN, h_idx, b_idx);
-        tma_load_4d(smem + OFF_V + vs * V_BYTES + V_BYTES / 2, &tm_v, &misc->v_full[vs], 64, j * BN, h_idx, b_idx);
+      bool ok = true;
+      int ks = 0, vs = 0;                 // ring slots; the parity bits are those of an "empty" wait (a first pass never waits)
+      uint32_t k_par = 1, v_par = 1;
+      for (int it = 0; ok && work.valid(); ++it, work.next()) {
+        const WorkItem wi = work.item();
+        const int nkv = key_tiles(args.causal, args.n, wi.tile);
+        const int b_idx = wi.bh / args.h, h_idx = wi.bh % args.h;
+        if (it > 0) {
+          ok = mbar_wait(&misc->q_empty, (it - 1) & 1, abort_flag, 103, it);
+          if (!ok) break;
+          mbar_expect_tx(&misc->bar_q, 2 * Q_BYTES);
+          tma_load_4d(smem + OFF_Q1, &tm_q1, &misc->bar_q, 0, wi.tile * BM, h_idx, b_idx);
+          tma_load_4d(smem + OFF_Q2, &tm_q2, &misc->bar_q, 0, wi.tile * BM, h_idx, b_idx);
+        }
+        for (int j = 0; j < nkv; ++j) {
+          const bool requested = it == 0 && j < PRELOAD;
+          if (!requested) {
+            ok = mbar_wait(&misc->k_empty[ks], k_par, abort_flag, 101, j);
+            if (!ok) break;
+            mbar_expect_tx(&misc->k_full[ks], 2 * K_BYTES);
+            tma_load_4d(smem + OFF_K + ks * 2 * K_BYTES, &tm_k1, &misc->k_full[ks], 0, j * BN, h_idx, b_idx);
+            tma_load_4d(smem + OFF_K + ks * 2 * K_BYTES + K_BYTES, &tm_k2, &misc->k_full[ks], 0, j * BN, h_idx, b_idx);
+            // the previous tile's y and a2 (and its gained y, in the K slot after the one just requested) have to leave first
+            if (it > 0 && j == 0) ok = mbar_wait(&misc->stored, (it - 1) & 1, abort_flag, 104, it);
+            ok = ok && mbar_wait(&misc->v_empty[vs], v_par, abort_flag, 102, j);
+            if (!ok) break;
+            mbar_expect_tx(&misc->v_full[vs], V_BYTES);
+            tma_load_4d(smem + OFF_V + vs * V_BYTES, &tm_v, &misc->v_full[vs], 0, j * BN, h_idx, b_idx);
+            tma_load_4d(smem + OFF_V + vs * V_BYTES + V_BYTES / 2, &tm_v, &misc->v_full[vs], 64, j * BN, h_idx, b_idx);
+          }
+          if (++ks == KS) { ks = 0; k_par ^= 1; }
+          if (++vs == VS) { vs = 0; v_par ^= 1; }
+        }
       }
     }
   } else if (warp == WARP_MMA) {
     // ------------- MMA issuer: O_b += P_b(t) V(sub-tile t), S_b(t+2) = Q_b K_b(sub-tile t+2)^T, branch 1 then branch 2 -------------
     // The thread that issues is chosen by elect.sync.  (A thread picked by comparing the lane id issues
     // tcgen05.mma about three times slower: 152 against 48 clocks per instruction, measured.)
+    // Every trip makes its barrier calls whether or not a wait gave up, so nobody is left without a partner.
     reg_dec<REGS_ROLE>();
-    {
-      const uint32_t IDESC_O = make_idesc(BM, 2 * args.d, 0, 1, BF);    // V is MN-major; head dim 32: the 64 real value columns only
-      constexpr uint32_t IDESC_S = make_idesc(BM, SUB, 0, 0, BF);
-      constexpr uint32_t HALF = (SUB * 128) >> 4;
-      const uint32_t v_lo0 = sdesc_lo(smem_u32(smem + OFF_V), V_BYTES / 2);
-      const int kd = args.d >> 4;
-      const uint32_t q_lo = sdesc_lo(smem_u32(smem + OFF_Q1));
-      const uint32_t k_lo0 = sdesc_lo(smem_u32(smem + OFF_K));
-      auto issue_s = [&](uint32_t k_lo, int br, int u) {
+    const uint32_t IDESC_O = make_idesc(BM, 2 * args.d, 0, 1, BF);    // V is MN-major; head dim 32: the 64 real value columns only
+    constexpr uint32_t IDESC_S = make_idesc(BM, SUB, 0, 0, BF);
+    constexpr uint32_t HALF = (SUB * 128) >> 4;
+    const uint32_t v_lo0 = sdesc_lo(smem_u32(smem + OFF_V), V_BYTES / 2);
+    const int kd = args.d >> 4;
+    const uint32_t q_lo = sdesc_lo(smem_u32(smem + OFF_Q1));
+    const uint32_t k_lo0 = sdesc_lo(smem_u32(smem + OFF_K));
+    auto issue_s = [&](uint32_t k_lo, int br, int u) {
 #pragma unroll
-        for (int k = 0; k < HD / 16; ++k)
-          if (k < kd)
-            mma_ss_lo(tmem_base + br * 128 + u * SUB, q_lo + br * (Q_BYTES >> 4) + k * 2, k_lo + br * (K_BYTES >> 4) + u * HALF + k * 2, IDESC_S, k > 0);
-        mma_commit(&misc->s_full[br][u]);
-      };
-      int vs = 0, ks = 0;
-      bool ok = mbar_wait_warp(&misc->bar_q, 0, abort_flag, 201);
-      ok = ok && mbar_wait_warp(&misc->k_full[0], 0, abort_flag, 202);
-      if (ok) {
-        tc_fence_after();
-        if (elect_one()) {
-          for (int u = 0; u < 2; ++u)
-            for (int br = 0; br < 2; ++br) issue_s(k_lo0, br, u);
-          mma_commit(&misc->k_empty[0]);
-        }
-        __syncwarp();
-        if (++ks == KS) ks = 0;
+      for (int k = 0; k < HD / 16; ++k)
+        if (k < kd)
+          mma_ss_lo(tmem_base + br * 128 + u * SUB, q_lo + br * (Q_BYTES >> 4) + k * 2, k_lo + br * (K_BYTES >> 4) + u * HALF + k * 2, IDESC_S, k > 0);
+      mma_commit(&misc->s_full[br][u]);
+    };
+    bool ok = true;
+    int vs = 0, ks = 0;
+    uint32_t k_par = 0;
+    for (int it = 0; work.valid(); ++it, work.next()) {
+      const int nkv = key_tiles(args.causal, args.n, work.item().tile);
+      ok = ok && mbar_wait_warp(&misc->bar_q, it & 1, abort_flag, 201, it);
+      ok = ok && mbar_wait_warp(&misc->k_full[ks], k_par, abort_flag, 202, it);
+      tc_fence_after();
+      if (ok && elect_one()) {
+        const uint32_t k_lo = k_lo0 + ks * ((2 * K_BYTES) >> 4);
+        for (int u = 0; u < 2; ++u)
+          for (int br = 0; br < 2; ++br) issue_s(k_lo, br, u);
+        mma_commit(&misc->k_empty[ks]);
+        if (nkv == 1) mma_commit(&misc->q_empty);
       }
-      for (int j = 0; ok && j < nkv; ++j) {
+      __syncwarp();
+      if (++ks == KS) { ks = 0; k_par ^= 1; }
+      for (int j = 0; j < nkv; ++j) {
         const uint32_t v_lo = v_lo0 + vs * (V_BYTES >> 4);
         const uint32_t k_lo = k_lo0 + ks * ((2 * K_BYTES) >> 4);       // key tile j+1
         const bool more = j + 1 < nkv;
         named_bar_sync(NB_KV, 64);               // V of tile j and K of tile j + 1 have landed (the watcher warp)
+        if (j == 0 && it > 0) named_bar_sync(NB_O, NUM_SOFTMAX + 32);  // the previous tile's accumulators are in registers
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int u = i >> 1, br = i & 1;
           named_bar_sync(NB_P + br * 2 + u, 160);
           tc_fence_after();
-          if (elect_one()) {
+          if (ok && elect_one()) {
 #pragma unroll
             for (int k = 0; k < SUB / 16; ++k)
               mma_ts_lo(tmem_base + T_O + br * 128, tmem_base + br * 128 + u * SUB + k * 8, v_lo + u * HALF + k * (2048 >> 4), IDESC_O,
@@ -171,156 +200,194 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
             if (more) issue_s(k_lo, br, u);
             if (i == 3) {
               if (more) mma_commit(&misc->k_empty[ks]);
+              if (j == nkv - 2) mma_commit(&misc->q_empty);
               mma_commit(&misc->v_empty[vs]);
             }
           }
           __syncwarp();
         }
-        if (++ks == KS) ks = 0;
+        if (more && ++ks == KS) { ks = 0; k_par ^= 1; }
         if (++vs == VS) vs = 0;
       }
-      if (!ok)
-        for (int j = 0; j < nkv; ++j) named_bar_arrive(NB_KV, 64);      // the watcher must not wait for this warp
-      if (elect_one()) mma_commit(&misc->o_full);
+      if (ok && elect_one()) mma_commit(&misc->o_full);
+      __syncwarp();
     }
   } else if (warp == WARP_ALLOC) {
     // Load watcher: waits for V of tile j and K of tile j + 1 on behalf of the MMA issuer.  A wait on an mbarrier costs
     // 150-300 clocks while MMAs saturate shared memory, even when the phase completed long ago; a named barrier costs
     // a tenth of that, and the issuer is the busiest thread of the CTA.
     reg_dec<REGS_ROLE>();
-    int vs = 0, ks = 1 % KS;
+    bool ok = true;
+    int vs = 0, ks = 0;
     uint32_t v_par = 0, k_par = 0;
-    for (int j = 0; j < nkv; ++j) {
-      mbar_wait_warp(&misc->v_full[vs], v_par, abort_flag, 205, j);
-      if (j + 1 < nkv) mbar_wait_warp(&misc->k_full[ks], k_par, abort_flag, 203, j);
-      named_bar_sync(NB_KV, 64);
-      if (++ks == KS) { ks = 0; k_par ^= 1; }
-      if (++vs == VS) { vs = 0; v_par ^= 1; }
+    for (; work.valid(); work.next()) {
+      const int nkv = key_tiles(args.causal, args.n, work.item().tile);
+      for (int j = 0; j < nkv; ++j) {
+        if (++ks == KS) { ks = 0; k_par ^= 1; }          // key tile j + 1 (the issuer waits for tile 0 itself)
+        ok = ok && mbar_wait_warp(&misc->v_full[vs], v_par, abort_flag, 205, j);
+        if (j + 1 < nkv) ok = ok && mbar_wait_warp(&misc->k_full[ks], k_par, abort_flag, 203, j);
+        named_bar_sync(NB_KV, 64);
+        if (++vs == VS) { vs = 0; v_par ^= 1; }
+      }
     }
-  } else if (warp >= NUM_SOFTMAX / 32) {
-    // (idle: completes the role warpgroup, whose registers go to the softmax warpgroups)
+  } else if (warp == WARP_STORE) {
+    // y and a2 leave through the TMA engine from the V ring (idle between a tile's last P V and the next tile's first), the gained
+    // y from the K slot that the next tile fills second.  A warp of its own waits for the engine, so nobody else does.
     reg_dec<REGS_ROLE>();
+    const int dv_real = 2 * args.d;
+    int ks = 0;
+    for (; work.valid(); work.next()) {
+      const WorkItem wi = work.item();
+      ks = (ks + key_tiles(args.causal, args.n, wi.tile)) % KS;
+      for (int br = 0; br < 2; ++br) {
+        named_bar_sync(NB_STORE + br, NUM_SOFTMAX / 2 + 32);
+        if (elect_one() && !*abort_flag && br * 64 < dv_real) {
+          const uint8_t* ytile = smem + OFF_V + br * (2 * STORE_TILE_BYTES);
+          tma_store_4d(ytile, &tm_y, br * 64, wi.tile * BM, wi.bh, 0);
+          tma_store_4d(ytile + STORE_TILE_BYTES, &tm_a2, br * 64, wi.tile * BM, wi.bh, 0);
+          if (args.gain) tma_store_4d(smem + OFF_K + ((ks + 1) % KS) * 2 * K_BYTES + br * STORE_TILE_BYTES, &tm_yg, br * 64, wi.tile * BM, wi.bh, 0);
+          tma_store_commit();
+        }
+        __syncwarp();
+      }
+      tma_store_wait_read();       // (every lane: the elected one of either half has the groups)
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&misc->stored);
+    }
   } else {
     // ------------------------- softmax warpgroups + epilogue -------------------------
     reg_inc<REGS_SOFTMAX>();
     const int br = warp >> 3;                       // branch
     const int u = (warp >> 2) & 1;                  // sub-tile parity = score buffer of this warpgroup
-    const int row = (warp & 3) * 32 + lane;         // query row inside the tile = TMEM lane
     const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
+    // query row inside the tile = TMEM lane; computed anew where it is needed (the softmax pass leaves no register to keep it)
+    auto softmax_row = [] {
+      uint32_t t;
+      asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+      return int(t & 127u);
+    };
     const float sl2 = args.sm_scale * 1.4426950408889634f;
     bool ok = true;
-    SoftmaxState st;
-    {
-      const uint32_t t_s = tmem_base + lane_base + br * 128 + u * SUB;
-      const uint32_t t_o = tmem_base + lane_base + T_O + br * 128;
-      DropWalk dr;
-      if constexpr (DROP)
-        dr = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), uint32_t(br)), uint32_t(q_tile * BM + row) >> 1, row & 1, args.drop_thresh);
-      int t = u;
-      for (; t < nsub; t += 2) {
-        ok = mbar_wait_warp(&misc->s_full[br][u], (t >> 1) & 1, abort_flag, 301 + br, t);
-        if (!ok) break;
-        tc_fence_after();
-        int nv = args.n - t * SUB;                  // visible key columns: up to the sequence end, up to the diagonal
-        if (args.causal) nv = min(nv, q_tile * BM + row - t * SUB + 1);
-        ok = softmax_subtile<BF, DROP, DV>(
-            st, t_s, t_s, t_o, t, nv, sl2, &misc->m_run[br][row], dr, [] {}, [&] { named_bar_sync(NB_M + br * 2 + (u ^ 1), 256); },
-            [&] { if (t + 1 < nsub) named_bar_arrive(NB_M + br * 2 + u, 256); },
-            [&] { return mbar_wait_warp(&misc->pv_done[br][u ^ 1], ((t - 1) >> 1) & 1, abort_flag, 305 + br, t); }, [] {}, [] { return true; });
-        named_bar_arrive(NB_P + br * 2 + u, 160);
-        if (!ok) { t += 2; break; }
-      }
-      // a warp whose wait gave up stands in for the named-barrier arrivals it will no longer make
-      for (; t < nsub; t += 2) {
-        if (t > 0) named_bar_arrive(NB_M + br * 2 + (u ^ 1), 256);
-        if (t + 1 < nsub) named_bar_arrive(NB_M + br * 2 + u, 256);
-        named_bar_arrive(NB_P + br * 2 + u, 160);
-      }
-    }
-
-    // ---- epilogue: every thread runs every barrier; only the global writes depend on `ok`
-    ok = ok && mbar_wait(&misc->o_full, 0, abort_flag, 311 + br);
-    tc_fence_after();
-    misc->m_end[br][u][row] = st.m;
-    misc->l_end[br][u][row] = st.l;
-    named_bar_sync(1, NUM_SOFTMAX);
-    float m_fin[2], l_fin[2];         // both branches of this row: the later maximum of the two warpgroups, row sum relative to it
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      const float ma = misc->m_end[b][0][row], mb = misc->m_end[b][1][row];
-      m_fin[b] = fmaxf(ma, mb);
-      l_fin[b] = misc->l_end[b][0][row] * ex2((ma - m_fin[b]) * sl2) + misc->l_end[b][1][row] * ex2((mb - m_fin[b]) * sl2);
-    }
-    const float lam = load_lambda(args.lambda_ptr, args.lambda_dtype);
-    const float keep = DROP ? args.drop_scale : 1.f;       // kept probabilities are scaled by 1 / (1 - p)
-    const float c1 = keep / l_fin[0], c2 = keep / l_fin[1];
-    // this warpgroup owns value columns [32 q, 32 q + 32) of both accumulators
-    const int q = br * 2 + u;
-    uint32_t o1[32], o2[32];
-    tmem_ld32(tmem_base + lane_base + T_O + q * 32, o1);
-    tmem_ld32(tmem_base + lane_base + T_O + 128 + q * 32, o2);
-    tc_wait_ld();
-    float ssq = 0.f;
-    const int dv_real = 2 * args.d;                      // 128, or 64 when the head dim is 32 (upper columns are padding)
-    const bool pad = q * 32 >= dv_real;                  // head dim 32: columns 64..127 of the accumulators were never written
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float a2v = pad ? 0.f : __uint_as_float(o2[i]) * c2;
-      const float av = pad ? 0.f : __uint_as_float(o1[i]) * c1 - lam * a2v;
-      ssq += av * av;
-      o1[i] = __float_as_uint(av);
-      o2[i] = __float_as_uint(a2v);
-    }
-    misc->ssq[q][row] = ssq;
-    named_bar_sync(1, NUM_SOFTMAX);
-    const float rstd = rsqrtf(((misc->ssq[0][row] + misc->ssq[1][row]) + (misc->ssq[2][row] + misc->ssq[3][row])) / float(dv_real) + args.eps);
-    const float yscale = args.rms_norm ? args.out_scale * rstd : 1.f;
-    const size_t grow = size_t(bh) * args.n + size_t(q_tile) * BM + row;
-    ok = ok && (q_tile * BM + row < args.n);            // rows past the sequence end are computed on zero padding and dropped
-    // y and a2 leave through shared memory and the TMA engine: each thread lays its 32 columns into a swizzled
-    // [128 rows][64 columns] tile in the (now idle) K ring, and one thread per tile stores it.
-    // (Row-per-thread global stores of 16-byte pieces cost 3.6 us per CTA, 8 % of the kernel at N = 4096.)
-    {
-      uint8_t* ytile = smem + OFF_K + br * (3 * STORE_TILE_BYTES);
-      uint8_t* atile = ytile + STORE_TILE_BYTES;
-      uint8_t* gtile = atile + STORE_TILE_BYTES;          // y * gain, only with a gain
-      const float4* gp = reinterpret_cast<const float4*>(args.gain + q * 32);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float f[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) f[k] = __uint_as_float(o1[8 * i + k]) * yscale;
-        uint4 av;
-        av.x = pack2<BF>(__uint_as_float(o2[8 * i + 0]), __uint_as_float(o2[8 * i + 1]));
-        av.y = pack2<BF>(__uint_as_float(o2[8 * i + 2]), __uint_as_float(o2[8 * i + 3]));
-        av.z = pack2<BF>(__uint_as_float(o2[8 * i + 4]), __uint_as_float(o2[8 * i + 5]));
-        av.w = pack2<BF>(__uint_as_float(o2[8 * i + 6]), __uint_as_float(o2[8 * i + 7]));
-        st_swizzled_chunk(ytile, row, u * 4 + i, make_uint4(pack2<BF>(f[0], f[1]), pack2<BF>(f[2], f[3]), pack2<BF>(f[4], f[5]), pack2<BF>(f[6], f[7])));
-        st_swizzled_chunk(atile, row, u * 4 + i, av);
-        if (args.gain && !pad) {
-          const float4 g0 = __ldg(gp + 2 * i), g1 = __ldg(gp + 2 * i + 1);
-          st_swizzled_chunk(gtile, row, u * 4 + i, make_uint4(pack2<BF>(f[0] * g0.x, f[1] * g0.y), pack2<BF>(f[2] * g0.z, f[3] * g0.w),
-                                                      pack2<BF>(f[4] * g1.x, f[5] * g1.y), pack2<BF>(f[6] * g1.z, f[7] * g1.w)));
+    int tc = u;                                     // sub-tiles, counted on from tile to tile: tc >> 1 is the phase of the buffers' barriers
+    auto hand_over = [&](int id, int threads) {
+      if (ok) named_bar_arrive(id, threads);
+      else named_bar_sync(id, threads);
+    };
+    for (; work.valid(); work.next()) {
+      SoftmaxState st;
+      {
+        const WorkItem wi = work.item();
+        const int row = softmax_row();
+        const int nsub = 2 * key_tiles(args.causal, args.n, wi.tile);
+        const uint32_t t_s = tmem_base + lane_base + br * 128 + u * SUB;
+        const uint32_t t_o = tmem_base + lane_base + T_O + br * 128;
+        DropWalk dr;
+        if constexpr (DROP)
+          dr = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(wi.bh), uint32_t(br)), uint32_t(wi.tile * BM + row) >> 1, row & 1,
+                             args.drop_thresh);
+        const int t0 = tc - u, t_first = u ? -1 : tc, t_end = t0 + nsub;
+        int seen = args.n;                            // visible key columns: up to the sequence end, up to the diagonal
+        if (args.causal) seen = min(seen, wi.tile * BM + row + 1);
+        seen += t0 * SUB;
+        for (; ok && tc < t_end; tc += 2) {
+          if (!mbar_wait_warp(&misc->s_full[br][u], (tc >> 1) & 1, abort_flag, 301 + br, tc)) { ok = false; break; }
+          tc_fence_after();
+          // P_b V of sub-tile tc - 1 used the other buffer
+          ok = softmax_subtile<BF, DROP, DV>(
+              st, t_s, t_s, t_o, tc == t_first, tc - t0, seen - tc * SUB, sl2, &misc->m_run[br][row], dr, [] {},
+              [&] { named_bar_sync(NB_M + br * 2 + (u ^ 1), 256); }, [&] { if (tc + 1 < t_end) named_bar_arrive(NB_M + br * 2 + u, 256); },
+              [&] { return mbar_wait_warp(&misc->pv_done[br][u ^ 1], ((tc - 1) >> 1) & 1, abort_flag, 305 + br, tc); }, [] {}, [] { return true; });
+          named_bar_arrive(NB_P + br * 2 + u, 160);
+        }
+        // after a wait that gave up: the named barriers of the sub-tiles left, synced on instead of arrived at, so that nobody is left
+        // waiting and nobody runs ahead
+        for (; tc < t_end; tc += 2) {
+          if (tc != t_first) named_bar_sync(NB_M + br * 2 + (u ^ 1), 256);
+          if (tc + 1 < t_end) named_bar_sync(NB_M + br * 2 + u, 256);
+          named_bar_sync(NB_P + br * 2 + u, 160);
         }
       }
-      fence_proxy_async_smem();
-      named_bar_sync(2 + br, NUM_SOFTMAX / 2);
-      if ((warp & 7) == 0 && elect_one()) {
-        if (!*abort_flag && br * 64 < dv_real) {
-          tma_store_4d(ytile, &tm_y, br * 64, q_tile * BM, bh, 0);
-          tma_store_4d(atile, &tm_a2, br * 64, q_tile * BM, bh, 0);
-          if (args.gain) tma_store_4d(gtile, &tm_yg, br * 64, q_tile * BM, bh, 0);
-          tma_store_commit();
-          tma_store_wait_read();
-        }
+      work.forget();
+      const int row = softmax_row();
+      // ---- epilogue: every thread runs every barrier; only the global writes depend on `ok`
+      ok = ok && mbar_wait_warp(&misc->o_full, work.round & 1, abort_flag, 311 + br);
+      tc_fence_after();
+      misc->m_end[br][u][row] = st.m;
+      misc->l_end[br][u][row] = st.l;
+      named_bar_sync(NB_ALL, NUM_SOFTMAX);
+      float m_fin[2], l_fin[2];         // both branches of this row: the later maximum of the two warpgroups, row sum relative to it
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        const float ma = misc->m_end[b][0][row], mb = misc->m_end[b][1][row];
+        m_fin[b] = fmaxf(ma, mb);
+        l_fin[b] = misc->l_end[b][0][row] * ex2((ma - m_fin[b]) * sl2) + misc->l_end[b][1][row] * ex2((mb - m_fin[b]) * sl2);
       }
-    }
-    if (ok && !*abort_flag && u == 0) {
-      if (br == 0) {
-        args.lse1[grow] = m_fin[0] * args.sm_scale + logf(l_fin[0]);
-        args.rstd[grow] = rstd;
-      } else {
-        args.lse2[grow] = m_fin[1] * args.sm_scale + logf(l_fin[1]);
+      const float lam = load_lambda(args.lambda_ptr, args.lambda_dtype);
+      const float keep = DROP ? args.drop_scale : 1.f;       // kept probabilities are scaled by 1 / (1 - p)
+      const float c1 = keep / l_fin[0], c2 = keep / l_fin[1];
+      // this warpgroup owns value columns [32 q, 32 q + 32) of both accumulators
+      const int q = br * 2 + u;
+      uint32_t o1[32], o2[32];
+      tmem_ld32(tmem_base + lane_base + T_O + q * 32, o1);
+      tmem_ld32(tmem_base + lane_base + T_O + 128 + q * 32, o2);
+      tc_wait_ld();
+      tc_fence_before();
+      if (work.has_next()) hand_over(NB_O, NUM_SOFTMAX + 32);
+      float ssq = 0.f;
+      const int dv_real = 2 * args.d;                      // 128, or 64 when the head dim is 32 (upper columns are padding)
+      const bool pad = q * 32 >= dv_real;                  // head dim 32: columns 64..127 of the accumulators were never written
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const float a2v = pad ? 0.f : __uint_as_float(o2[i]) * c2;
+        const float av = pad ? 0.f : __uint_as_float(o1[i]) * c1 - lam * a2v;
+        ssq += av * av;
+        o1[i] = __float_as_uint(av);
+        o2[i] = __float_as_uint(a2v);
+      }
+      misc->ssq[q][row] = ssq;
+      named_bar_sync(NB_ALL, NUM_SOFTMAX);
+      const float rstd = rsqrtf(((misc->ssq[0][row] + misc->ssq[1][row]) + (misc->ssq[2][row] + misc->ssq[3][row])) / float(dv_real) + args.eps);
+      const float yscale = args.rms_norm ? args.out_scale * rstd : 1.f;
+      const WorkItem wi = work.item();
+      const int q_tile = wi.tile;
+      const size_t grow = size_t(wi.bh) * args.n + size_t(q_tile) * BM + row;
+      const bool write = ok && q_tile * BM + row < args.n;     // rows past the sequence end are computed on zero padding and dropped
+      // y and a2 leave through shared memory and the TMA engine: each thread lays its 32 columns into a swizzled
+      // [128 rows][64 columns] tile in the (now idle) V ring, and the store warp stores the tiles.
+      // (Row-per-thread global stores of 16-byte pieces cost 3.6 us per CTA, 8 % of the kernel at N = 4096.)
+      {
+        uint8_t* ytile = smem + OFF_V + br * (2 * STORE_TILE_BYTES);
+        uint8_t* atile = ytile + STORE_TILE_BYTES;
+        uint8_t* gtile = smem + OFF_K + ((tc >> 1) + 1) % KS * 2 * K_BYTES + br * STORE_TILE_BYTES;          // y * gain, only with a gain
+        const float4* gp = reinterpret_cast<const float4*>(args.gain + q * 32);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float f[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) f[k] = __uint_as_float(o1[8 * i + k]) * yscale;
+          uint4 av;
+          av.x = pack2<BF>(__uint_as_float(o2[8 * i + 0]), __uint_as_float(o2[8 * i + 1]));
+          av.y = pack2<BF>(__uint_as_float(o2[8 * i + 2]), __uint_as_float(o2[8 * i + 3]));
+          av.z = pack2<BF>(__uint_as_float(o2[8 * i + 4]), __uint_as_float(o2[8 * i + 5]));
+          av.w = pack2<BF>(__uint_as_float(o2[8 * i + 6]), __uint_as_float(o2[8 * i + 7]));
+          st_swizzled_chunk(ytile, row, u * 4 + i, make_uint4(pack2<BF>(f[0], f[1]), pack2<BF>(f[2], f[3]), pack2<BF>(f[4], f[5]), pack2<BF>(f[6], f[7])));
+          st_swizzled_chunk(atile, row, u * 4 + i, av);
+          if (args.gain && !pad) {
+            const float4 g0 = __ldg(gp + 2 * i), g1 = __ldg(gp + 2 * i + 1);
+            st_swizzled_chunk(gtile, row, u * 4 + i, make_uint4(pack2<BF>(f[0] * g0.x, f[1] * g0.y), pack2<BF>(f[2] * g0.z, f[3] * g0.w),
+                                                        pack2<BF>(f[4] * g1.x, f[5] * g1.y), pack2<BF>(f[6] * g1.z, f[7] * g1.w)));
+          }
+        }
+        fence_proxy_async_smem();
+        hand_over(NB_STORE + br, NUM_SOFTMAX / 2 + 32);
+      }
+      if (write && !*abort_flag && u == 0) {
+        if (br == 0) {
+          args.lse1[grow] = m_fin[0] * args.sm_scale + logf(l_fin[0]);
+          args.rstd[grow] = rstd;
+        } else {
+          args.lse2[grow] = m_fin[1] * args.sm_scale + logf(l_fin[1]);
+        }
       }
     }
   }

@@ -51,6 +51,48 @@ __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.al
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// ------------------------------- work of a persistent CTA -----------------------------------
+// A persistent kernel runs min(items, SMs) CTAs; CTA c takes one item of every round of gridDim.x.  Without a mask items
+// run tile by tile through one (batch, head) after the other.  Under a causal mask the cost of a tile grows with its index (or falls,
+// on the key side), so a group of heads is walked from its heaviest tiles to its lightest and every other round runs
+// backwards: each CTA's sum comes out alike.
+struct WorkArgs {
+  int items, tiles, heads;     // tiles * heads; tiles per (batch, head); batch * heads
+  int group;                   // causal: heads walked together (0: no mask)
+  int heavy_last;              // causal: 1 = the last tile is the heaviest (query side), 0 = the first (key side)
+  uint32_t magic;              // ceil(2^32 / tiles) for w / tiles without a division; 0: one tile
+};
+struct WorkItem { int tile, bh; };
+template <bool LIST>          // false: one item per CTA, grid (tiles, heads)
+struct WorkList {
+  const WorkArgs& a;
+  int round = 0;
+  __device__ __forceinline__ explicit WorkList(const WorkArgs& args) : a(args) {}
+  __device__ __forceinline__ int index(int r) const {
+    return r * int(gridDim.x) + ((a.group && (r & 1)) ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x));
+  }
+  __device__ __forceinline__ bool valid() const { return LIST ? index(round) < a.items : round == 0; }
+  __device__ __forceinline__ bool has_next() const { return LIST && index(round + 1) < a.items; }
+  __device__ __forceinline__ void next() { ++round; }
+  // the compiler forgets what it knows about the round: item() is then computed again instead of kept in registers
+  __device__ __forceinline__ void forget() {
+    if (LIST) asm volatile("" : "+r"(round));
+  }
+  __device__ __forceinline__ WorkItem item() const {
+    if (!LIST) return WorkItem{int(blockIdx.x), int(blockIdx.y)};
+    const int w = index(round);
+    if (!a.group) {
+      // w < 2^32 and magic - 2^32 / tiles < 1: the product is at most one quotient too high
+      int bh = a.magic ? int(__umulhi(uint32_t(w), a.magic)) : w;
+      if ((long long)bh * a.tiles > w) --bh;
+      return WorkItem{w - bh * a.tiles, bh};
+    }
+    const int first = w / (a.group * a.tiles) * a.group, r = w - first * a.tiles, heads = min(a.group, a.heads - first);
+    const int rank = r / heads;
+    return WorkItem{a.heavy_last ? a.tiles - 1 - rank : rank, first + r % heads};
+  }
+};
+
 // ------------------------------------------ mbarrier -----------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
