@@ -21,7 +21,26 @@ from . import _lib
 EPS = 1e-5   # reference src/kernel.py:50
 
 
+_IO_DTYPES = (torch.float16, torch.bfloat16)
+_LAMBDA_DTYPES = {torch.float16: _lib.LAMBDA_F16, torch.bfloat16: _lib.LAMBDA_BF16, torch.float32: _lib.LAMBDA_F32}
+
+
+def _inputs_plainly_good(q1, q2, k1, k2, v, lam):
+    """All of `_check_inputs` as one expression, for calls that pass it; whatever it does not accept is looked at there."""
+    if not all(isinstance(t, torch.Tensor) for t in (q1, q2, k1, k2, v, lam)):
+        return False
+    dtype, device, shape = q1.dtype, q1.device, q1.shape
+    return (q1.is_cuda and dtype in _IO_DTYPES and len(shape) == 4
+            and q2.dtype == dtype and k1.dtype == dtype and k2.dtype == dtype and v.dtype == dtype
+            and q2.shape == shape and k1.shape == shape and k2.shape == shape
+            and v.shape == (shape[0], shape[1], shape[2], 2 * shape[3])
+            and q2.device == device and k1.device == device and k2.device == device and v.device == device
+            and lam.device == device and lam.numel() == 1 and lam.dtype in _LAMBDA_DTYPES)
+
+
 def _check_inputs(q1, q2, k1, k2, v, lambda_scale):
+    if _inputs_plainly_good(q1, q2, k1, k2, v, lambda_scale):
+        return
     if not torch.is_tensor(lambda_scale):
         raise TypeError("lambda_scale must be a 1-element CUDA tensor (the reference loads it from a "
                         "device pointer, src/kernel.py:138)")
@@ -67,6 +86,11 @@ def _tma_ready(t):
 
 def _same_layout(ts):
     """q1,q2,k1,k2 must share strides (the reference reads them from Q1 only, src/kernel.py:487-490)."""
+    a, b, c, d = ts
+    sb, sh, sn, sd = strides = a.stride()
+    if (sd == 1 and sb > 0 and sh > 0 and sn > 0 and not (sb | sh | sn) % 8 and b.stride() == strides and c.stride() == strides
+            and d.stride() == strides and not (a.data_ptr() | b.data_ptr() | c.data_ptr() | d.data_ptr()) % 16):
+        return ts          # (the common case: what the general rule below would return)
     ts = [_tma_ready(t) for t in ts]
     if any(t.stride() != ts[0].stride() for t in ts):
         ts = [t.contiguous() for t in ts]
@@ -87,14 +111,14 @@ def dropout_threshold(dropout_p: float) -> int:
 def _fill_common(p, q1, q2, k1, k2, v, lam, lambda_init, rms_norm, saved, causal=False, drop_threshold=0, drop_seed=0,
                  gain=None, y_gained=None, single_pass=False):
     b, h, n, d = q1.shape
-    p.device = q1.device.index if q1.device.index is not None else torch.cuda.current_device()
-    p.stream = torch.cuda.current_stream(q1.device).cuda_stream
+    p.device = q1.get_device()
+    p.stream = torch._C._cuda_getCurrentRawStream(p.device)      # the handle alone: a Stream object costs 3 us to build
     p.B, p.H, p.N, p.D = b, h, n, d
-    p.qk_stride_b, p.qk_stride_h, p.qk_stride_n = q1.stride(0), q1.stride(1), q1.stride(2)
-    p.v_stride_b, p.v_stride_h, p.v_stride_n = v.stride(0), v.stride(1), v.stride(2)
-    p.q1, p.q2, p.k1, p.k2, p.v = (t.data_ptr() for t in (q1, q2, k1, k2, v))
+    p.qk_stride_b, p.qk_stride_h, p.qk_stride_n, _ = q1.stride()
+    p.v_stride_b, p.v_stride_h, p.v_stride_n, _ = v.stride()
+    p.q1, p.q2, p.k1, p.k2, p.v = q1.data_ptr(), q2.data_ptr(), k1.data_ptr(), k2.data_ptr(), v.data_ptr()
     p.lambda_scale = lam.data_ptr()
-    p.lambda_dtype = {torch.float16: _lib.LAMBDA_F16, torch.bfloat16: _lib.LAMBDA_BF16}.get(lam.dtype, _lib.LAMBDA_F32)
+    p.lambda_dtype = _LAMBDA_DTYPES[lam.dtype]
     p.io_dtype = _lib.IO_BF16 if q1.dtype == torch.bfloat16 else _lib.IO_F16
     p.rms_norm = 1 if rms_norm else 0
     p.causal = 1 if causal else 0
@@ -107,7 +131,7 @@ def _fill_common(p, q1, q2, k1, k2, v, lam, lambda_init, rms_norm, saved, causal
     p.lambda_init = float(lambda_init)
     p.eps = EPS
     y, a2, lse1, lse2, rstd = saved
-    p.y, p.a2, p.lse1, p.lse2, p.rstd = (t.data_ptr() for t in (y, a2, lse1, lse2, rstd))
+    p.y, p.a2, p.lse1, p.lse2, p.rstd = y.data_ptr(), a2.data_ptr(), lse1.data_ptr(), lse2.data_ptr(), rstd.data_ptr()
 
 
 class DiffAttnFunction(torch.autograd.Function):
@@ -125,18 +149,18 @@ class DiffAttnFunction(torch.autograd.Function):
         v = _tma_ready(v)
         b, h, n, d = q1.shape
         dev = q1.device
-        with torch.cuda.device(dev):
-            y = torch.empty((b, h, n, 2 * d), dtype=v.dtype, device=dev)
-            a2 = torch.empty_like(y)
-            lse1 = torch.empty((b, h, n), dtype=torch.float32, device=dev)
-            lse2 = torch.empty_like(lse1)
-            rstd = torch.empty_like(lse1)
-            gain32 = gain.detach().to(torch.float32).contiguous() if gain is not None else None
-            y_gained = torch.empty_like(y) if gain is not None else None
-            p = _lib.new_params()
-            _fill_common(p, q1, q2, k1, k2, v, lambda_scale, lambda_init, rms_norm, (y, a2, lse1, lse2, rstd), causal,
-                         drop_threshold, drop_seed, gain32, y_gained)
-            _lib.check(_lib.lib.diffattn_fwd(p), "diffattn_fwd")
+        # (no device context: every allocation names its device, and the library makes the call's device current by itself)
+        y = torch.empty((b, h, n, 2 * d), dtype=v.dtype, device=dev)
+        a2 = torch.empty_like(y)
+        lse1 = torch.empty((b, h, n), dtype=torch.float32, device=dev)
+        lse2 = torch.empty_like(lse1)
+        rstd = torch.empty_like(lse1)
+        gain32 = gain.detach().to(torch.float32).contiguous() if gain is not None else None
+        y_gained = torch.empty_like(y) if gain is not None else None
+        p = _lib.new_params()
+        _fill_common(p, q1, q2, k1, k2, v, lambda_scale, lambda_init, rms_norm, (y, a2, lse1, lse2, rstd), causal,
+                     drop_threshold, drop_seed, gain32, y_gained)
+        _lib.check(_lib.lib.diffattn_fwd(p), "diffattn_fwd")
         ctx.save_for_backward(q1, q2, k1, k2, v, lambda_scale, y, a2, lse1, lse2, rstd)
         ctx.gain32 = gain32
         ctx.gain_dtype = gain.dtype if gain is not None else None
@@ -153,24 +177,23 @@ class DiffAttnFunction(torch.autograd.Function):
         b, h, n, d = q1.shape
         dev = q1.device
         dy = dy.to(v.dtype).contiguous()   # the kernels index dY densely (as src/kernel.py:278-280)
-        with torch.cuda.device(dev):
-            dq1 = torch.empty((b, h, n, d), dtype=q1.dtype, device=dev)
-            dq2, dk1, dk2 = torch.empty_like(dq1), torch.empty_like(dq1), torch.empty_like(dq1)
-            dv = torch.empty((b, h, n, 2 * d), dtype=v.dtype, device=dev)
-            dlam = torch.zeros(1, dtype=torch.float32, device=dev)
-            p = _lib.new_params()
-            dgain = torch.zeros(2 * d, dtype=torch.float32, device=dev) if ctx.gain32 is not None else None
-            _fill_common(p, q1, q2, k1, k2, v, lam, ctx.lambda_init, ctx.rms_norm, (y, a2, lse1, lse2, rstd), ctx.causal,
-                         *ctx.drop, ctx.gain32, y, ctx.single_pass)     # y_gained is not read by the backward
-            if dgain is not None:
-                p.dgain = dgain.data_ptr()
-            nbytes = int(_lib.lib.diffattn_workspace_bytes(p))
-            ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=dev)
-            p.dy = dy.data_ptr()
-            p.dq1, p.dq2, p.dk1, p.dk2, p.dv = (t.data_ptr() for t in (dq1, dq2, dk1, dk2, dv))
-            p.dlambda = dlam.data_ptr()
-            p.workspace, p.workspace_bytes = ws.data_ptr(), nbytes
-            _lib.check(_lib.lib.diffattn_bwd(p), "diffattn_bwd")
+        dq1 = torch.empty((b, h, n, d), dtype=q1.dtype, device=dev)
+        dq2, dk1, dk2 = torch.empty_like(dq1), torch.empty_like(dq1), torch.empty_like(dq1)
+        dv = torch.empty((b, h, n, 2 * d), dtype=v.dtype, device=dev)
+        dlam = torch.zeros(1, dtype=torch.float32, device=dev)
+        p = _lib.new_params()
+        dgain = torch.zeros(2 * d, dtype=torch.float32, device=dev) if ctx.gain32 is not None else None
+        _fill_common(p, q1, q2, k1, k2, v, lam, ctx.lambda_init, ctx.rms_norm, (y, a2, lse1, lse2, rstd), ctx.causal,
+                     *ctx.drop, ctx.gain32, y, ctx.single_pass)     # y_gained is not read by the backward
+        if dgain is not None:
+            p.dgain = dgain.data_ptr()
+        nbytes = int(_lib.lib.diffattn_workspace_bytes(p))
+        ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=dev)
+        p.dy = dy.data_ptr()
+        p.dq1, p.dq2, p.dk1, p.dk2, p.dv = (t.data_ptr() for t in (dq1, dq2, dk1, dk2, dv))
+        p.dlambda = dlam.data_ptr()
+        p.workspace, p.workspace_bytes = ws.data_ptr(), nbytes
+        _lib.check(_lib.lib.diffattn_bwd(p), "diffattn_bwd")
         # fp32 partial kept for callers that shard (batch*head) and sum partials themselves
         DiffAttnFunction.last_dlambda_fp32 = dlam
         dlam_out = dlam.to(lam.dtype).reshape(lam.shape) if ctx.needs_input_grad[5] else None
