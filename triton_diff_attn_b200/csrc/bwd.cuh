@@ -67,29 +67,30 @@ __device__ __forceinline__ float4 stat_row(const float4* stats, size_t idx) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// 1. preprocess: one warp per row, DV = 32 * VPL halves per row
+// 1. preprocess: HBM-bound (three [N, 2D] tensors in, one out).  A lane holds 8 elements (16-byte loads and stores), DV / 8
+// lanes share a row, so a warp works on 4, 2 or 1 rows at head dims 32, 64, 128 and a row's sums take 3 to 5 shuffles.
+// One such row set per warp and trip, four CTAs per SM: the other warps keep enough bytes in flight (two or four sets loaded before
+// the first reduction cost registers and were slower: 60 / 70 / 93 us at B4 H16 N4096 D64).  Against a row per warp with 4, 8 and 16
+// bytes per lane: B8 H16 N2048 D32 64 -> 31 us, B4 H16 N4096 D64 84 -> 60 (4.6 TB/s), B2 H8 N8192 D128 81 -> 67.
 // ------------------------------------------------------------------------------------------------
-template <int VPL, bool BF>   // 16-bit elements per lane: 2 (DV=64), 4 (DV=128), 8 (DV=256); BF: bf16 tensors
-__global__ void __launch_bounds__(256) diffattn_bwd_pre_kernel(const BwdArgs args) {
-  // rows per warp and trip (see below).  Measured at B4 H16 N4096 D64: 1 / 2 / 3 / 4 / 8 rows 0.103 / 0.072 / 0.078 / 0.093 /
-  // 0.089 ms (two rows keep the kernel at 63 registers, four resident CTAs per SM); at D = 128 and D = 32 four rows are
-  // as good or better (0.062 ms each).
-  constexpr int PRE_ROWS = VPL == 4 ? 2 : 4;
-  constexpr int DV = 32 * VPL;
+template <int DV, bool BF>   // value width 64, 128, 256; BF: bf16 tensors
+__global__ void __launch_bounds__(256, 4) diffattn_bwd_pre_kernel(const BwdArgs args) {
+  constexpr int LANES = DV / 8, SETS = 32 / LANES;      // lanes per row, rows per warp
   griddep_launch();      // the first tensor-core kernel may set itself up; it waits for this one before it reads dA or the statistics
   constexpr float LOG2E = 1.4426950408889634f;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  const long long warps_total = (long long)gridDim.x * (blockDim.x >> 5);
+  const int sub = lane % LANES;                          // this lane's 8 columns: [8 sub, 8 sub + 8)
+  const uint32_t rows = uint32_t(args.rows), n = uint32_t(args.n);      // (rows < 2^31: a row is at least 128 bytes)
   const float lam = load_lambda(args.lambda_ptr, args.lambda_dtype);
   const float c = args.out_scale;
   float dl_acc = 0.f;
   __shared__ float red[8];
   // learnable gain of the output norm: Y_out = Y * gain, so dY = dY_out * gain and d(gain) = sum over rows of dY_out * Y
   const bool has_gain = args.gain != nullptr;
-  float gn[VPL], dg_acc[VPL];
+  float gn[8], dg_acc[8];
 #pragma unroll
-  for (int i = 0; i < VPL; ++i) { gn[i] = has_gain ? args.gain[lane * VPL + i] : 1.f; dg_acc[i] = 0.f; }
+  for (int i = 0; i < 8; ++i) { gn[i] = has_gain ? args.gain[sub * 8 + i] : 1.f; dg_acc[i] = 0.f; }
   __shared__ float dg_red[8][DV];
   // the dQ partial sums of the single-pass backward start from zero
   if (args.dq_acc) {
@@ -97,7 +98,6 @@ __global__ void __launch_bounds__(256) diffattn_bwd_pre_kernel(const BwdArgs arg
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < args.dq_acc_f4; t += (long long)gridDim.x * blockDim.x)
       z[t] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-
   // rows N..n_pad-1 of every (batch, head) in `stats`: neutral values (see BwdArgs::n_pad)
   if (const int pad = args.n_pad - args.n) {
     const long long total = args.rows / args.n * pad;
@@ -106,101 +106,85 @@ __global__ void __launch_bounds__(256) diffattn_bwd_pre_kernel(const BwdArgs arg
       stat_store(args.stats, bh_i * args.n_pad + args.n + (i - bh_i * pad), make_float4(-INFINITY, -INFINITY, 0.f, 0.f));
     }
   }
-  // PRE_ROWS rows per warp and trip: all their loads are issued before the first reduction, which keeps that many
-  // times the bytes in flight per warp (one row per trip ran at 26 % of the DRAM rate: the shuffles of a row's two
-  // reductions sat between its loads and the next row's).
-  const long long first = (long long)blockIdx.x * (blockDim.x >> 5) + warp;
-  for (long long row0 = first; row0 < args.rows; row0 += warps_total * PRE_ROWS) {
-    __align__(16) __half hdr[PRE_ROWS][VPL], hyr[PRE_ROWS][VPL], har[PRE_ROWS][VPL];
-    float rsr[PRE_ROWS], l1r[PRE_ROWS], l2r[PRE_ROWS];
-#pragma unroll
-    for (int rr = 0; rr < PRE_ROWS; ++rr) {
-      const long long row = row0 + rr * warps_total;
-      if (row < args.rows) {
-        const size_t off = size_t(row) * DV + lane * VPL;
-        __half* hd = hdr[rr]; __half* hy = hyr[rr]; __half* ha = har[rr];
-        if constexpr (VPL == 8) {
-          *reinterpret_cast<uint4*>(hd) = *reinterpret_cast<const uint4*>(args.dy + off);
-          *reinterpret_cast<uint4*>(hy) = *reinterpret_cast<const uint4*>(args.y + off);
-          *reinterpret_cast<uint4*>(ha) = *reinterpret_cast<const uint4*>(args.a2 + off);
-        } else if constexpr (VPL == 4) {
-          *reinterpret_cast<uint2*>(hd) = *reinterpret_cast<const uint2*>(args.dy + off);
-          *reinterpret_cast<uint2*>(hy) = *reinterpret_cast<const uint2*>(args.y + off);
-          *reinterpret_cast<uint2*>(ha) = *reinterpret_cast<const uint2*>(args.a2 + off);
-        } else {
-          *reinterpret_cast<uint32_t*>(hd) = *reinterpret_cast<const uint32_t*>(args.dy + off);
-          *reinterpret_cast<uint32_t*>(hy) = *reinterpret_cast<const uint32_t*>(args.y + off);
-          *reinterpret_cast<uint32_t*>(ha) = *reinterpret_cast<const uint32_t*>(args.a2 + off);
-        }
-        rsr[rr] = args.rstd[row]; l1r[rr] = args.lse1[row]; l2r[rr] = args.lse2[row];
-      }
+
+  const uint32_t step = gridDim.x * (blockDim.x >> 5) * SETS;           // rows of one trip of the grid
+  for (uint32_t row = (blockIdx.x * (blockDim.x >> 5) + warp) * SETS + lane / LANES; row - lane / LANES < rows; row += step) {
+    uint4 vd, vy, va;
+    float rstd = 1.f, lse1 = 0.f, lse2 = 0.f;
+    vd = vy = va = make_uint4(0, 0, 0, 0);               // (lanes past the last row take part in the shuffles)
+    if (row < rows) {
+      const size_t off = size_t(row) * DV + sub * 8;
+      vd = *reinterpret_cast<const uint4*>(args.dy + off);
+      vy = *reinterpret_cast<const uint4*>(args.y + off);
+      va = *reinterpret_cast<const uint4*>(args.a2 + off);
+      rstd = args.rstd[row]; lse1 = args.lse1[row]; lse2 = args.lse2[row];
     }
+    float dy[8], yv[8];
+    const uint32_t wd[4] = {vd.x, vd.y, vd.z, vd.w}, wy[4] = {vy.x, vy.y, vy.z, vy.w};
+    const uint32_t wa[4] = {va.x, va.y, va.z, va.w};
 #pragma unroll
-    for (int rr = 0; rr < PRE_ROWS; ++rr) {      // (body kept at the indentation of the one-row loop it came from)
-    const long long row = row0 + rr * warps_total;
-    if (row >= args.rows) break;
-    const size_t off = size_t(row) * DV + lane * VPL;
-    const __half* hd = hdr[rr]; const __half* hy = hyr[rr]; const __half* ha = har[rr];
-    float dy[VPL], yv[VPL], a2[VPL];
-    {
-#pragma unroll
-      for (int i = 0; i < VPL; ++i) { dy[i] = to_float16b<BF>(hd[i]); yv[i] = to_float16b<BF>(hy[i]); a2[i] = to_float16b<BF>(ha[i]); }
+    for (int i = 0; i < 4; ++i) {
+      const float2 fd = unpack2<BF>(wd[i]), fy = unpack2<BF>(wy[i]);
+      dy[2 * i] = fd.x; dy[2 * i + 1] = fd.y;
+      yv[2 * i] = fy.x; yv[2 * i + 1] = fy.y;
     }
     if (has_gain) {
 #pragma unroll
-      for (int i = 0; i < VPL; ++i) { dg_acc[i] = fmaf(dy[i], yv[i], dg_acc[i]); dy[i] *= gn[i]; }
+      for (int i = 0; i < 8; ++i) { dg_acc[i] = fmaf(dy[i], yv[i], dg_acc[i]); dy[i] *= gn[i]; }
     }
-    float da[VPL], av[VPL];
+    float k1 = 1.f, k2 = 0.f, k3 = 1.f;
     if (args.rms_norm) {
       // Y = c r A  =>  A = Y/(c r),  dA = r (c dY - Y (dY.Y) / (c Dv));  c == 0 gives dA = 0
       float t = 0.f;
 #pragma unroll
-      for (int i = 0; i < VPL; ++i) t += dy[i] * yv[i];
+      for (int i = 0; i < 8; ++i) t += dy[i] * yv[i];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      const float r = rsr[rr];
+      for (int o = LANES / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
       const float inv_c = c != 0.f ? 1.f / c : 0.f;
-      const float k1 = r * c, k2 = r * inv_c * t * (1.f / DV), k3 = inv_c / r;
-#pragma unroll
-      for (int i = 0; i < VPL; ++i) { da[i] = k1 * dy[i] - k2 * yv[i]; av[i] = yv[i] * k3; }
-    } else {
-#pragma unroll
-      for (int i = 0; i < VPL; ++i) { da[i] = dy[i]; av[i] = yv[i]; }
+      k1 = rstd * c; k2 = rstd * inv_c * t * (1.f / DV); k3 = inv_c / rstd;
     }
     // round dA to the 16-bit type first: the row sums below must agree with what the MMAs will see
-    __half hda[VPL];
+    uint32_t hda[4];
     float e2 = 0.f, ea = 0.f;
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      hda[i] = from_float16b<BF>(da[i]);
-      const float d = to_float16b<BF>(hda[i]);
-      e2 += d * a2[i];
-      ea += d * av[i];
+    for (int i = 0; i < 4; ++i) {
+      hda[i] = args.rms_norm ? pack2<BF>(k1 * dy[2 * i] - k2 * yv[2 * i], k1 * dy[2 * i + 1] - k2 * yv[2 * i + 1])
+                             : pack2<BF>(dy[2 * i], dy[2 * i + 1]);
+      const float2 d = unpack2<BF>(hda[i]), a2 = unpack2<BF>(wa[i]);
+      e2 += d.x * a2.x + d.y * a2.y;
+      ea += d.x * (yv[2 * i] * k3) + d.y * (yv[2 * i + 1] * k3);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = LANES / 2; o > 0; o >>= 1) {
       e2 += __shfl_xor_sync(0xffffffffu, e2, o);
       ea += __shfl_xor_sync(0xffffffffu, ea, o);
     }
-    if constexpr (VPL == 8) *reinterpret_cast<uint4*>(args.da + off) = *reinterpret_cast<uint4*>(hda);
-    else if constexpr (VPL == 4) *reinterpret_cast<uint2*>(args.da + off) = *reinterpret_cast<uint2*>(hda);
-    else *reinterpret_cast<uint32_t*>(args.da + off) = *reinterpret_cast<uint32_t*>(hda);
-    if (lane == 0) {
-      // E1 - lam E2 = rowsum(dA * A).  lambda is folded into the branch-2 statistics so that the tensor-core
-      // kernels need no multiply for it: with P2' = |lam| P2 = 2^(s S2 log2e - y) and sg = -sign(lam),
-      // -lam P2 = sg P2' and -lam P2 (dP - E2) = P2' (sg dP - w).  lam = 0 gives y = +inf, P2' = 0.
-      const float sg = lam < 0.f ? 1.f : -1.f;
-      const long long bh_i = row / args.n;
-      stat_store(args.stats, bh_i * args.n_pad + (row - bh_i * args.n),
-                 make_float4(-l1r[rr] * LOG2E, log2f(fabsf(lam)) - l2r[rr] * LOG2E, -(ea + lam * e2), -sg * e2));
-      dl_acc -= e2;
+    if (row < rows) {
+      *reinterpret_cast<uint4*>(args.da + size_t(row) * DV + sub * 8) = make_uint4(hda[0], hda[1], hda[2], hda[3]);
+      if (sub == 0) {
+        // E1 - lam E2 = rowsum(dA * A).  lambda is folded into the branch-2 statistics so that the tensor-core
+        // kernels need no multiply for it: with P2' = |lam| P2 = 2^(s S2 log2e - y) and sg = -sign(lam),
+        // -lam P2 = sg P2' and -lam P2 (dP - E2) = P2' (sg dP - w).  lam = 0 gives y = +inf, P2' = 0.
+        const float sg = lam < 0.f ? 1.f : -1.f;
+        const uint32_t bh_i = row / n;
+        stat_store(args.stats, (long long)bh_i * args.n_pad + (row - bh_i * n),
+                   make_float4(-lse1 * LOG2E, log2f(fabsf(lam)) - lse2 * LOG2E, -(ea + lam * e2), -sg * e2));
+        dl_acc -= e2;
+      }
     }
   }
+#pragma unroll
+  for (int o = LANES; o < 32; o <<= 1) {       // the row sets of the warp
+    dl_acc += __shfl_xor_sync(0xffffffffu, dl_acc, o);
+    if (has_gain) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) dg_acc[i] += __shfl_xor_sync(0xffffffffu, dg_acc[i], o);
+    }
   }
   if (lane == 0) red[warp] = dl_acc;
-  if (has_gain) {
+  if (has_gain && lane < LANES) {
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) dg_red[warp][lane * VPL + i] = dg_acc[i];
+    for (int i = 0; i < 8; ++i) dg_red[warp][sub * 8 + i] = dg_acc[i];
   }
   __syncthreads();
   if (threadIdx.x == 0) {

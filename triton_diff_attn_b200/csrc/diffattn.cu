@@ -427,11 +427,11 @@ int bwd_impl(const DiffAttnParams* p, int32_t stages) {
 
   // 1. preprocess (grid-stride; one atomic per CTA for d(lambda)); zeroes the dQ partial sums of the single-pass form
   if (stages & DIFFATTN_STAGE_PRE) {
-    long long blocks = (long long)((rows + 7) / 8);
-    if (blocks > (long long)sms * 8) blocks = (long long)sms * 8;
-    if (D == 128) da::diffattn_bwd_pre_kernel<8, BF><<<(unsigned)blocks, 256, 0, stream>>>(a);
-    else if (D == 64) da::diffattn_bwd_pre_kernel<4, BF><<<(unsigned)blocks, 256, 0, stream>>>(a);
-    else da::diffattn_bwd_pre_kernel<2, BF><<<(unsigned)blocks, 256, 0, stream>>>(a);
+    const uint64_t rows_per_cta = 8 * (256 / DV);
+    const unsigned blocks = (unsigned)std::min<uint64_t>((rows + rows_per_cta - 1) / rows_per_cta, uint64_t(sms) * 8);
+    if (D == 128) da::diffattn_bwd_pre_kernel<256, BF><<<blocks, 256, 0, stream>>>(a);
+    else if (D == 64) da::diffattn_bwd_pre_kernel<128, BF><<<blocks, 256, 0, stream>>>(a);
+    else da::diffattn_bwd_pre_kernel<64, BF><<<blocks, 256, 0, stream>>>(a);
     DA_CUDA(cudaGetLastError());
   }
   if (D == 128) {
