@@ -144,6 +144,15 @@ int diffattn_bwd_stages(const DiffAttnParams* p, int32_t stages);
 #define DIFFATTN_STATIC_SCRATCH_BYTES (32u << 20)
 int diffattn_bwd_static(const DiffAttnParams* p);
 
+/* The re-parameterisation of lambda in the layer around the operator (src/layers.py:114 names that layer; the reference itself
+ * takes lambda ready-made): out = { exp(<q1,k1>) - exp(<q2,k2>) + lambda_init, exp(<q1,k1>), exp(<q2,k2>) } from four fp32 vectors of
+ * n elements, and the vectors' gradients from dlambda (one fp32) and that `out`.  One kernel each, enqueued on `stream`; every
+ * pointer is device memory of `device`. */
+int diffattn_lambda_fwd(int32_t device, void* stream, int32_t n, const float* q1, const float* k1, const float* q2, const float* k2,
+                        float lambda_init, float* out);
+int diffattn_lambda_bwd(int32_t device, void* stream, int32_t n, const float* q1, const float* k1, const float* q2, const float* k2,
+                        const float* out, const float* dlambda, float* dq1, float* dk1, float* dq2, float* dk2);
+
 /* Scratch bytes diffattn_bwd needs for these shapes and p->single_pass (the reference allocates its
  * D1/D2 and dLambda partial buffers itself, src/kernel.py:522-529).  The forward needs none. */
 uint64_t diffattn_workspace_bytes(const DiffAttnParams* p);

@@ -107,3 +107,29 @@ def test_several_tiles_per_cta(b, h, n, d, causal, p, gain):
         # the repository's fp16 bound, for each head: a wrong tile must not hide among the others
         err = (got.float().cpu() - ref.float()).flatten(2).norm(dim=2)
         assert bool((err <= 2e-3 * ref.float().flatten(2).norm(dim=2)).all()), (name, float((err / ref.float().flatten(2).norm(dim=2)).max()))
+
+
+@pytest.mark.parametrize("n", [1, 32, 64, 128, 300])
+@pytest.mark.parametrize("create_graph", [False, True])
+def test_core_lambda_in_one_launch(n, create_graph):
+    """lambda and the four vectors' gradients against 64 bits: sums of n products and one exponential in fp32."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import triton_diff_attn_b200 as pkg
+    dev = torch.device("cuda", 0)
+    gen = torch.Generator().manual_seed(n)
+    host = [torch.randn(n, generator=gen) * 0.2 for _ in range(4)]
+    ref = [t.double().requires_grad_(True) for t in host]
+    want = torch.exp((ref[0] * ref[1]).sum()) - torch.exp((ref[2] * ref[3]).sum()) + 0.8
+    wg = torch.autograd.grad(want, ref, torch.tensor(1.7, dtype=torch.float64))
+    vec = [torch.nn.Parameter(t.to(dev)) for t in host]
+    lam = pkg.layers._core_lambda(vec, 0.8, vec[0].device)
+    got = torch.autograd.grad(lam, vec, torch.full((1,), 1.7, device=dev), create_graph=create_graph)
+    # n products of at most 1 in magnitude summed in fp32 (n 2^-24), an exponential of |x| < 10 (2^-22), a difference of O(1) terms
+    assert abs(float(lam.detach()) - float(want.detach())) <= 1e-5 * (1 + abs(float(want.detach())))
+    for a, b in zip(got, wg):
+        assert torch.allclose(a.detach().cpu().double(), b, rtol=1e-5, atol=1e-6)
+    if create_graph:
+        assert all(t is not None for t in torch.autograd.grad(sum(t.sum() for t in got), vec))
+    half = [t.half().to(dev) for t in host]                      # anything but fp32 goes through tensor operations as before
+    assert torch.equal(pkg.layers._core_lambda(half, 0.8, dev), pkg.lambda_from_reparam(*half, 0.8))

@@ -12,7 +12,7 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 # DIFFATTN_LIBRARY names another build of the same library (for instance one compiled with other tuning macros)
 LIB_PATH = os.environ.get("DIFFATTN_LIBRARY") or os.path.join(PKG_DIR, "libdiffattn.so")
 
-EXPORTS = ("diffattn_fwd", "diffattn_bwd", "diffattn_bwd_stages", "diffattn_bwd_static", "diffattn_workspace_bytes", "diffattn_status",
+EXPORTS = ("diffattn_fwd", "diffattn_bwd", "diffattn_bwd_stages", "diffattn_bwd_static", "diffattn_lambda_fwd", "diffattn_lambda_bwd", "diffattn_workspace_bytes", "diffattn_status",
            "diffattn_last_error", "diffattn_version", "diffattn_supports")
 
 ERR_NAMES = {
@@ -61,6 +61,10 @@ def _load() -> C.CDLL:
     lib.diffattn_bwd_stages.restype = C.c_int
     lib.diffattn_bwd_static.argtypes = [C.POINTER(DiffAttnParams)]
     lib.diffattn_bwd_static.restype = C.c_int
+    lib.diffattn_lambda_fwd.argtypes = [C.c_int32, C.c_void_p, C.c_int32] + [C.c_void_p] * 4 + [C.c_float, C.c_void_p]
+    lib.diffattn_lambda_fwd.restype = C.c_int
+    lib.diffattn_lambda_bwd.argtypes = [C.c_int32, C.c_void_p, C.c_int32] + [C.c_void_p] * 10
+    lib.diffattn_lambda_bwd.restype = C.c_int
     lib.diffattn_workspace_bytes.argtypes = [C.POINTER(DiffAttnParams)]
     lib.diffattn_workspace_bytes.restype = C.c_uint64
     lib.diffattn_status.argtypes = [C.c_int32]

@@ -19,6 +19,7 @@
 #include "fwd.cuh"
 #include "fwd64.cuh"
 #include "fwd128.cuh"
+#include "lambda.cuh"
 #include "sm100.cuh"
 
 namespace {
@@ -528,6 +529,21 @@ int bwd_impl(const DiffAttnParams* p, int32_t stages) {
   return DIFFATTN_OK;
 }
 
+int lambda_impl(int32_t device, void* stream, bool bwd, const da::LambdaArgs& a) {
+  if (a.n <= 0) return fail(DIFFATTN_ERR_BAD_SHAPE, "lambda vectors of %d elements", a.n);
+  DeviceGuard guard;
+  int rc = guard.enter(device);
+  if (rc) return rc;
+  const void* ptrs[] = {a.q1, a.k1, a.q2, a.k2, a.out, a.dlambda, a.dq1, a.dk1, a.dq2, a.dk2};
+  const char* names[] = {"q1", "k1", "q2", "k2", "out", "dlambda", "dq1", "dk1", "dq2", "dk2"};
+  for (int i = 0; i < (bwd ? 10 : 5); ++i) {
+    if (!ptrs[i]) return fail(DIFFATTN_ERR_NULL_PTR, "%s is NULL", names[i]);
+    if ((rc = check_on_device(ptrs[i], device, names[i]))) return rc;
+  }
+  return launch(bwd ? da::diffattn_lambda_bwd_kernel : da::diffattn_lambda_fwd_kernel, dim3(1), da::LAMBDA_THREADS, 0, static_cast<cudaStream_t>(stream),
+                false, a);
+}
+
 int all_stages(const DiffAttnParams* p) {
   return fused_form(p) ? (DIFFATTN_STAGE_PRE | DIFFATTN_STAGE_FUSED | DIFFATTN_STAGE_DQ_FINISH)
                        : (DIFFATTN_STAGE_PRE | DIFFATTN_STAGE_DKDV | DIFFATTN_STAGE_DQ);
@@ -623,6 +639,16 @@ int diffattn_bwd_static(const DiffAttnParams* p) {
   q.workspace = scratch;
   q.workspace_bytes = DIFFATTN_STATIC_SCRATCH_BYTES;
   return diffattn_bwd_stages(&q, all_stages(&q));
+}
+
+int diffattn_lambda_fwd(int32_t device, void* stream, int32_t n, const float* q1, const float* k1, const float* q2, const float* k2,
+                        float lambda_init, float* out) {
+  return lambda_impl(device, stream, false, {q1, k1, q2, k2, n, lambda_init, out, nullptr, nullptr, nullptr, nullptr, nullptr});
+}
+
+int diffattn_lambda_bwd(int32_t device, void* stream, int32_t n, const float* q1, const float* k1, const float* q2, const float* k2,
+                        const float* out, const float* dlambda, float* dq1, float* dk1, float* dq2, float* dk2) {
+  return lambda_impl(device, stream, true, {q1, k1, q2, k2, n, 0.f, const_cast<float*>(out), dlambda, dq1, dk1, dq2, dk2});
 }
 
 int diffattn_status(int32_t device) {

@@ -180,9 +180,12 @@ class DiffAttnFunction(torch.autograd.Function):
         dq1 = torch.empty((b, h, n, d), dtype=q1.dtype, device=dev)
         dq2, dk1, dk2 = torch.empty_like(dq1), torch.empty_like(dq1), torch.empty_like(dq1)
         dv = torch.empty((b, h, n, 2 * d), dtype=v.dtype, device=dev)
-        dlam = torch.zeros(1, dtype=torch.float32, device=dev)
+        if ctx.gain32 is None:
+            dgain, dlam = None, torch.zeros(1, dtype=torch.float32, device=dev)
+        else:
+            zeros = torch.zeros(2 * d + 1, dtype=torch.float32, device=dev)      # one launch for both
+            dgain, dlam = zeros[:2 * d], zeros[2 * d:]
         p = _lib.new_params()
-        dgain = torch.zeros(2 * d, dtype=torch.float32, device=dev) if ctx.gain32 is not None else None
         _fill_common(p, q1, q2, k1, k2, v, lam, ctx.lambda_init, ctx.rms_norm, (y, a2, lse1, lse2, rstd), ctx.causal,
                      *ctx.drop, ctx.gain32, y, ctx.single_pass)     # y_gained is not read by the backward
         if dgain is not None:
@@ -252,6 +255,43 @@ def lambda_from_reparam(lambda_q1, lambda_k1, lambda_q2, lambda_k2, lambda_init:
     return (l1 - l2 + float(lambda_init)).reshape(1)
 
 
+class _LambdaReparam(torch.autograd.Function):
+    """`lambda_from_reparam` in one launch each way, for fp32 vectors on one GPU."""
+
+    @staticmethod
+    def forward(ctx, q1, k1, q2, k2, lambda_init):
+        out = torch.empty(3, dtype=torch.float32, device=q1.device)      # lambda, exp(<q1, k1>), exp(<q2, k2>)
+        dev = q1.get_device()
+        _lib.check(_lib.lib.diffattn_lambda_fwd(dev, torch._C._cuda_getCurrentRawStream(dev), q1.numel(), q1.data_ptr(), k1.data_ptr(),
+                                                q2.data_ptr(), k2.data_ptr(), lambda_init, out.data_ptr()), "diffattn_lambda_fwd")
+        ctx.save_for_backward(q1, k1, q2, k2, out)
+        return out[:1]
+
+    @staticmethod
+    def backward(ctx, g):
+        q1, k1, q2, k2, out = ctx.saved_tensors
+        if torch.is_grad_enabled():          # create_graph=True: the gradients have to be differentiable themselves
+            g1, g2 = g * torch.exp(torch.sum(q1 * k1)), -g * torch.exp(torch.sum(q2 * k2))
+            return g1 * k1, g1 * q1, g2 * k2, g2 * q2, None
+        g = g.contiguous()
+        d = [torch.empty_like(t) for t in (q1, k1, q2, k2)]
+        dev = q1.get_device()
+        _lib.check(_lib.lib.diffattn_lambda_bwd(dev, torch._C._cuda_getCurrentRawStream(dev), q1.numel(), q1.data_ptr(), k1.data_ptr(),
+                                                q2.data_ptr(), k2.data_ptr(), out.data_ptr(), g.data_ptr(), *[t.data_ptr() for t in d]),
+                   "diffattn_lambda_bwd")
+        return (*d, None)
+
+
+def _core_lambda(vectors, lambda_init, device):
+    """lambda of a `DiffAttnCore`: one launch where the four vectors are plain dense fp32 vectors of one length on the inputs' GPU,
+    tensor operations for everything else (other types, moved or replaced parameters)."""
+    a = vectors[0]
+    if all(type(t) in (torch.nn.Parameter, torch.Tensor) and t.is_cuda and t.dtype == torch.float32 and t.dim() == 1 and t.is_contiguous()
+           and t.shape == a.shape and t.device == device for t in vectors) and a.numel() > 0:
+        return _LambdaReparam.apply(*vectors, lambda_init)
+    return lambda_from_reparam(*vectors, lambda_init)
+
+
 class DiffAttnCore(torch.nn.Module):
     """The attention core of a differential-attention layer around the operator: owns the four lambda vectors
     and the output norm's gain, forms lambda on the device and calls `MultiheadDiffAttnKernel` with rms_norm on.
@@ -266,7 +306,7 @@ class DiffAttnCore(torch.nn.Module):
         self.lambda_init, self.causal, self.dropout_p = float(lambda_init), bool(causal), float(dropout_p)
 
     def forward(self, q1, q2, k1, k2, v):
-        lam = lambda_from_reparam(self.lambda_q1, self.lambda_k1, self.lambda_q2, self.lambda_k2, self.lambda_init)
+        lam = _core_lambda((self.lambda_q1, self.lambda_k1, self.lambda_q2, self.lambda_k2), self.lambda_init, q1.device)
         return MultiheadDiffAttnKernel(q1, q2, k1, k2, v, lam, self.lambda_init, True, causal=self.causal,
                                        dropout_p=self.dropout_p if self.training else 0.0, gain=self.gain)
 
