@@ -456,8 +456,6 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
     const float sg = load_lambda(args.lambda_ptr, args.lambda_dtype) < 0.f ? 1.f : -1.f;   // -sign(lambda)
     const f32x2 dscale_2 = pk2(args.drop_scale, args.drop_scale), sgd_2 = pk2(sg * args.drop_scale, sg * args.drop_scale);     // DROP only
     const f32x2 sl2_2 = pk2(sl2, sl2), sg_2 = pk2(sg, sg);
-    // (once a wait has given up the loop goes on without waiting, on whatever TMEM holds, and syncs on the named barriers
-    // instead of only arriving: nobody is left waiting and nobody runs ahead)
     bool ok = true;
     auto hand_over = [&](int id, int threads) {
       tc_fence_before();
@@ -478,16 +476,18 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
           dw1 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(wi.bh), 0u), col2, row & 1, args.drop_thresh);
           dw2 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(wi.bh), 1u), col2, row & 1, args.drop_thresh);
         }
-        for (int i = 0; i < nq; ++i) {
+        int i = 0;
+        for (; ok && i < nq; ++i) {
           const float4* stats = reinterpret_cast<const float4*>(smem + OFF_STAGE + st * STAGE_BYTES + 2 * Q_BYTES + DA_BYTES) + g * 16;
-          if (!__all_sync(0xffffffffu, s_ready)) ok = ok && mbar_wait_warp(&misc->s_full, i & 1, abort_flag, 601 + g, i);
+          if (!__all_sync(0xffffffffu, s_ready) && !mbar_wait_warp(&misc->s_full, i & 1, abort_flag, 601 + g, i)) { ok = false; break; }
           tc_fence_after();
           uint32_t s1[16], s2[16], dp[16];
           tmem_ld16(tb + T_S1 + g * 16, s1);
           tmem_ld16(tb + T_S2 + g * 16, s2);
           tmem_ld16(tb + T_DP + g * 16, dp);
           tc_wait_ld();
-          hand_over(NB_SFREE, NB_SFREE_THREADS);
+          tc_fence_before();
+          named_bar_arrive(NB_SFREE, NB_SFREE_THREADS);
           if (args.causal) {
             // this thread's key row sees query columns >= its own index only: the first c0 columns of its 16 are hidden
             const int c0 = row - (i * BQ + g * 16);          // kv_tile * BKV = i0 * BQ
@@ -550,7 +550,7 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           if (i > 0) {
-            if (!__all_sync(0xffffffffu, md_ready)) ok = ok && mbar_wait_warp(&misc->mma_done, (i - 1) & 1, abort_flag, 605 + g, i);
+            if (!__all_sync(0xffffffffu, md_ready)) ok = mbar_wait_warp(&misc->mma_done, (i - 1) & 1, abort_flag, 605 + g, i);
             tc_fence_after();
           }
           s_ready = i + 1 < nq ? mbar_probe(&misc->s_full, (i + 1) & 1) : 0u;
@@ -560,8 +560,15 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
           asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
                        ::"r"(tb + T_DS2 + g * 8), "r"(d2[0]), "r"(d2[1]), "r"(d2[2]), "r"(d2[3]), "r"(d2[4]), "r"(d2[5]), "r"(d2[6]), "r"(d2[7]) : "memory");
           tc_wait_st();
-          hand_over(NB_E + (i & 1), NB_E_THREADS);
+          tc_fence_before();
+          named_bar_arrive(NB_E + (i & 1), NB_E_THREADS);
           if (++st == ST) st = 0;
+        }
+        // after a wait that gave up: the named barriers of the query tiles left, synced on instead of arrived at, so that nobody is left
+        // waiting and nobody runs ahead
+        for (; i < nq; ++i) {
+          named_bar_sync(NB_SFREE, NB_SFREE_THREADS);
+          named_bar_sync(NB_E + (i & 1), NB_E_THREADS);
         }
       }
       work.forget();
@@ -829,8 +836,6 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
     const float sg = lam < 0.f ? 1.f : -1.f;       // branch 2: -sign(lambda) (|lambda| sits in its statistics, the sign in e)
     const float dscale = DROP ? args.drop_scale : 1.f;
     const f32x2 sl2_2 = pk2(sl2, sl2);
-    // (once a wait has given up the loop goes on without waiting, on whatever TMEM holds, and syncs on the named barriers
-    // instead of only arriving: nobody is left waiting and nobody runs ahead)
     bool ok = true;
     auto hand_over = [&](int id) {
       tc_fence_before();
@@ -877,30 +882,45 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
           dw1 = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 0u), row2, row & 1, args.drop_thresh);
           dw2 = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 1u), row2, row & 1, args.drop_thresh);
         }
-        for (int j = 0; j < nkv; ++j, ++done) {
+        int j = 0;
+        for (; ok && j < nkv; ++j, ++done) {
           // key columns past the sequence end or (causal) right of the diagonal: score -inf, probability 0
           const int c_first = j * BN + g * 32;
           int nv = args.n - c_first;
           if (args.causal) nv = min(nv, q_tile * BM + row - c_first + 1);
           uint32_t s[32], dp[32];
-          ok = ok && mbar_wait_warp(&misc->s_full[0], done & 1, abort_flag, 901, j);
+          if (!mbar_wait_warp(&misc->s_full[0], done & 1, abort_flag, 901, j)) { ok = false; break; }
           tc_fence_after();
           tmem_ld32(t_dp, dp);
           tmem_ld32(t_s1, s);
           tc_wait_ld();
-          hand_over(NB_DP);
+          tc_fence_before();
+          named_bar_arrive(NB_DP, NB_THREADS);
           branch(s, dp, nv, j, sv.x, sv.z, 1.f, dw1, [&] { if (done == 0 && g < 2) named_bar_arrive(NB_START, NWG * 128); });
           tmem_st16(t_s1, s);
           tc_wait_st();
-          hand_over(NB_DS1);
-          ok = ok && mbar_wait_warp(&misc->s_full[1], done & 1, abort_flag, 902, j);
+          tc_fence_before();
+          named_bar_arrive(NB_DS1, NB_THREADS);
+          ok = mbar_wait_warp(&misc->s_full[1], done & 1, abort_flag, 902, j);
           tc_fence_after();
           tmem_ld32(t_s2, s);
           tc_wait_ld();
           branch(s, dp, nv, j, sv.y, sv.w, sg, dw2, [] {});
           tmem_st16(t_s2, s);
           tc_wait_st();
-          hand_over(NB_DS2);
+          tc_fence_before();
+          named_bar_arrive(NB_DS2, NB_THREADS);
+        }
+        // after a wait that gave up: the named barriers of the tiles left, synced on instead of arrived at, so that nobody is left
+        // waiting and nobody runs ahead
+        if (!ok && done == 0) {          // given up before the first half branch: team 1 must not wait for it
+          if (g < 2) named_bar_arrive(NB_START, NWG * 128);
+          done = 1;
+        }
+        for (; j < nkv; ++j) {
+          named_bar_sync(NB_DP, NB_THREADS);
+          named_bar_sync(NB_DS1, NB_THREADS);
+          named_bar_sync(NB_DS2, NB_THREADS);
         }
       }
       work.forget();

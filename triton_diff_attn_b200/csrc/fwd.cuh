@@ -1,7 +1,7 @@
 // Differential-attention forward for sm_100a: what the forward kernels share (arguments, tile geometry of the
 // D <= 64 kernel).  The kernels themselves: fwd64.cuh (head dims 32 and 64), fwd128.cuh (head dim 128).
 //
-// One CTA owns one tile of 128 query rows of one (batch, head).  TMEM (512 columns of 128 lanes x 32 bit) at
+// A CTA works on one tile of 128 query rows of one (batch, head) at a time.  TMEM (512 columns of 128 lanes x 32 bit) at
 // D <= 64: S1 two 64-column buffers [0,128), S2 likewise [128,256), O1 [256,384), O2 [384,512).  Scores are
 // produced in sub-tiles of 64 key rows into alternating buffers, so the MMA for sub-tile t+1 runs while the
 // softmax warps work on sub-tile t.  P_b (16-bit, two per column) overwrites the first 32 columns of its S
