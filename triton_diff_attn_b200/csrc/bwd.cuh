@@ -327,7 +327,7 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
     for (; work.valid(); ++it, work.next()) {
       const WorkItem wi = work.item();
       const int b_idx = wi.bh / args.h, h_idx = wi.bh % args.h, i0 = first_q(wi.tile), nq = nq_all - i0;
-      if (it > 0) ok = ok && mbar_wait_warp(&misc->kv_empty, (it - 1) & 1, abort_flag, 402, it);
+      if (it > 0) ok = ok && mbar_wait_warp(&misc->kv_empty, (it - 1) & 1, abort_flag, 402, it) && !*abort_flag;      // (as mbar_wait_free)
       if (ok && elect_one()) {
         mbar_expect_tx(&misc->bar_kv, 2 * K_BYTES + V_BYTES);
         tma_load_4d(smem + OFF_K1, &tm_k1, &misc->bar_kv, 0, wi.tile * BKV, h_idx, b_idx);
@@ -343,7 +343,7 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
       __syncwarp();
       for (int i = 0; i < nq; ++i) {
         if (i == 1 && it > 0) store(st);     // (every tile has at least two query tiles)
-        ok = ok && mbar_wait_warp(&misc->empty[st], par, abort_flag, 401, i);
+        ok = ok && mbar_wait_warp(&misc->empty[st], par, abort_flag, 401, i) && !*abort_flag;
         if (ok && elect_one()) {
           uint8_t* sp = smem + OFF_STAGE + st * STAGE_BYTES;
           mbar_expect_tx(&misc->full[st], STAGE_BYTES);
@@ -364,7 +364,7 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
     // MMA issue is spread over three warps on three schedulers (these two and the output issuer below): one warp
     // issuing all 32 MMAs of a tile takes ~300 clocks per tile from the elementwise warps of its scheduler, and
     // every tile waits for that slowest quarter.  One elected thread per warp; descriptors advance by 32-bit adds.
-    // (Every trip makes its barrier calls whether or not a wait gave up: nobody is left without a partner.)
+    // (Every trip makes its barrier calls, issues and commits whether or not a wait for a load gave up, see mbar_wait_issued.)
     const bool is_dp = warp == WARP_MMA + 1;
     constexpr uint32_t IDESC_S = make_idesc(BKV, BQ, 0, 0, BF);     // S^T = K Q^T, dP^T = V dA^T
     const uint32_t k1_lo = sdesc_lo(smem_u32(smem + OFF_K1)), k2_lo = sdesc_lo(smem_u32(smem + OFF_K2));
@@ -399,7 +399,7 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
         ok = ok && mbar_wait_warp(&misc->full[st], par, abort_flag, 502, i);      // under the warpgroups' pass over the tile before
         if (it > 0 || i > 0) named_bar_sync(NB_SFREE, NB_SFREE_THREADS);          // the scores before these are in registers
         tc_fence_after();
-        if (ok && elect_one()) {
+        if (elect_one()) {
           issue_scores(st_lo0 + st * (STAGE_BYTES >> 4));
           if (i == nq - 1) mma_commit(&misc->kv_empty);
         }
@@ -456,12 +456,6 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
     const float sg = load_lambda(args.lambda_ptr, args.lambda_dtype) < 0.f ? 1.f : -1.f;   // -sign(lambda)
     const f32x2 dscale_2 = pk2(args.drop_scale, args.drop_scale), sgd_2 = pk2(sg * args.drop_scale, sg * args.drop_scale);     // DROP only
     const f32x2 sl2_2 = pk2(sl2, sl2), sg_2 = pk2(sg, sg);
-    bool ok = true;
-    auto hand_over = [&](int id, int threads) {
-      tc_fence_before();
-      if (ok) named_bar_arrive(id, threads);
-      else named_bar_sync(id, threads);
-    };
     uint32_t s_ready = 0;            // answers of the early probes (see mbar_probe)
     int st = 0;
     for (; work.valid(); work.next()) {
@@ -476,10 +470,9 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
           dw1 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(wi.bh), 0u), col2, row & 1, args.drop_thresh);
           dw2 = drop_walk_col(drop_key(args.seed_lo, args.seed_hi, uint32_t(wi.bh), 1u), col2, row & 1, args.drop_thresh);
         }
-        int i = 0;
-        for (; ok && i < nq; ++i) {
+        for (int i = 0; i < nq; ++i) {
           const float4* stats = reinterpret_cast<const float4*>(smem + OFF_STAGE + st * STAGE_BYTES + 2 * Q_BYTES + DA_BYTES) + g * 16;
-          if (!__all_sync(0xffffffffu, s_ready) && !mbar_wait_warp(&misc->s_full, i & 1, abort_flag, 601 + g, i)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, s_ready)) mbar_wait_issued_warp(&misc->s_full, i & 1, abort_flag, 601 + g, i);
           tc_fence_after();
           uint32_t s1[16], s2[16], dp[16];
           tmem_ld16(tb + T_S1 + g * 16, s1);
@@ -550,7 +543,7 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           if (i > 0) {
-            if (!__all_sync(0xffffffffu, md_ready)) ok = mbar_wait_warp(&misc->mma_done, (i - 1) & 1, abort_flag, 605 + g, i);
+            if (!__all_sync(0xffffffffu, md_ready)) mbar_wait_issued_warp(&misc->mma_done, (i - 1) & 1, abort_flag, 605 + g, i);
             tc_fence_after();
           }
           s_ready = i + 1 < nq ? mbar_probe(&misc->s_full, (i + 1) & 1) : 0u;
@@ -564,22 +557,19 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
           named_bar_arrive(NB_E + (i & 1), NB_E_THREADS);
           if (++st == ST) st = 0;
         }
-        // after a wait that gave up: the named barriers of the query tiles left, synced on instead of arrived at, so that nobody is left
-        // waiting and nobody runs ahead
-        for (; i < nq; ++i) {
-          named_bar_sync(NB_SFREE, NB_SFREE_THREADS);
-          named_bar_sync(NB_E + (i & 1), NB_E_THREADS);
-        }
       }
       work.forget();
-      ok = ok && mbar_wait_warp(&misc->acc_full, work.round & 1, abort_flag, 611 + g);
+      mbar_wait_issued_warp(&misc->acc_full, work.round & 1, abort_flag, 611 + g);
       tc_fence_after();
       // warpgroup g reads accumulator columns [64g, 64g+64): g = 0,1 -> the two halves of dV, g = 2 -> dK1, g = 3 -> dK2
       uint32_t acc[64];
       tmem_ld32(tb + g * 64, acc);
       tmem_ld32(tb + g * 64 + 32, acc + 32);
       tc_wait_ld();
-      if (work.has_next()) hand_over(NB_ACC, NB_E_THREADS);
+      if (work.has_next()) {
+        tc_fence_before();
+        named_bar_arrive(NB_ACC, NB_E_THREADS);
+      }
       // The gradients leave through shared memory and the TMA engine (row-per-thread global stores of 16-byte
       // pieces are several times slower): each warpgroup lays its 64 columns into a swizzled [128][64] tile over buffers that
       // no MMA reads any more and the next tile does not fill at once, and the TMA warp stores the tiles.
@@ -597,7 +587,7 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
           st_swizzled_chunk(tile, row, i, v);
         }
         fence_proxy_async_smem();
-        hand_over(NB_STORE, NB_E_THREADS);
+        named_bar_arrive(NB_STORE, NB_E_THREADS);
       }
     }
   }
@@ -725,16 +715,16 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
         const WorkItem wi = work.item();
         const int nkv = key_tiles(args.causal, args.n, wi.tile), b_idx = wi.bh / args.h, h_idx = wi.bh % args.h;
         if (it > 0) {
-          ok = mbar_wait(&misc->q_empty, (it - 1) & 1, abort_flag, 703, it);
+          ok = mbar_wait_free(&misc->q_empty, (it - 1) & 1, abort_flag, 703, it);
           if (!ok) break;
           load_q(wi.tile, wi.bh, h_idx, b_idx);
         }
         for (int j = 0; j < nkv; ++j) {
           if (it > 0 || j >= VS) {
-            ok = mbar_wait(&misc->v_empty[vs], v_par, abort_flag, 701, j);
+            ok = mbar_wait_free(&misc->v_empty[vs], v_par, abort_flag, 701, j);
             if (!ok) break;
             load_v(vs, j, h_idx, b_idx);
-            ok = mbar_wait(&misc->k_empty[ks], k_par, abort_flag, 702, j);
+            ok = mbar_wait_free(&misc->k_empty[ks], k_par, abort_flag, 702, j);
             if (!ok) break;
             load_k(ks, j, h_idx, b_idx);
           }
@@ -744,8 +734,8 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
       }
     }
   } else if (warp == WARP_MMA) {
-    // One warp issues every MMA.  Every trip makes its barrier calls whether or not a wait gave up, so no warpgroup is left
-    // without its partner.
+    // One warp issues every MMA.  Every trip makes its barrier calls, issues and commits whether or not a wait for a load gave up (see
+    // mbar_wait_issued).
     constexpr uint32_t IDESC_S = make_idesc(BM, BN, 0, 0, BF);     // S = Q K^T, dP = dA V^T
     const uint32_t IDESC_DQ = make_idesc(BM, args.d, 0, 1, BF);    // dQ += dS K   (K MN-major); head dim 32: 32 columns
     const int kd = args.d >> 4;       // 16-deep MMA steps over the head dim: head dim 32 skips the zero padding
@@ -784,7 +774,7 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
       ok = ok && mbar_wait_warp(&misc->v_full[vs], v_par, abort_flag, 802, it);
       ok = ok && mbar_wait_warp(&misc->k_full[ks], k_par, abort_flag, 803, it);
       tc_fence_after();
-      if (ok && elect_one()) {
+      if (elect_one()) {
         issue_dp(vs);
         issue_s(0, ks);
         issue_s(1, ks);
@@ -803,18 +793,18 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
         if (j == 0 && it > 0) named_bar_sync(NB_ACC, NB_THREADS);        // the previous tile's accumulators are in registers
         named_bar_sync(NB_DP, NB_THREADS);                               // dP(j) is in registers
         tc_fence_after();
-        if (ok && more && elect_one()) issue_dp(vs_n);
+        if (more && elect_one()) issue_dp(vs_n);
         __syncwarp();
         named_bar_sync(NB_DS1, NB_THREADS);                              // dS1(j) written
         tc_fence_after();
-        if (ok && elect_one()) {
+        if (elect_one()) {
           issue_dq(0, ks, j > 0);
           if (more) issue_s(0, ks_n);
         }
         __syncwarp();
         named_bar_sync(NB_DS2, NB_THREADS);                              // dS2(j) written
         tc_fence_after();
-        if (ok && elect_one()) {
+        if (elect_one()) {
           issue_dq(1, ks, j > 0);
           mma_commit(&misc->k_empty[ks]);
           if (more) issue_s(1, ks_n);
@@ -836,12 +826,6 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
     const float sg = lam < 0.f ? 1.f : -1.f;       // branch 2: -sign(lambda) (|lambda| sits in its statistics, the sign in e)
     const float dscale = DROP ? args.drop_scale : 1.f;
     const f32x2 sl2_2 = pk2(sl2, sl2);
-    bool ok = true;
-    auto hand_over = [&](int id) {
-      tc_fence_before();
-      if (ok) named_bar_arrive(id, NB_THREADS);
-      else named_bar_sync(id, NB_THREADS);
-    };
     const uint32_t t_s1 = tb + T_S1 + g * 32, t_s2 = tb + T_S2 + g * 32, t_dp = tb + T_DP + g * 32;
     // own 32 columns of one branch: dS over the first 16 of them
     auto branch = [&](uint32_t* s, const uint32_t* dp, int nv, int j, float neg_l, float neg_e, float sgn, const DropWalk& dw, auto mid) {
@@ -882,14 +866,13 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
           dw1 = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 0u), row2, row & 1, args.drop_thresh);
           dw2 = drop_walk_row(drop_key(args.seed_lo, args.seed_hi, uint32_t(bh), 1u), row2, row & 1, args.drop_thresh);
         }
-        int j = 0;
-        for (; ok && j < nkv; ++j, ++done) {
+        for (int j = 0; j < nkv; ++j, ++done) {
           // key columns past the sequence end or (causal) right of the diagonal: score -inf, probability 0
           const int c_first = j * BN + g * 32;
           int nv = args.n - c_first;
           if (args.causal) nv = min(nv, q_tile * BM + row - c_first + 1);
           uint32_t s[32], dp[32];
-          if (!mbar_wait_warp(&misc->s_full[0], done & 1, abort_flag, 901, j)) { ok = false; break; }
+          mbar_wait_issued_warp(&misc->s_full[0], done & 1, abort_flag, 901, j);
           tc_fence_after();
           tmem_ld32(t_dp, dp);
           tmem_ld32(t_s1, s);
@@ -901,7 +884,7 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
           tc_wait_st();
           tc_fence_before();
           named_bar_arrive(NB_DS1, NB_THREADS);
-          ok = mbar_wait_warp(&misc->s_full[1], done & 1, abort_flag, 902, j);
+          mbar_wait_issued_warp(&misc->s_full[1], done & 1, abort_flag, 902, j);
           tc_fence_after();
           tmem_ld32(t_s2, s);
           tc_wait_ld();
@@ -911,31 +894,23 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
           tc_fence_before();
           named_bar_arrive(NB_DS2, NB_THREADS);
         }
-        // after a wait that gave up: the named barriers of the tiles left, synced on instead of arrived at, so that nobody is left
-        // waiting and nobody runs ahead
-        if (!ok && done == 0) {          // given up before the first half branch: team 1 must not wait for it
-          if (g < 2) named_bar_arrive(NB_START, NWG * 128);
-          done = 1;
-        }
-        for (; j < nkv; ++j) {
-          named_bar_sync(NB_DP, NB_THREADS);
-          named_bar_sync(NB_DS1, NB_THREADS);
-          named_bar_sync(NB_DS2, NB_THREADS);
-        }
       }
       work.forget();
-      ok = ok && mbar_wait_warp(&misc->acc_full, work.round & 1, abort_flag, 911);
+      mbar_wait_issued_warp(&misc->acc_full, work.round & 1, abort_flag, 911);
       tc_fence_after();
       const int u = g >> 1, half = g & 1;            // this warpgroup stores columns [32 half, 32 half + 32) of dQ of branch u
       uint32_t acc[32];
       tmem_ld32(tb + (u ? T_DQ2 : T_DQ1) + half * 32, acc);
       tc_wait_ld();
-      if (work.has_next()) hand_over(NB_ACC);
+      if (work.has_next()) {
+        tc_fence_before();
+        named_bar_arrive(NB_ACC, NB_THREADS);
+      }
       const WorkItem wi = work.item();
       const int q_tile = wi.tile;
       // (32 columns per thread: direct 16-byte stores; a shared-memory tile and a TMA store, as the other two
       // kernels use for their wider rows, measured 4 % slower here)
-      if (ok && !*abort_flag && half * 32 < args.d && q_tile * BM + row < args.n) {
+      if (!*abort_flag && half * 32 < args.d && q_tile * BM + row < args.n) {
         const float sc = args.sm_scale;
         const size_t grow = size_t(wi.bh) * args.n + size_t(q_tile) * BM + row;
         uint4* p = reinterpret_cast<uint4*>((u ? args.dq2 : args.dq1) + grow * args.d + half * 32);

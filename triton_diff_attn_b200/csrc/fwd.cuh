@@ -99,9 +99,9 @@ struct SoftmaxState {
 // t_s); t_o, O_COLS: the branch's accumulator; first: sub-tile 0; t: its index, only read with dropout; nv: visible columns of this row (the rest get -inf, probability 0); loaded:
 // the scores are in registers; wait_m / publish_m: hand-over of the running maximum; wait_pv: P_b V of
 // sub-tile t-1 has completed; mid: runs half way through the exponentials; p_free: the
-// columns behind t_p may be overwritten (both false: a bounded wait gave up).
+// columns behind t_p may be overwritten.
 template <bool BF, bool DROP, int O_COLS, class Loaded, class WaitM, class PublishM, class WaitPv, class Mid, class PFree>
-__device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, uint32_t t_p, uint32_t t_o, bool first, int t, int nv, float sl2,
+__device__ __forceinline__ void softmax_subtile(SoftmaxState& st, uint32_t t_s, uint32_t t_p, uint32_t t_o, bool first, int t, int nv, float sl2,
                                                 volatile float* m_row, const DropWalk& dr, Loaded loaded, WaitM wait_m, PublishM publish_m,
                                                 WaitPv wait_pv, Mid mid, PFree p_free) {
   uint32_t sr[64];
@@ -130,7 +130,7 @@ __device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, 
   if (need) *m_row = m;
   publish_m();
   if (__any_sync(0xffffffffu, need) && !first) {
-    if (!wait_pv()) return false;
+    wait_pv();
     tc_fence_after();
     const float scale = need ? ex2((m_prev - m) * sl2) : 1.f;
 #pragma unroll 1
@@ -167,11 +167,10 @@ __device__ __forceinline__ bool softmax_subtile(SoftmaxState& st, uint32_t t_s, 
     for (int i = 0; i < 32; ++i)
       sr[i] &= drop_mask_pair(drop_at_col(dr, uint32_t(t * 32), i));
   }
-  const bool ok = p_free();
+  p_free();
   tmem_st32(t_p, sr);
   tc_wait_st();
   tc_fence_before();
-  return ok;
 }
 
 }  // namespace da

@@ -112,7 +112,7 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
   if (warp == WARP_TMA) {
     if (elect_one()) {
       for (int t = 2; t < nsub; ++t) {
-        if (!mbar_wait(&misc->k_empty[t % KS], ((t / KS) & 1) ^ 1, abort_flag, 2101, t)) break;
+        if (!mbar_wait_free(&misc->k_empty[t % KS], ((t / KS) & 1) ^ 1, abort_flag, 2101, t)) break;
         load_k(t);
       }
     }
@@ -121,7 +121,7 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
     // K waits behind a V whose stage is not free yet: 2.3 ms against 1.4 ms at B2 H8 N8192 D128)
     if (elect_one()) {
       for (int t = 2; t < nsub; ++t) {
-        if (!mbar_wait(&misc->v_empty[t % VS], ((t / VS) & 1) ^ 1, abort_flag, 2102, t)) break;
+        if (!mbar_wait_free(&misc->v_empty[t % VS], ((t / VS) & 1) ^ 1, abort_flag, 2102, t)) break;
         load_v(t);
       }
     }
@@ -129,14 +129,13 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
     // S(t+2) = Q K^T once the scores of sub-tile t are in registers.  Scores and probabilities have TMEM columns of their
     // own, so a warpgroup finds its next scores ready when it has stored its probabilities, and the two kinds of MMAs need no
     // order between them: two issuing warps, so that one's waits run under the other's MMAs (1.198 ms against 1.207 ms
-    // with one warp for both at B2 H8 N8192 D128).
+    // with one warp for both at B2 H8 N8192 D128).  Both run every trip, whether or not a wait for a load gave up (see mbar_wait_issued).
     constexpr uint32_t IDESC_S = make_idesc(BM, SUB, 0, 0, BF);
     const uint32_t k_lo0 = sdesc_lo(smem_u32(smem + OFF_K));
     bool ok = mbar_wait_warp(&misc->q_ready, 0, abort_flag, 2201);
-    for (int t = 0; ok && t < nsub; ++t) {
+    for (int t = 0; t < nsub; ++t) {
       const int ks = t % KS, u = t & 1;
-      ok = mbar_wait_warp(&misc->k_full[ks], (t / KS) & 1, abort_flag, 2202, t);
-      if (!ok) break;
+      ok = ok && mbar_wait_warp(&misc->k_full[ks], (t / KS) & 1, abort_flag, 2202, t);
       if (t >= 2) named_bar_sync(NB_SF + u, 160);
       tc_fence_after();
       if (elect_one()) {
@@ -152,9 +151,10 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
     // O += P(t) V(t)
     constexpr uint32_t IDESC_O = make_idesc(BM, DV, 0, 1, BF);      // V as MN-major B: four 64-column atoms 8 KB apart
     const uint32_t v_lo0 = sdesc_lo(smem_u32(smem + OFF_V), 8192);
+    bool ok = true;
     for (int t = 0; t < nsub; ++t) {
       const int vs = t % VS, u = t & 1;
-      if (!mbar_wait_warp(&misc->v_full[vs], (t / VS) & 1, abort_flag, 2203, t)) break;
+      ok = ok && mbar_wait_warp(&misc->v_full[vs], (t / VS) & 1, abort_flag, 2203, t);
       named_bar_sync(NB_P + u, 160);
       tc_fence_after();
       if (elect_one()) {
@@ -177,7 +177,7 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
     // Q into TMEM, the A operand of S = Q K^T: this thread's row, the 64 columns of box u (128 bytes, swizzled in 16-byte
     // chunks) -> 32 columns.  The score MMAs then read only K from shared memory (with both operands there an N = 64 step
     // takes 48 clocks of shared-memory bandwidth for 32 of tensor time).
-    bool ok = mbar_wait_warp(&misc->bar_q, 0, abort_flag, 2300);
+    mbar_wait_warp(&misc->bar_q, 0, abort_flag, 2300);
     {
       uint32_t qv[32];
       const uint8_t* qrow = smem + OFF_Q + u * 16384 + row * 128;
@@ -202,32 +202,22 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
       // leave the exp unit idle together.
       if (u == 1) named_bar_sync(NB_START, 256);
       uint32_t s_ready = 0;             // answer of the early probe (see mbar_probe)
-      for (; ok && t < nsub; t += 2) {
-        ok = s_ready || mbar_wait(&misc->s_full[u], (t >> 1) & 1, abort_flag, 2301 + br, t);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+      for (; t < nsub; t += 2) {
+        if (!s_ready) mbar_wait_issued(&misc->s_full[u], (t >> 1) & 1, abort_flag, 2301 + br, t);
+        __syncwarp();
         tc_fence_after();
         int nv = args.n - t * SUB;             // visible key columns of this row in this sub-tile
         if (args.causal) nv = min(nv, q_tile * BM + row - t * SUB + 1);
-        ok = softmax_subtile<BF, DROP, DV>(
+        softmax_subtile<BF, DROP, DV>(
                  st, t_s, t_p, t_o, t == 0, t, nv, sl2, &misc->m_run[row], dr,
                  [&] { if (t + 2 < nsub) { tc_fence_before(); named_bar_arrive(NB_SF + u, 160); } },
                  [&] { named_bar_sync(NB_M + (u ^ 1), 256); }, [&] { if (t + 1 < nsub) named_bar_arrive(NB_M + u, 256); },
-                 [&] { return mbar_wait_warp(&misc->pv_done[u ^ 1], ((t - 1) >> 1) & 1, abort_flag, 2305 + br, t); },
+                 [&] { mbar_wait_issued_warp(&misc->pv_done[u ^ 1], ((t - 1) >> 1) & 1, abort_flag, 2305 + br, t); },
                  [&] {
                    if (t == 0) named_bar_arrive(NB_START, 256);
                    if (t + 2 < nsub) s_ready = mbar_probe(&misc->s_full[u], ((t + 2) >> 1) & 1);
                  },
-                 [&] { return t < 2 || mbar_wait_warp(&misc->pv_done[u], ((t - 2) >> 1) & 1, abort_flag, 2303 + br, t); });
-        named_bar_arrive(NB_P + u, 160);
-        if (!ok) { t += 2; break; }
-      }
-      // a warp whose wait gave up stands in for the named-barrier arrivals it will no longer make
-      if (!ok && t == 0) named_bar_arrive(NB_START, 256);
-      for (; t < nsub; t += 2) {
-        if (t + 2 < nsub) named_bar_arrive(NB_SF + u, 160);
-        if (t > 0) named_bar_arrive(NB_M + (u ^ 1), 256);
-        if (t + 1 < nsub) named_bar_arrive(NB_M + u, 256);
+                 [&] { if (t >= 2) mbar_wait_issued_warp(&misc->pv_done[u], ((t - 2) >> 1) & 1, abort_flag, 2303 + br, t); });
         named_bar_arrive(NB_P + u, 160);
       }
     }
@@ -235,8 +225,8 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
     // ---- epilogue.  The two CTAs of a cluster hold A1 = O_1 / l_1 (branch 1) and A2 = O_2 / l_2 (branch 2) of the same 128
     // query rows.  Branch 2 writes a2 and hands its A2 in fp32 to branch 1 through distributed shared memory (into branch
     // 1's rings, idle by then); branch 1 forms y = RMSNorm(A1 - lambda A2) (1 - lambda_init) and rstd.  Warpgroup u has
-    // value columns [128 u, 128 u + 128).  Every thread runs every barrier; only the global writes depend on `ok`.
-    ok = mbar_wait_warp(&misc->o_full, 0, abort_flag, 2311 + br) && ok;
+    // value columns [128 u, 128 u + 128).  Every thread runs every barrier; only the global writes depend on the waits.
+    mbar_wait_issued_warp(&misc->o_full, 0, abort_flag, 2311 + br);
     tc_fence_after();
     misc->m_end[u][row] = st.m;
     misc->l_end[u][row] = st.l;
@@ -244,7 +234,7 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
     const float ma = misc->m_end[0][row], mb = misc->m_end[1][row], m_fin = fmaxf(ma, mb);
     const float l_fin = misc->l_end[0][row] * ex2((ma - m_fin) * sl2) + misc->l_end[1][row] * ex2((mb - m_fin) * sl2);
     const float inv_l = (DROP ? args.drop_scale : 1.f) / l_fin;
-    const bool live = ok && !*abort_flag && (q_tile * BM + row < args.n);
+    const bool live = !*abort_flag && (q_tile * BM + row < args.n);
     uint8_t* out = smem + OFF_OUT + 2 * u * OUT_TILE_BYTES;      // this warpgroup's two 64-column tiles
     // stores the warpgroup's two tiles once all its threads have written them
     auto store_tiles = [&](const CUtensorMap* map, uint8_t* tiles) {
@@ -262,7 +252,7 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
     uint8_t* xtile = smem + OFF_X;
     if (br == 1) {
       const uint32_t x_remote = cluster_map(smem_u32(xtile), 0);
-      ok = mbar_wait_cluster(&misc->peer_ready, 0, abort_flag, 2313) && ok;       // branch 1's rings are idle
+      mbar_wait_cluster(&misc->peer_ready, 0, abort_flag, 2313);       // branch 1's rings are idle
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint32_t o[32];
@@ -286,7 +276,7 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
     } else {
       if (threadIdx.x == 0) cluster_mbar_arrive(cluster_map(smem_u32(&misc->peer_ready), 1));
       const float lam = load_lambda(args.lambda_ptr, args.lambda_dtype);
-      ok = mbar_wait_cluster(&misc->peer_data, 0, abort_flag, 2314) && ok;
+      const bool ok = mbar_wait_cluster(&misc->peer_data, 0, abort_flag, 2314);
       const float4* xrow = reinterpret_cast<const float4*>(xtile) + u * 32 * BM + row;
       // A = A1 - lambda A2 of one 32-column chunk (the accumulator and the exchange tile are read twice with rms_norm)
       auto load_a = [&](int c, float (&a)[32]) {

@@ -116,7 +116,7 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
         const int nkv = key_tiles(args.causal, args.n, wi.tile);
         const int b_idx = wi.bh / args.h, h_idx = wi.bh % args.h;
         if (it > 0) {
-          ok = mbar_wait(&misc->q_empty, (it - 1) & 1, abort_flag, 103, it);
+          ok = mbar_wait_free(&misc->q_empty, (it - 1) & 1, abort_flag, 103, it);
           if (!ok) break;
           mbar_expect_tx(&misc->bar_q, 2 * Q_BYTES);
           tma_load_4d(smem + OFF_Q1, &tm_q1, &misc->bar_q, 0, wi.tile * BM, h_idx, b_idx);
@@ -125,14 +125,14 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
         for (int j = 0; j < nkv; ++j) {
           const bool requested = it == 0 && j < PRELOAD;
           if (!requested) {
-            ok = mbar_wait(&misc->k_empty[ks], k_par, abort_flag, 101, j);
+            ok = mbar_wait_free(&misc->k_empty[ks], k_par, abort_flag, 101, j);
             if (!ok) break;
             mbar_expect_tx(&misc->k_full[ks], 2 * K_BYTES);
             tma_load_4d(smem + OFF_K + ks * 2 * K_BYTES, &tm_k1, &misc->k_full[ks], 0, j * BN, h_idx, b_idx);
             tma_load_4d(smem + OFF_K + ks * 2 * K_BYTES + K_BYTES, &tm_k2, &misc->k_full[ks], 0, j * BN, h_idx, b_idx);
             // the previous tile's y and a2 (and its gained y, in the K slot after the one just requested) have to leave first
-            if (it > 0 && j == 0) ok = mbar_wait(&misc->stored, (it - 1) & 1, abort_flag, 104, it);
-            ok = ok && mbar_wait(&misc->v_empty[vs], v_par, abort_flag, 102, j);
+            if (it > 0 && j == 0) ok = mbar_wait_free(&misc->stored, (it - 1) & 1, abort_flag, 104, it);
+            ok = ok && mbar_wait_free(&misc->v_empty[vs], v_par, abort_flag, 102, j);
             if (!ok) break;
             mbar_expect_tx(&misc->v_full[vs], V_BYTES);
             tma_load_4d(smem + OFF_V + vs * V_BYTES, &tm_v, &misc->v_full[vs], 0, j * BN, h_idx, b_idx);
@@ -147,7 +147,7 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
     // ------------- MMA issuer: O_b += P_b(t) V(sub-tile t), S_b(t+2) = Q_b K_b(sub-tile t+2)^T, branch 1 then branch 2 -------------
     // The thread that issues is chosen by elect.sync.  (A thread picked by comparing the lane id issues
     // tcgen05.mma about three times slower: 152 against 48 clocks per instruction, measured.)
-    // Every trip makes its barrier calls whether or not a wait gave up, so nobody is left without a partner.
+    // Every trip makes its barrier calls, issues and commits whether or not a wait for a load gave up (see mbar_wait_issued).
     reg_dec<REGS_ROLE>();
     const uint32_t IDESC_O = make_idesc(BM, 2 * args.d, 0, 1, BF);    // V is MN-major; head dim 32: the 64 real value columns only
     constexpr uint32_t IDESC_S = make_idesc(BM, SUB, 0, 0, BF);
@@ -171,7 +171,7 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
       ok = ok && mbar_wait_warp(&misc->bar_q, it & 1, abort_flag, 201, it);
       ok = ok && mbar_wait_warp(&misc->k_full[ks], k_par, abort_flag, 202, it);
       tc_fence_after();
-      if (ok && elect_one()) {
+      if (elect_one()) {
         const uint32_t k_lo = k_lo0 + ks * ((2 * K_BYTES) >> 4);
         for (int u = 0; u < 2; ++u)
           for (int br = 0; br < 2; ++br) issue_s(k_lo, br, u);
@@ -191,7 +191,7 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
           const int u = i >> 1, br = i & 1;
           named_bar_sync(NB_P + br * 2 + u, 160);
           tc_fence_after();
-          if (ok && elect_one()) {
+          if (elect_one()) {
 #pragma unroll
             for (int k = 0; k < SUB / 16; ++k)
               mma_ts_lo(tmem_base + T_O + br * 128, tmem_base + br * 128 + u * SUB + k * 8, v_lo + u * HALF + k * (2048 >> 4), IDESC_O,
@@ -209,7 +209,7 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
         if (more && ++ks == KS) { ks = 0; k_par ^= 1; }
         if (++vs == VS) vs = 0;
       }
-      if (ok && elect_one()) mma_commit(&misc->o_full);
+      if (elect_one()) mma_commit(&misc->o_full);
       __syncwarp();
     }
   } else if (warp == WARP_ALLOC) {
@@ -267,12 +267,7 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
       return int(t & 127u);
     };
     const float sl2 = args.sm_scale * 1.4426950408889634f;
-    bool ok = true;
     int tc = u;                                     // sub-tiles, counted on from tile to tile: tc >> 1 is the phase of the buffers' barriers
-    auto hand_over = [&](int id, int threads) {
-      if (ok) named_bar_arrive(id, threads);
-      else named_bar_sync(id, threads);
-    };
     for (; work.valid(); work.next()) {
       SoftmaxState st;
       {
@@ -289,28 +284,21 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
         int seen = args.n;                            // visible key columns: up to the sequence end, up to the diagonal
         if (args.causal) seen = min(seen, wi.tile * BM + row + 1);
         seen += t0 * SUB;
-        for (; ok && tc < t_end; tc += 2) {
-          if (!mbar_wait_warp(&misc->s_full[br][u], (tc >> 1) & 1, abort_flag, 301 + br, tc)) { ok = false; break; }
+        for (; tc < t_end; tc += 2) {
+          mbar_wait_issued_warp(&misc->s_full[br][u], (tc >> 1) & 1, abort_flag, 301 + br, tc);
           tc_fence_after();
           // P_b V of sub-tile tc - 1 used the other buffer
-          ok = softmax_subtile<BF, DROP, DV>(
+          softmax_subtile<BF, DROP, DV>(
               st, t_s, t_s, t_o, tc == t_first, tc - t0, seen - tc * SUB, sl2, &misc->m_run[br][row], dr, [] {},
               [&] { named_bar_sync(NB_M + br * 2 + (u ^ 1), 256); }, [&] { if (tc + 1 < t_end) named_bar_arrive(NB_M + br * 2 + u, 256); },
-              [&] { return mbar_wait_warp(&misc->pv_done[br][u ^ 1], ((tc - 1) >> 1) & 1, abort_flag, 305 + br, tc); }, [] {}, [] { return true; });
+              [&] { mbar_wait_issued_warp(&misc->pv_done[br][u ^ 1], ((tc - 1) >> 1) & 1, abort_flag, 305 + br, tc); }, [] {}, [] {});
           named_bar_arrive(NB_P + br * 2 + u, 160);
-        }
-        // after a wait that gave up: the named barriers of the sub-tiles left, synced on instead of arrived at, so that nobody is left
-        // waiting and nobody runs ahead
-        for (; tc < t_end; tc += 2) {
-          if (tc != t_first) named_bar_sync(NB_M + br * 2 + (u ^ 1), 256);
-          if (tc + 1 < t_end) named_bar_sync(NB_M + br * 2 + u, 256);
-          named_bar_sync(NB_P + br * 2 + u, 160);
         }
       }
       work.forget();
       const int row = softmax_row();
-      // ---- epilogue: every thread runs every barrier; only the global writes depend on `ok`
-      ok = ok && mbar_wait_warp(&misc->o_full, work.round & 1, abort_flag, 311 + br);
+      // ---- epilogue: every thread runs every barrier; only the global writes depend on abort_flag
+      mbar_wait_issued_warp(&misc->o_full, work.round & 1, abort_flag, 311 + br);
       tc_fence_after();
       misc->m_end[br][u][row] = st.m;
       misc->l_end[br][u][row] = st.l;
@@ -332,7 +320,7 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
       tmem_ld32(tmem_base + lane_base + T_O + 128 + q * 32, o2);
       tc_wait_ld();
       tc_fence_before();
-      if (work.has_next()) hand_over(NB_O, NUM_SOFTMAX + 32);
+      if (work.has_next()) named_bar_arrive(NB_O, NUM_SOFTMAX + 32);
       float ssq = 0.f;
       const int dv_real = 2 * args.d;                      // 128, or 64 when the head dim is 32 (upper columns are padding)
       const bool pad = q * 32 >= dv_real;                  // head dim 32: columns 64..127 of the accumulators were never written
@@ -351,7 +339,7 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
       const WorkItem wi = work.item();
       const int q_tile = wi.tile;
       const size_t grow = size_t(wi.bh) * args.n + size_t(q_tile) * BM + row;
-      const bool write = ok && q_tile * BM + row < args.n;     // rows past the sequence end are computed on zero padding and dropped
+      const bool write = q_tile * BM + row < args.n;     // rows past the sequence end are computed on zero padding and dropped
       // y and a2 leave through shared memory and the TMA engine: each thread lays its 32 columns into a swizzled
       // [128 rows][64 columns] tile in the (now idle) V ring, and the store warp stores the tiles.
       // (Row-per-thread global stores of 16-byte pieces cost 3.6 us per CTA, 8 % of the kernel at N = 4096.)
@@ -379,7 +367,7 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
           }
         }
         fence_proxy_async_smem();
-        hand_over(NB_STORE + br, NUM_SOFTMAX / 2 + 32);
+        named_bar_arrive(NB_STORE + br, NUM_SOFTMAX / 2 + 32);
       }
       if (write && !*abort_flag && u == 0) {
         if (br == 0) {

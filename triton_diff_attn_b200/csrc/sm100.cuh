@@ -176,6 +176,44 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, site, iter));
 }
 
+// Named barriers have no time limit, and an arrival on one that its partner has not yet reached the call before of completes the
+// wrong phase: where a barrier call relies on an MMA completion in between, the wait for that completion must not end early.  In kernels
+// whose roles meet in named barriers, a role whose wait for a load gave up therefore goes on as if the load had landed: issuers issue and
+// commit in every trip, everybody makes every barrier call, the results are dropped.  Only producers stop (mbar_wait_free).
+//
+// Wait for a completion that this CTA's own issuers commit.  It does not look at abort_flag; the commit comes, at the latest once
+// the issuer's own wait has given up.  The longer limit is for a tensor core that never completes (abort_flag 2: no further wait).
+__device__ __forceinline__ void mbar_wait_issued(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int site, int iter = 0) {
+  if (mbar_try_wait(bar, parity)) return;
+  unsigned long long t0 = 0;
+  uint32_t spins = 0;
+  while (!mbar_try_wait(bar, parity)) {
+    if ((++spins & 0xff) == 0) {
+      if (*abort_flag == 2) return;
+      unsigned long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > 4 * kWaitLimitNs) {
+        *abort_flag = 2;
+        if (atomicCAS(&g_status[0], 0, site) == 0) {
+          g_status[1] = blockIdx.x;
+          g_status[2] = blockIdx.y;
+          g_status[3] = iter;
+        }
+        return;
+      }
+    }
+  }
+}
+__device__ __forceinline__ void mbar_wait_issued_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int site, int iter = 0) {
+  mbar_wait_issued(bar, parity, abort_flag, site, iter);
+  __syncwarp();
+}
+// A producer's wait for a free ring slot: false also when another role has given up, since the load it missed may still hold the
+// slot's barrier in its phase, and nothing more may be requested onto that.
+__device__ __forceinline__ bool mbar_wait_free(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int site, int iter = 0) {
+  return mbar_wait(bar, parity, abort_flag, site, iter) && !*abort_flag;
+}
+
 // ---------------------------------- thread-block clusters ----------------------------------
 // The partner CTA's shared memory (distributed shared memory): a local shared-memory address mapped into CTA `rank`.
 __device__ __forceinline__ uint32_t cluster_map(uint32_t local_smem_addr, uint32_t rank) {
@@ -231,8 +269,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
-// non-blocking arrival on a named barrier: lets a warp that has given up (a bounded wait expired) stand in for the
-// bar.sync calls it will no longer make, so that a partner still running its loop is never left waiting on it
+// non-blocking arrival on a named barrier
 __device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
