@@ -105,6 +105,7 @@ int diffattn_fwd(const DiffAttnParams* p);
 
 /* Backward.  Reads the forward's inputs and outputs plus dy; writes dq1,dq2,dk1,dk2,dv and adds the
  * lambda gradient into *dlambda (zero it first; partials of several shards add up on the host).
+ * No output may overlap an input or another output, except that dq1, dq2 may be dense q1, q2 themselves (default form, head dim 128).
  * Replaces _diff_attention.backward + diff_attn_bwd (reference src/kernel.py:516-575, :221-458). */
 int diffattn_bwd(const DiffAttnParams* p);
 

@@ -32,8 +32,9 @@ def test_gradients_at_tile_edges(d, n, causal, p):
         assert m["rel_l2"] <= 1e-3, (name, m)
 
 
+@pytest.mark.parametrize("options", [{}, {"causal": True, "bf16": True}, {"p": 0.25}, {"causal": True, "bf16": True, "p": 0.25}])
 @pytest.mark.parametrize("b,h,n,d", [(1, 1, 64, 64), (2, 5, 200, 32), (3, 7, 640, 64), (1, 3, 300, 128), (2, 20, 512, 128)])
-def test_overlapping_kernels_equal_separate_ones(b, h, n, d):
+def test_overlapping_kernels_equal_separate_ones(b, h, n, d, options):
     """In one call the backward's kernels start before the one ahead of them has ended; issued one stage at a time they do not.
     Several calls follow each other on the stream with fresh inputs in the same buffers, smaller and larger than the chip."""
     if not torch.cuda.is_available():
@@ -41,14 +42,16 @@ def test_overlapping_kernels_equal_separate_ones(b, h, n, d):
     import triton_diff_attn_b200 as pkg
     from triton_diff_attn_b200 import _lib
     dev = torch.device("cuda", 0)
-    ins = [t.to(dev) for t in oracle.make_inputs(b, h, n, d, 77)]
+    dt = torch.bfloat16 if options.get("bf16") else torch.float16
+    ins = [t.to(dev, dt) for t in oracle.make_inputs(b, h, n, d, 77)]
     q1, q2, k1, k2, v, dy = ins
     lam = torch.tensor([0.5], device=dev)
     saved = [torch.empty_like(v), torch.empty_like(v)] + [torch.empty((b, h, n), device=dev) for _ in range(3)]
     grads = [torch.empty_like(t) for t in (q1, q2, k1, k2, v)]
     dlam = torch.zeros(1, device=dev)
     p = _lib.new_params()
-    pkg.layers._fill_common(p, q1, q2, k1, k2, v, lam, 0.2, True, saved)
+    pkg.layers._fill_common(p, q1, q2, k1, k2, v, lam, 0.2, True, saved, options.get("causal", False),
+                            pkg.layers.dropout_threshold(options.get("p", 0.0)), 4321)
     ws = torch.empty(_lib.lib.diffattn_workspace_bytes(p), dtype=torch.uint8, device=dev)
     p.dy, p.dlambda, p.workspace, p.workspace_bytes = dy.data_ptr(), dlam.data_ptr(), ws.data_ptr(), ws.numel()
     p.dq1, p.dq2, p.dk1, p.dk2, p.dv = (t.data_ptr() for t in grads)
@@ -70,8 +73,12 @@ def test_overlapping_kernels_equal_separate_ones(b, h, n, d):
 
     want = rounds(separate)
     got = rounds(lambda: _lib.check(_lib.lib.diffattn_bwd(p), "bwd"))
+    # dQ waits for dK/dV before it stores, and a CTA of it reads no query rows but its own: dq1, dq2 may lie over q1, q2
+    p.dq1, p.dq2 = q1.data_ptr(), q2.data_ptr()
+    grads[:2] = [q1, q2]
+    got += rounds(lambda: _lib.check(_lib.lib.diffattn_bwd(p), "bwd"))
     pkg.device_status(0)
-    assert all(torch.equal(a, w) for a, w in zip(got, want))
+    assert all(torch.equal(a, w) for a, w in zip(got, want + want))
 
 
 @pytest.mark.parametrize("b,h,n,d,causal,p,gain", [

@@ -337,7 +337,7 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
         if (it == 0) {
           tma_prefetch_desc(&tm_dv); tma_prefetch_desc(&tm_dk1); tma_prefetch_desc(&tm_dk2);
           griddep_wait();        // dA and the statistics come from the preprocess kernel
-          griddep_launch();      // the dQ kernel depends on nothing else: it may fill the SMs that this grid's last wave leaves idle
+          griddep_launch();      // dQ CTAs may set themselves up on the SMs that this grid's last wave leaves idle
         }
       }
       __syncwarp();
@@ -675,10 +675,12 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
     tma_load_4d(sp, &tm_v, &misc->v_full[st], 0, j * BN, h_idx, b_idx);
     tma_load_4d(sp + V_BYTES / 2, &tm_v, &misc->v_full[st], 64, j * BN, h_idx, b_idx);
   };
-  auto load_q = [&](int q_tile, int bh, int h_idx, int b_idx) {
-    mbar_expect_tx(&misc->bar_q, 2 * Q_BYTES + DA_BYTES);
+  auto load_da = [&](int q_tile, int bh) {
     tma_load_4d(smem + OFF_DA, &tm_da, &misc->bar_q, 0, q_tile * BM, bh, 0);
     tma_load_4d(smem + OFF_DA + DA_BYTES / 2, &tm_da, &misc->bar_q, 64, q_tile * BM, bh, 0);
+  };
+  auto load_q = [&](int q_tile, int h_idx, int b_idx) {
+    mbar_expect_tx(&misc->bar_q, 2 * Q_BYTES + DA_BYTES);       // Q1, Q2 here, dA by load_da
     tma_load_4d(smem + OFF_Q1, &tm_q1, &misc->bar_q, 0, q_tile * BM, h_idx, b_idx);
     tma_load_4d(smem + OFF_Q2, &tm_q2, &misc->bar_q, 0, q_tile * BM, h_idx, b_idx);
   };
@@ -691,10 +693,10 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
     mbar_init(&misc->acc_full, 1);
     misc->abort_flag = 0;
     mbar_init_fence();
-    // the resident tiles and the first pass over the rings are requested before the CTA-wide setup barrier
+    // what the caller gave (Q and the first pass over the rings) is requested before the CTA-wide setup barrier
     const WorkItem wi = work.item();
     const int nkv = key_tiles(args.causal, args.n, wi.tile), b_idx = wi.bh / args.h, h_idx = wi.bh % args.h;
-    load_q(wi.tile, wi.bh, h_idx, b_idx);
+    load_q(wi.tile, h_idx, b_idx);
     for (int j = 0; j < VS && j < nkv; ++j) {
       load_v(j, j, h_idx, b_idx);
       load_k(j, j, h_idx, b_idx);
@@ -717,8 +719,11 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
         if (it > 0) {
           ok = mbar_wait_free(&misc->q_empty, (it - 1) & 1, abort_flag, 703, it);
           if (!ok) break;
-          load_q(wi.tile, wi.bh, h_idx, b_idx);
+          load_q(wi.tile, h_idx, b_idx);
+        } else {
+          griddep_wait();        // dA comes from the preprocess kernel, for which the grid before this one has waited
         }
+        load_da(wi.tile, wi.bh);
         for (int j = 0; j < nkv; ++j) {
           if (it > 0 || j >= VS) {
             ok = mbar_wait_free(&misc->v_empty[vs], v_par, abort_flag, 701, j);
@@ -853,6 +858,7 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
         s[i] = pack2<BF>(r0, r1);
       }
     };
+    griddep_wait();                                // the statistics come from the preprocess kernel
     if (g >= 2) named_bar_sync(NB_START, NWG * 128);
     uint32_t done = 0;                             // key tiles done: the phase of the score barriers
     for (; work.valid(); work.next()) {
@@ -932,8 +938,6 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
-  // whoever waits for this grid waits for the one before it too
-  if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) griddep_wait();
 }
 
 }  // namespace da

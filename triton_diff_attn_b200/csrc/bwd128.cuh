@@ -98,13 +98,15 @@ diffattn_bwd_side128_kernel(const __grid_constant__ CUtensorMap tm_x0, const __g
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&misc->tmem_slot);
 
-  // (launched after the dV kernel's every CTA has seen the preprocess kernel complete: nothing to wait for here)
-  if (!QSIDE && threadIdx.x == 0) griddep_launch();
+  if (!QSIDE && threadIdx.x == 0) griddep_launch();      // the query side may set itself up
   if (warp == WARP_TMA) {
     if (elect_one()) {
       mbar_expect_tx(&misc->bar_xy, X_BYTES + Y_BYTES);
       for (int c = 0; c < 2; ++c) tma_load_4d(smem + OFF_X + c * 16384, tm_x, &misc->bar_xy, c * 64, tile * BM, h_idx, b_idx);
+      // dA (Y or W) and the statistics come from the preprocess kernel, for which the grid before this one has waited
+      if (QSIDE) griddep_wait();
       for (int c = 0; c < 4; ++c) tma_load_4d(smem + OFF_Y + c * 16384, &tm_y, &misc->bar_xy, c * 64, tile * BM, y_c2, y_c3);
+      if (!QSIDE) griddep_wait();
       int zs = 0, ws = 0;
       uint32_t zpar = 1, wpar = 1;
       for (int t = 0; t < nsub; ++t) {
@@ -189,6 +191,7 @@ diffattn_bwd_side128_kernel(const __grid_constant__ CUtensorMap tm_x0, const __g
     const size_t grow = size_t(bh) * args.n + size_t(tile) * BM + row;
     float neg_l = 0.f, neg_e = 0.f;        // the statistics are stored negated (BwdArgs::stats)
     if (QSIDE) {
+      griddep_wait();
       const float4 sv = stat_row(args.stats, size_t(bh) * args.n_pad + size_t(tile) * BM + row);
       neg_l = br ? sv.y : sv.x;
       neg_e = br ? sv.w : sv.z;
@@ -313,8 +316,6 @@ diffattn_bwd_side128_kernel(const __grid_constant__ CUtensorMap tm_x0, const __g
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
-  // whoever waits for this grid waits for the one before it too
-  if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) griddep_wait();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -403,7 +404,7 @@ diffattn_bwd_dv128_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gri
         tma_load_4d(smem + OFF_K2 + c * 16384, &tm_k2, &misc->bar_kv, c * 64, kv_tile * BKV, h_idx, b_idx);
       }
       griddep_wait();        // dA and the statistics come from the preprocess kernel
-      griddep_launch();      // the side kernels depend on nothing else
+      griddep_launch();      // the key side may set itself up
       int qs = 0, as = 0, ts = 0;
       uint32_t qpar = 1, apar = 1, tpar = 1;
       for (int i = 0; i < nq; ++i) {

@@ -419,11 +419,11 @@ int bwd_impl(const DiffAttnParams* p, int32_t stages) {
   a.gain = p->gain; a.dgain = p->dgain;
   const int n_tiles = a.n_pad / 128;
   const int sms = sm_count(p->device);
-  // Within one call the kernels overlap: the first tensor-core kernel sets itself up under the preprocess kernel and waits
-  // for it; the later ones read nothing that an earlier tensor-core kernel writes, so they start as soon as every CTA
-  // of the one before has started (all of those have seen the preprocess kernel complete) and fill its last wave.
-  // Backward, one launch after the other -> overlapping: B2 H4 N128 D64 21.8 -> 12.5 us, B3 H5 N777 D64 53.6 -> 43.4, B4 H16
-  // N2048 D64 causal 383 -> 351, B2 H16 N2048 D64 dropout 416 -> 362.
+  // Within one call the kernels overlap: each sets itself up and requests the caller's tensors under the one before, then waits for it.
+  // (The later ones need nothing that an earlier tensor-core kernel writes, only the preprocess kernel's results.  But a dependent
+  // launch sees another grid's writes only after its own griddepcontrol.wait, which waits for the whole grid ahead of it.)
+  // Backward, one launch after the other -> overlapping: B2 H4 N128 D64 22.3 -> 16.8 us, B3 H5 N777 D64 47.3 -> 42.9, B4 H16
+  // N2048 D64 causal 348 -> 337, B2 H16 N2048 D64 dropout 406 -> 396.
   const bool pre = stages & DIFFATTN_STAGE_PRE, dkdv = stages & DIFFATTN_STAGE_DKDV;
 
   // 1. preprocess (grid-stride; one atomic per CTA for d(lambda)); zeroes the dQ partial sums of the single-pass form
