@@ -37,3 +37,32 @@ def test_running_maximum_changes_hands(d, n, jumps1, jumps2):
     # scores reach a few hundred: their fp32 rounding (6e-8 relative) and the exp unit's 2^-22 stay below 1e-5 of lse + 1e-3
     assert torch.allclose(lse1, want["lse1"], atol=2e-3, rtol=1e-5)
     assert torch.allclose(lse2, want["lse2"], atol=2e-3, rtol=1e-5)
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.1, 0.125])
+@pytest.mark.parametrize("b,h,n,d", [(1, 2, 128, 64), (1, 3, 384, 32), (4, 40, 128, 64), (2, 40, 256, 64), (1, 2, 384, 128)])
+def test_any_softmax_scale(b, h, n, d, scale):
+    """The C entry point takes the scale as it is given: 0 (every key alike) and negative scales (that of negated queries) too, also where
+    a CTA goes on to a second tile with the first one's running maximum still in shared memory."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import triton_diff_attn_b200 as pkg
+    from triton_diff_attn_b200 import _lib
+    q1, q2, k1, k2, v, _ = oracle.make_inputs(b, h, n, d, 700 + n + d)
+    lam = torch.tensor([0.5])
+    factor = scale * d ** 0.5                         # the oracle scales by 1 / sqrt(D)
+    want = oracle.forward(q1.double() * factor, q2.double() * factor, k1.double(), k2.double(), v.double(), lam, 0.2, False)
+    dev = torch.device("cuda", 0)
+    ins = [t.to(dev) for t in (q1, q2, k1, k2, v)]
+    saved = [torch.empty_like(ins[4]), torch.empty_like(ins[4])] + [torch.empty((b, h, n), device=dev) for _ in range(3)]
+    glam = lam.to(dev)
+    p = _lib.new_params()
+    pkg.layers._fill_common(p, *ins, glam, 0.2, False, saved)
+    p.sm_scale = scale
+    _lib.check(_lib.lib.diffattn_fwd(p), "fwd")
+    pkg.device_status(0)
+    m = oracle.error_metrics(saved[0].cpu(), want["y"])
+    # the repository's fp16 bound (with a negative scale the kernel's reference is the first sub-tile's maximum: unnormalised probabilities reach e^6 here, in range)
+    assert m["rel_l2"] <= 1e-3, m
+    assert torch.allclose(saved[2].cpu().double(), want["lse1"].double(), atol=2e-3, rtol=1e-5)
+    assert torch.allclose(saved[3].cpu().double(), want["lse2"].double(), atol=2e-3, rtol=1e-5)

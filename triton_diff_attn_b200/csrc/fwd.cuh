@@ -121,11 +121,12 @@ __device__ __forceinline__ void softmax_subtile(SoftmaxState& st, uint32_t t_s, 
   for (int i = 2; i < 32; ++i) mx[i & 3] = max3(mx[i & 3], __uint_as_float(sr[2 * i]), __uint_as_float(sr[2 * i + 1]));
   const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
   float m_prev = -INFINITY;
+  bool need = true;
   if (!first) {
     wait_m();
     m_prev = *m_row;
+    need = (m_tile - m_prev) * sl2 > 8.f;
   }
-  const bool need = (m_tile - m_prev) * sl2 > 8.f;       // t = 0: infinity
   const float m = need ? m_tile : m_prev;
   if (need) *m_row = m;
   publish_m();
@@ -144,7 +145,7 @@ __device__ __forceinline__ void softmax_subtile(SoftmaxState& st, uint32_t t_s, 
     }
   }
   if (m != st.m) {
-    st.l *= ex2((st.m - m) * sl2);
+    st.l *= ex2(fminf((st.m - m) * sl2, 0.f));        // (at first 0 times something finite, whatever the sign of the scale)
     st.m = m;
   }
   const f32x2 sl2_2 = pk2(sl2, sl2), neg_2 = pk2(-m * sl2, -m * sl2);

@@ -231,7 +231,7 @@ diffattn_fwd128_branch_kernel(const __grid_constant__ CUtensorMap tm_q1, const _
     misc->m_end[u][row] = st.m;
     misc->l_end[u][row] = st.l;
     named_bar_sync(1, NUM_SOFTMAX);
-    const float ma = misc->m_end[0][row], mb = misc->m_end[1][row], m_fin = fmaxf(ma, mb);
+    const float ma = misc->m_end[0][row], mb = misc->m_end[1][row], m_fin = misc->m_run[row];      // O is relative to the last running maximum
     const float l_fin = misc->l_end[0][row] * ex2((ma - m_fin) * sl2) + misc->l_end[1][row] * ex2((mb - m_fin) * sl2);
     const float inv_l = (DROP ? args.drop_scale : 1.f) / l_fin;
     const bool live = !*abort_flag && (q_tile * BM + row < args.n);

@@ -303,11 +303,11 @@ diffattn_fwd64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_co
       misc->m_end[br][u][row] = st.m;
       misc->l_end[br][u][row] = st.l;
       named_bar_sync(NB_ALL, NUM_SOFTMAX);
-      float m_fin[2], l_fin[2];         // both branches of this row: the later maximum of the two warpgroups, row sum relative to it
+      float m_fin[2], l_fin[2];         // both branches of this row: the last running maximum, to which O_b is relative; row sum relative to it
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
         const float ma = misc->m_end[b][0][row], mb = misc->m_end[b][1][row];
-        m_fin[b] = fmaxf(ma, mb);
+        m_fin[b] = misc->m_run[b][row];
         l_fin[b] = misc->l_end[b][0][row] * ex2((ma - m_fin[b]) * sl2) + misc->l_end[b][1][row] * ex2((mb - m_fin[b]) * sl2);
       }
       const float lam = load_lambda(args.lambda_ptr, args.lambda_dtype);
