@@ -165,3 +165,11 @@ def test_dropout_probability_quantisation():
     for bad in (-0.1, 1.0, 0.999):
         with pytest.raises(ValueError):
             dropout_threshold(bad)
+
+
+def test_core_refuses_what_is_no_tensor():
+    import triton_diff_attn_b200 as pkg
+    core = pkg.DiffAttnCore(32)
+    t = torch.zeros(1, 1, 4, 32, dtype=torch.float16)
+    with pytest.raises(TypeError, match="q1 must be a tensor"):
+        core([0.0], t, t, t, torch.zeros(1, 1, 4, 64, dtype=torch.float16))

@@ -306,7 +306,7 @@ class DiffAttnCore(torch.nn.Module):
         self.lambda_init, self.causal, self.dropout_p = float(lambda_init), bool(causal), float(dropout_p)
 
     def forward(self, q1, q2, k1, k2, v):
-        lam = _core_lambda((self.lambda_q1, self.lambda_k1, self.lambda_q2, self.lambda_k2), self.lambda_init, q1.device)
+        lam = _core_lambda((self.lambda_q1, self.lambda_k1, self.lambda_q2, self.lambda_k2), self.lambda_init, getattr(q1, "device", None))
         return MultiheadDiffAttnKernel(q1, q2, k1, k2, v, lam, self.lambda_init, True, causal=self.causal,
                                        dropout_p=self.dropout_p if self.training else 0.0, gain=self.gain)
 
