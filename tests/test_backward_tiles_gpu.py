@@ -1,6 +1,7 @@
 """The query-side backward consumes 128-key tiles in four column groups of 32, one group per warpgroup, two of them half a
 branch behind the others; the attention dropout mask is walked along rows there and along columns on the key side.  Sequence lengths
 put the last visible key at the edges of those groups and tiles, with one tile, an odd and an even number of them."""
+import numpy as np
 import pytest
 import torch
 
@@ -138,5 +139,7 @@ def test_core_lambda_in_one_launch(n, create_graph):
         assert torch.allclose(a.detach().cpu().double(), b, rtol=1e-5, atol=1e-6)
     if create_graph:
         assert all(t is not None for t in torch.autograd.grad(sum(t.sum() for t in got), vec))
+    for number in (np.float32(0.75), np.array(0.75), torch.tensor(0.75)):        # whatever float() takes, as in tensor operations
+        assert torch.equal(pkg.layers._core_lambda(vec, number, dev), pkg.layers._core_lambda(vec, 0.75, dev))
     half = [t.half().to(dev) for t in host]                      # anything but fp32 goes through tensor operations as before
     assert torch.equal(pkg.layers._core_lambda(half, 0.8, dev), pkg.lambda_from_reparam(*half, 0.8))
