@@ -148,7 +148,7 @@ int diffattn_bwd_static(const DiffAttnParams* p);
 /* The re-parameterisation of lambda in the layer around the operator (src/layers.py:114 names that layer; the reference itself
  * takes lambda ready-made): out = { exp(<q1,k1>) - exp(<q2,k2>) + lambda_init, exp(<q1,k1>), exp(<q2,k2>) } from four fp32 vectors of
  * n elements, and the vectors' gradients from dlambda (one fp32) and that `out`.  One kernel each, enqueued on `stream`; every
- * pointer is device memory of `device`. */
+ * pointer is device memory of `device`.  Added within version 2: a host that loads libraries of other builds looks the two up. */
 int diffattn_lambda_fwd(int32_t device, void* stream, int32_t n, const float* q1, const float* k1, const float* q2, const float* k2,
                         float lambda_init, float* out);
 int diffattn_lambda_bwd(int32_t device, void* stream, int32_t n, const float* q1, const float* k1, const float* q2, const float* k2,

@@ -173,3 +173,17 @@ def test_core_refuses_what_is_no_tensor():
     t = torch.zeros(1, 1, 4, 32, dtype=torch.float16)
     with pytest.raises(TypeError, match="q1 must be a tensor"):
         core([0.0], t, t, t, torch.zeros(1, 1, 4, 64, dtype=torch.float16))
+
+
+def test_library_without_the_lambda_entries_loads(tmp_path):
+    """The two entries came within version 2: a library of that version without them still serves the operator."""
+    import subprocess
+    import sys
+    from triton_diff_attn_b200 import _lib
+    src, lib = tmp_path / "stub.c", tmp_path / "libstub.so"
+    src.write_text("".join(f"long {n}(void) {{ return 2; }}\n" for n in _lib.EXPORTS if "lambda" not in n))
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(lib), str(src)], check=True)
+    code = ("import torch, triton_diff_attn_b200 as p; from triton_diff_attn_b200 import _lib; assert not _lib.lib.has_lambda; "
+            "assert _lib.lib.diffattn_version() == 2; v = [torch.ones(4)] * 4; print(p.layers._core_lambda(v, 0.5, v[0].device))")
+    out = subprocess.run([sys.executable, "-c", code], cwd=REPO, env=dict(os.environ, DIFFATTN_LIBRARY=str(lib)), capture_output=True, text=True)
+    assert out.returncode == 0 and "0.5" in out.stdout, out.stderr

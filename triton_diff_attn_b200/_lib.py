@@ -61,10 +61,13 @@ def _load() -> C.CDLL:
     lib.diffattn_bwd_stages.restype = C.c_int
     lib.diffattn_bwd_static.argtypes = [C.POINTER(DiffAttnParams)]
     lib.diffattn_bwd_static.restype = C.c_int
-    lib.diffattn_lambda_fwd.argtypes = [C.c_int32, C.c_void_p, C.c_int32] + [C.c_void_p] * 4 + [C.c_float, C.c_void_p]
-    lib.diffattn_lambda_fwd.restype = C.c_int
-    lib.diffattn_lambda_bwd.argtypes = [C.c_int32, C.c_void_p, C.c_int32] + [C.c_void_p] * 10
-    lib.diffattn_lambda_bwd.restype = C.c_int
+    # (added within version 2: another build of that version, named by DIFFATTN_LIBRARY, may not have them)
+    lib.has_lambda = hasattr(lib, "diffattn_lambda_fwd") and hasattr(lib, "diffattn_lambda_bwd")
+    if lib.has_lambda:
+        lib.diffattn_lambda_fwd.argtypes = [C.c_int32, C.c_void_p, C.c_int32] + [C.c_void_p] * 4 + [C.c_float, C.c_void_p]
+        lib.diffattn_lambda_fwd.restype = C.c_int
+        lib.diffattn_lambda_bwd.argtypes = [C.c_int32, C.c_void_p, C.c_int32] + [C.c_void_p] * 10
+        lib.diffattn_lambda_bwd.restype = C.c_int
     lib.diffattn_workspace_bytes.argtypes = [C.POINTER(DiffAttnParams)]
     lib.diffattn_workspace_bytes.restype = C.c_uint64
     lib.diffattn_status.argtypes = [C.c_int32]

@@ -286,7 +286,7 @@ def _core_lambda(vectors, lambda_init, device):
     """lambda of a `DiffAttnCore`: one launch where the four vectors are plain dense fp32 vectors of one length on the inputs' GPU,
     tensor operations for everything else (other types, moved or replaced parameters)."""
     a = vectors[0]
-    if all(type(t) in (torch.nn.Parameter, torch.Tensor) and t.is_cuda and t.dtype == torch.float32 and t.dim() == 1 and t.is_contiguous()
+    if _lib.lib.has_lambda and all(type(t) in (torch.nn.Parameter, torch.Tensor) and t.is_cuda and t.dtype == torch.float32 and t.dim() == 1 and t.is_contiguous()
            and t.shape == a.shape and t.device == device for t in vectors) and a.numel() > 0:
         return _LambdaReparam.apply(*vectors, float(lambda_init))      # (ctypes takes nothing but a Python number)
     return lambda_from_reparam(*vectors, lambda_init)
