@@ -8,7 +8,7 @@
 // A2 = O_2 / l_2 in fp32 to branch 1 through distributed shared memory, and branch 1 forms y and rstd.
 // What bounds it: the tensor pipe needs 768 clocks per sub-tile (S 256, P V 512), and at B2 H8 N8192 D128 it executes
 // 1377 TFLOP/s sustained, the rate a plain cuBLAS loop reaches under the 1 kW cap.  Against one softmax warpgroup with P over
-// its scores and Q in shared memory: 1.44 -> 1.20 ms there, 0.206 -> 0.160 ms at B1 H8 N4096 causal; both warpgroups in phase 1.29.
+// its scores and Q in shared memory: 1.44 -> 1.20 ms there, a call at B1 H8 N4096 causal 168 -> 126 us; both warpgroups in phase 1.29 ms.
 // (An earlier form kept both branches in one CTA and made two passes over the keys, with the probabilities recomputed in
 // the second: 1.97 ms.  A form without the cluster -- branch 1 writes A1 as 16-bit values into y, a second kernel
 // combines -- lost accuracy where A1 - lambda A2 cancels: with bf16 tensors, lambda 0.8, a causal mask and rms_norm two of 400
