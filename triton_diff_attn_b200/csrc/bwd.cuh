@@ -389,6 +389,7 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
       }
       mma_commit(&misc->s_full);        // two arrivals per tile: this warp's and the other score issuer's
     };
+    griddep_wait();
     bool ok = true;
     int st = 0;
     uint32_t par = 0;
@@ -456,6 +457,7 @@ diffattn_bwd_dkdv64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gr
     const float sg = load_lambda(args.lambda_ptr, args.lambda_dtype) < 0.f ? 1.f : -1.f;   // -sign(lambda)
     const f32x2 dscale_2 = pk2(args.drop_scale, args.drop_scale), sgd_2 = pk2(sg * args.drop_scale, sg * args.drop_scale);     // DROP only
     const f32x2 sl2_2 = pk2(sl2, sl2), sg_2 = pk2(sg, sg);
+    griddep_wait();
     uint32_t s_ready = 0;            // answers of the early probes (see mbar_probe)
     int st = 0;
     for (; work.valid(); work.next()) {
@@ -770,6 +772,7 @@ diffattn_bwd_dq64_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid
         mma_ts_lo(tb + (br ? T_DQ2 : T_DQ1), tb + (br ? T_S2 : T_S1) + (k / 2) * 32 + (k % 2) * 8, k_lo + k * (2048 >> 4), IDESC_DQ,
                   k > 0 ? 1u : first);
     };
+    griddep_wait();
     bool ok = true;
     int ks = 0, vs = 0;                // ring slots of tile j
     uint32_t k_par = 0, v_par = 0;     // parities of their passes over the rings

@@ -146,6 +146,7 @@ diffattn_bwd_side128_kernel(const __grid_constant__ CUtensorMap tm_x0, const __g
         mma_commit(&misc->s_full[u]);
         mma_commit(&misc->wempty[ws]);
       };
+      griddep_wait();
       bool ok = mbar_wait(&misc->bar_xy, 0, abort_flag, 1201);
       ok = ok && mbar_wait(&misc->y_ready, 0, abort_flag, 1206);
       ok = ok && mbar_wait(&misc->full[0], 0, abort_flag, 1202);
@@ -220,6 +221,7 @@ diffattn_bwd_side128_kernel(const __grid_constant__ CUtensorMap tm_x0, const __g
       tc_fence_before();
       mbar_arrive(&misc->y_ready);
     }
+    if (!QSIDE) griddep_wait();
     int st = 0;
     for (int t = 0; ok && t < nsub; ++t) {
       const int u = t & 1;
@@ -448,6 +450,7 @@ diffattn_bwd_dv128_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gri
         mma_commit(&misc->s_full);             // (the statistics of the tile arrived with Q: s_full implies them)
         mma_commit(&misc->qempty[qs]);
       };
+      griddep_wait();
       bool ok = mbar_wait(&misc->k_ready, 0, abort_flag, 1501);
       ok = ok && mbar_wait(&misc->qfull[0], 0, abort_flag, 1502);
       if (ok) {
@@ -514,6 +517,7 @@ diffattn_bwd_dv128_kernel(const __grid_constant__ CUtensorMap tm_q1, const __gri
       tc_fence_before();
       mbar_arrive(&misc->k_ready);
     }
+    griddep_wait();
     int st = 0;
     for (int i = 0; ok && i < nq; ++i) {
       const float4* stats = reinterpret_cast<const float4*>(smem + OFF_ST + st * STAT_BYTES) + g * 16;

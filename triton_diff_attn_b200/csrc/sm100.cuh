@@ -47,7 +47,8 @@ __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.al
 
 // Programmatic dependent launch.  griddep_launch: once every CTA of this grid has called it (or ended), a following kernel
 // that was launched with the attribute may start in whatever room the SMs have.  griddep_wait: returns when the grid before
-// this one has completed and its writes are visible (at once in a kernel launched without the attribute).
+// this one has completed and its writes are visible (at once in a kernel launched without the attribute).  It has no time limit; a bounded
+// wait for anything that comes after it would count the time that the grid ahead still takes, so such a wait goes behind it in every role.
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
